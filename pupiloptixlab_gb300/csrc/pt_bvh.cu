@@ -515,12 +515,12 @@ __device__ __forceinline__ void write_slot(float *node, int c, float3 lo, float3
     node[3 * K + c] = hi.y;
     node[4 * K + c] = lo.z;
     node[5 * K + c] = hi.z;
-    node[6 * K + c] = __int_as_float(child);
-    node[7 * K + c] = __int_as_float(count);
+    node[6 * K + c] = __int_as_float(count > 0 ? ptd::make_leaf(child, count) : child);
 }
+__device__ __forceinline__ int item_count(int item) { return ptd::is_leaf(item) ? ptd::leaf_count(item) : 0; }
 template <int K>
 __device__ __forceinline__ void write_empty(float *node, int c) {
-    write_slot<K>(node, c, f3(1e30f, 1e30f, 1e30f), f3(1e30f, 1e30f, 1e30f), -1, 0);
+    write_slot<K>(node, c, f3(1e30f, 1e30f, 1e30f), f3(1e30f, 1e30f, 1e30f), ptd::kNoItem, 0);
 }
 
 // 6. SAH-optimal wide collapse (Ylitie, Karras and Laine, HPG 2017): for
@@ -687,11 +687,11 @@ __global__ void k_sah(const float *nodes, uint32_t num_nodes, double *acc) {
     if (i < num_nodes) {
         const float *nd = nodes + (size_t)i * 8 * K;
         for (int c = 0; c < K; c++) {
-            int ch = __float_as_int(nd[6 * K + c]);
-            if (ch < 0) continue;
+            const int item = __float_as_int(nd[6 * K + c]);
+            if (item == ptd::kNoItem) continue;
             float ex = nd[K + c] - nd[c], ey = nd[3 * K + c] - nd[2 * K + c], ez = nd[5 * K + c] - nd[4 * K + c];
             float a = ex * ey + ey * ez + ez * ex;
-            int cnt = __float_as_int(nd[7 * K + c]);
+            const int cnt = item_count(item);
             v += (double)a * (cnt > 0 ? (double)kCostPrim * cnt : (double)kCostNode);
         }
     }
@@ -707,9 +707,9 @@ __global__ void k_refit_level(float *nodes, uint32_t first, uint32_t last, const
     if (i >= last) return;
     float *nd = nodes + (size_t)i * 8 * K;
     for (int c = 0; c < K; c++) {
-        int ch = __float_as_int(nd[6 * K + c]);
-        if (ch < 0) continue;
-        int cnt = __float_as_int(nd[7 * K + c]);
+        const int item = __float_as_int(nd[6 * K + c]);
+        if (item == ptd::kNoItem) continue;
+        const int cnt = item_count(item), ch = cnt > 0 ? ptd::leaf_first(item) : item;
         float4 lo = make_float4(FLT_MAX, FLT_MAX, FLT_MAX, 0.f), hi = make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, 0.f);
         if (cnt > 0) {
             for (int j = 0; j < cnt; j++) {
@@ -721,7 +721,7 @@ __global__ void k_refit_level(float *nodes, uint32_t first, uint32_t last, const
         } else {
             const float *cn = nodes + (size_t)ch * 8 * K;
             for (int g = 0; g < K; g++) {
-                if (__float_as_int(cn[6 * K + g]) < 0) continue;
+                if (__float_as_int(cn[6 * K + g]) == ptd::kNoItem) continue;
                 lo = make_float4(fminf(lo.x, cn[g]), fminf(lo.y, cn[2 * K + g]), fminf(lo.z, cn[4 * K + g]), 0.f);
                 hi = make_float4(fmaxf(hi.x, cn[K + g]), fmaxf(hi.y, cn[3 * K + g]), fmaxf(hi.z, cn[5 * K + g]), 0.f);
             }
@@ -787,7 +787,7 @@ __global__ void k_root_area(const float *nodes, double *out) {
     if (threadIdx.x || blockIdx.x) return;
     float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
     for (int c = 0; c < K; c++) {
-        if (__float_as_int(nodes[6 * K + c]) < 0) continue;
+        if (__float_as_int(nodes[6 * K + c]) == ptd::kNoItem) continue;
         for (int a = 0; a < 3; a++) {
             lo[a] = fminf(lo[a], nodes[2 * a * K + c]);
             hi[a] = fmaxf(hi[a], nodes[(2 * a + 1) * K + c]);
@@ -814,7 +814,7 @@ __global__ void k_compress8(const float *nodes, uint32_t n, float4 *out) {
         float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
         uint32_t occupied = 0;
         for (int c = 0; c < 8; c++) {
-            if (__float_as_int(f[48 + c]) < 0) continue;
+            if (__float_as_int(f[48 + c]) == ptd::kNoItem) continue;
             occupied |= 1u << c;
             for (int a = 0; a < 3; a++) {
                 lo[a] = fminf(lo[a], f[16 * a + c]);
@@ -890,8 +890,7 @@ __global__ void k_compress8(const float *nodes, uint32_t n, float4 *out) {
                 cl[a][sl >> 2] |= (uint32_t)ql << (8 * (sl & 3));
                 ch[a][sl >> 2] |= (uint32_t)qh << (8 * (sl & 3));
             }
-            const int child = __float_as_int(f[48 + c]), count = __float_as_int(f[56 + c]);
-            items[sl] = count > 0 ? ptd::make_leaf(child, count) : child;
+            items[sl] = __float_as_int(f[48 + c]);
         }
         q[0] = make_float4(lo[0], lo[1], lo[2], __uint_as_float(eb[0] | eb[1] << 8 | eb[2] << 16 | used << 24));
         for (int a = 0; a < 3; a++)

@@ -1169,18 +1169,17 @@ struct Launcher {
 };
 
 // Merged-BVH child rebasing: inner children move by the scene's first node,
-// leaf children (count > 0) by its first primitive slot.
+// leaves by its first primitive slot.
 template <int K>
 __global__ void k_rebase_nodes(float4 *nodes, uint32_t num_nodes, int node_off, int prim_off) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < num_nodes; i += gridDim.x * blockDim.x) {
         float *f = reinterpret_cast<float *>(nodes + (size_t)i * 2 * K);
 #pragma unroll
         for (int c = 0; c < K; c++) {
-            int ch = __float_as_int(f[6 * K + c]);
-            const int cnt = __float_as_int(f[7 * K + c]);
-            if (ch < 0) continue;
-            ch += cnt > 0 ? prim_off : node_off;
-            f[6 * K + c] = __int_as_float(ch);
+            const int item = __float_as_int(f[6 * K + c]);
+            if (item == ptd::kNoItem) continue;
+            f[6 * K + c] = __int_as_float(is_leaf(item) ? make_leaf(leaf_first(item) + prim_off, leaf_count(item))
+                                                        : item + node_off);
         }
     }
 }

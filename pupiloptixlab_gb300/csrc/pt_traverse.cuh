@@ -13,9 +13,9 @@
 //
 // Memory layout (HBM):
 //   node  = 8*K floats: lo_x[K] hi_x[K] lo_y[K] hi_y[K] lo_z[K] hi_z[K]
-//           child[K] count[K]; count > 0: leaf over primitive slots
-//           [child, child + count); count == 0 and child >= 0: inner node;
-//           child < 0: empty slot.  Loaded as 2*K float4 (128-bit) loads.
+//           item[K], K unused.  item: a traversal item (below): an inner node's
+//           index, a leaf's first slot and count, or kNoItem (empty slot, a
+//           point box far away).  Loaded in 256-bit loads.
 //   prim  = 3 float4 per slot: triangle (v0, id) (v1, 0) (v2, 0);
 //           sphere (centre, id | 1<<31) (radius, 0, 0, 0) (0);
 //           curve piece (c0, id | 1<<31) (r0, r1, u0, kind bits) (c1, u1):
@@ -34,6 +34,16 @@ namespace ptd {
 constexpr int kShortStack = 16;  // shared-memory entries per thread
 constexpr int kSpillStack = kTraversalStackEntries - kShortStack;  // local-memory overflow entries per thread
 constexpr float kSlabScale = 1.0000004f;  // 1 + 2*gamma(3): robust slab far bound (Ize 2013)
+
+// Traversal items: a node index (>= 0), a leaf (bit 31 | first << 4 | count)
+// or kNoItem.  Leaves must start below 2^27 - 1 (checked at scene upload).
+// Nodes hold their children in this form: forming them at every visit (child
+// and count) cost the closest hit 105 against 89.5 ms and spilled registers.
+constexpr int kNoItem = -1;
+PT_DI int make_leaf(int first, int count) { return (int)(0x80000000u | ((uint32_t)first << 4) | (uint32_t)count); }
+PT_DI bool is_leaf(int item) { return item < 0 && item != kNoItem; }
+PT_DI int leaf_first(int item) { return (int)(((uint32_t)item >> 4) & 0x7ffffffu); }
+PT_DI int leaf_count(int item) { return item & 15; }
 
 struct TraceResult {
     float t;
@@ -239,8 +249,7 @@ struct WideNode {
     PT_DI float hiy(int c) const { return f[3 * K + c]; }
     PT_DI float loz(int c) const { return f[4 * K + c]; }
     PT_DI float hiz(int c) const { return f[5 * K + c]; }
-    PT_DI int child(int c) const { return __float_as_int(f[6 * K + c]); }
-    PT_DI int count(int c) const { return __float_as_int(f[7 * K + c]); }
+    PT_DI int item(int c) const { return __float_as_int(f[6 * K + c]); }
 };
 
 // BVH nodes and primitive records are read many times per wave while the ray
@@ -273,10 +282,24 @@ PT_DI void st_stream(T *p, T v) {
     __stcs(p, v);
 }
 
+// The 7*K floats in use: width 4 three 256-bit loads and one of 128 bits.
 template <int K>
 PT_DI void load_node(const float4 *__restrict__ p, WideNode<K> &n) {
 #pragma unroll
-    for (int i = 0; i < K; i++) ld_bvh8(p + 2 * i, n.f + 8 * i);
+    for (int i = 0; i < 7 * K / 8; i++) ld_bvh8(p + 2 * i, n.f + 8 * i);
+    if (7 * K % 8) {
+        const float4 v = ld_bvh(p + 7 * K / 8 * 2);
+        float *f = n.f + 7 * K / 8 * 8;
+        f[0] = v.x;
+        f[1] = v.y;
+        f[2] = v.z;
+        f[3] = v.w;
+        if (7 * K % 8 > 4) {  // width 2: floats 12, 13
+            const float4 u = ld_bvh(p + 7 * K / 8 * 2 + 1);
+            f[4] = u.x;
+            f[5] = u.y;
+        }
+    }
 }
 template <int K>
 PT_DI void load_node_smem(const float4 *p, WideNode<K> &n) {
@@ -289,14 +312,6 @@ PT_DI void load_node_smem(const float4 *p, WideNode<K> &n) {
         n.f[4 * i + 3] = v.w;
     }
 }
-
-// Traversal items: a node index (>= 0), a leaf (bit 31 | first << 4 | count)
-// or kNoItem.  Leaves must start below 2^27 - 1 (checked at scene upload).
-constexpr int kNoItem = -1;
-PT_DI int make_leaf(int first, int count) { return (int)(0x80000000u | ((uint32_t)first << 4) | (uint32_t)count); }
-PT_DI bool is_leaf(int item) { return item < 0 && item != kNoItem; }
-PT_DI int leaf_first(int item) { return (int)(((uint32_t)item >> 4) & 0x7ffffffu); }
-PT_DI int leaf_count(int item) { return item & 15; }
 
 // Compressed 8-wide nodes: 96 bytes (6 float4) per node, after the quantised
 // wide nodes of Ylitie, Karras and Laine ("Efficient Incoherent Ray Traversal
@@ -403,6 +418,12 @@ struct ShortStack {
             overflow = 1;
             return;
         }
+        sp++;
+    }
+    // room for n entries without a check for each: push_short may be used
+    PT_DI bool short_room(int n) const { return sp + n <= kShortStack; }
+    PT_DI void push_short(int item, float t) {
+        smem[sp * stride] = make_int2(item, __float_as_int(t));
         sp++;
     }
     PT_DI int2 pop() {
@@ -523,10 +544,14 @@ PT_DI void trace_persistent(const DevScene &s, const float4 *snodes, int2 *sstac
                 // the first hit child is descended, the later ones pushed (popped in visiting order)
                 int next = kNoItem;
                 float next_t = 0.f;
+                const bool room = st.short_room(7);
 #pragma unroll
                 for (int i = 7; i >= 0; i--) {
                     if (ci[i] == kNoItem) continue;
-                    if (next != kNoItem) st.push(next, next_t, ovf);
+                    if (next != kNoItem) {
+                        if (room) st.push_short(next, next_t);
+                        else st.push(next, next_t, ovf);
+                    }
                     next = ci[i];
                     next_t = ct[i];
                 }
@@ -543,8 +568,6 @@ PT_DI void trace_persistent(const DevScene &s, const float4 *snodes, int2 *sstac
                 for (int c = 0; c < K; c++) {
                     ci[c] = kNoItem;
                     ct[c] = __int_as_float(0x7f800000);
-                    int ch = nd.child(c);
-                    if (ch < 0) continue;
                     float tx0, tx1, ty0, ty1, tz0, tz1;
                     if (fma_slab) {  // t = lo * inv - o * inv: one rounding, conservative within pad_mag
                         tx0 = __fmaf_rn(nd.lox(c), inv.x, -oi.x);
@@ -565,8 +588,7 @@ PT_DI void trace_persistent(const DevScene &s, const float4 *snodes, int2 *sstac
                     float tf = fminf(fminf(fmaxf(tx0, tx1), fmaxf(ty0, ty1)), fmaxf(tz0, tz1));
                     tf = fminf(tf * kSlabScale, tlimit);
                     if (!(tn <= tf)) continue;
-                    int cnt = nd.count(c);
-                    ci[c] = cnt > 0 ? make_leaf(ch, cnt) : ch;
+                    ci[c] = nd.item(c);  // an empty slot's stays kNoItem whatever its box says
                     ct[c] = tn;
                 }
                 // closest hit: nearest child first (sorting network); any hit: order
@@ -593,9 +615,17 @@ PT_DI void trace_persistent(const DevScene &s, const float4 *snodes, int2 *sstac
                             ci[i] = kNoItem;
                         }
                 }
+                // one check for the whole node while the short stack has room
+                // (a check per push: closest / any hit 89.5 / 27.8 ms, so 85.9 / 25.8)
+                if (st.short_room(K - 1)) {
 #pragma unroll
-                for (int i = K - 1; i >= 1; i--)
-                    if (ci[i] != kNoItem) st.push(ci[i], ct[i], ovf);
+                    for (int i = K - 1; i >= 1; i--)
+                        if (ci[i] != kNoItem) st.push_short(ci[i], ct[i]);
+                } else {
+#pragma unroll
+                    for (int i = K - 1; i >= 1; i--)
+                        if (ci[i] != kNoItem) st.push(ci[i], ct[i], ovf);
+                }
                 item = ci[0] != kNoItem ? ci[0] : pop_valid();
             }
             if (is_leaf(item) && leaf == kNoItem) {  // postpone the first leaf
