@@ -302,10 +302,10 @@ struct UserSrc {  // pt_trace_rays
 
 // Stages the top smem_nodes nodes in shared memory; returns the stack base.
 template <int K>
-PT_DI int2 *stage_smem(const DevScene &s, float4 *smem) {
+PT_DI void *stage_smem(const DevScene &s, float4 *smem) {
     for (uint32_t i = threadIdx.x; i < s.smem_nodes * 2 * K; i += blockDim.x) smem[i] = __ldg(s.nodes + i);
     __syncthreads();
-    return reinterpret_cast<int2 *>(smem + s.smem_nodes * 2 * K);
+    return smem + s.smem_nodes * 2 * K;
 }
 
 // ANY = false: closest hit of the extension rays; ANY = true: shadow rays.
@@ -314,7 +314,7 @@ PT_DI int2 *stage_smem(const DevScene &s, float4 *smem) {
 template <int K, bool ANY, bool COUNT, bool BATCH = false, bool CURVES = false>
 __global__ void __maxnreg__(K == 8 ? 96 : 72) k_trace_queue(DevScene s, State st, Batch bt, uint32_t frames) {
     extern __shared__ float4 smem[];
-    int2 *sstack = stage_smem<K>(s, smem);
+    void *sstack = stage_smem<K>(s, smem);
     if (ANY) {
         if (BATCH) {
             BatchShadowSrc src;
@@ -792,7 +792,7 @@ __global__ void k_accumulate(State st, Wave w, Outputs out0, Batch bt, uint32_t 
 template <int K, bool ANY, bool CURVES>
 __global__ void k_trace_rays(DevScene s, const float4 *rays, float4 *hits, uint32_t n, uint32_t *work, uint32_t *ovf_flag) {
     extern __shared__ float4 smem[];
-    int2 *sstack = stage_smem<K>(s, smem);
+    void *sstack = stage_smem<K>(s, smem);
     UserSrc<ANY> src{rays, hits, n};
     trace_persistent<K, ANY, false, UserSrc<ANY>, CURVES>(s, smem, sstack, src, work, ovf_flag, nullptr, nullptr, nullptr);
 }
@@ -949,16 +949,19 @@ struct Launcher {
         stt.stats = reinterpret_cast<unsigned long long *>(ws.counters.as<uint32_t>() + kStatBase);
 
         const int tb = p->block_size ? (int)p->block_size : (t.tuned_block ? (int)t.tuned_block : 128);
-        const size_t smem = (size_t)d.smem_nodes * 32 * K + (size_t)kShortStack * 8 * tb;
+        const size_t smem = (size_t)d.smem_nodes * 32 * K + (size_t)kShortStack * stack_entry_bytes(false) * tb;
+        const size_t smem_sh = (size_t)d.smem_nodes * 32 * K + (size_t)kShortStack * stack_entry_bytes(true) * tb;
         auto k_ext = t.curves ? (count ? k_trace_queue<K, false, true, BATCH, true> : k_trace_queue<K, false, false, BATCH, true>)
                               : (count ? k_trace_queue<K, false, true, BATCH> : k_trace_queue<K, false, false, BATCH>);
         auto k_sh = t.curves ? (count ? k_trace_queue<K, true, true, BATCH, true> : k_trace_queue<K, true, false, BATCH, true>)
                              : (count ? k_trace_queue<K, true, true, BATCH> : k_trace_queue<K, true, false, BATCH>);
-        if ((e = set_smem(k_ext, smem)) != PT_OK || (e = set_smem(k_sh, smem)) != PT_OK) return e;
-        int occ_t = 0, occ_s = 0;
+        if ((e = set_smem(k_ext, smem)) != PT_OK || (e = set_smem(k_sh, smem_sh)) != PT_OK) return e;
+        int occ_t = 0, occ_s = 0, occ_h = 0;
         PT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_t, k_ext, tb, smem));
         PT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s, k_shade<BATCH>, 256, 0));
+        PT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_h, k_sh, tb, smem_sh));
         const uint32_t grid_trace = (uint32_t)std::max(1, occ_t) * t.num_sms;
+        const uint32_t grid_shadow = (uint32_t)std::max(1, occ_h) * t.num_sms;
         const uint32_t grid_shade = (uint32_t)std::max(1, occ_s) * t.num_sms;
 
         const bool sort = (p->flags & PT_RENDER_NO_MATERIAL_SORT) == 0;
@@ -1044,7 +1047,7 @@ struct Launcher {
                 if (timing) { tm.mark(2, ls); tm.mark(1, ls); }
                 {
                     pt_nvtx::Range r("shadow (any hit)");
-                    k_sh<<<grid_trace, tb, smem, ls>>>(d, stt, bt, w.frames);
+                    k_sh<<<grid_shadow, tb, smem_sh, ls>>>(d, stt, bt, w.frames);
                 }
                 if (timing) tm.mark(1, ls);
                 k_advance<<<1, 1, 0, ls>>>(stt.counters);
@@ -1145,7 +1148,7 @@ struct Launcher {
         int e = s->ws.counters.ensure(256);
         if (e != PT_OK) return e;
         const int tb = 128;
-        const size_t smem = (size_t)d.smem_nodes * 32 * K + (size_t)kShortStack * 8 * tb;
+        const size_t smem = (size_t)d.smem_nodes * 32 * K + (size_t)kShortStack * stack_entry_bytes(anyhit != 0) * tb;
         const bool curves = s->num_curve_pieces > 0;
         auto kern = curves ? (anyhit ? k_trace_rays<K, true, true> : k_trace_rays<K, false, true>)
                            : (anyhit ? k_trace_rays<K, true, false> : k_trace_rays<K, false, false>);
@@ -1544,16 +1547,19 @@ int render_noalloc(pt_scene *s, const pt_render_params *p, const pt_frame_buffer
 
     // the traversal block size pt_render would use: the caller's, else the autotuned one, else 128
     const int tb = p->block_size ? (int)p->block_size : (s->tuned_block ? (int)s->tuned_block : 128);
-    const size_t smem = (size_t)d.smem_nodes * 32 * K + (size_t)kShortStack * 8 * tb;
+    const size_t smem = (size_t)d.smem_nodes * 32 * K + (size_t)kShortStack * stack_entry_bytes(false) * tb;
+    const size_t smem_sh = (size_t)d.smem_nodes * 32 * K + (size_t)kShortStack * stack_entry_bytes(true) * tb;
     const bool curves = s->num_curve_pieces > 0;
     auto k_ext = curves ? k_trace_queue<K, false, false, false, true> : k_trace_queue<K, false, false>;
     auto k_sh = curves ? k_trace_queue<K, true, false, false, true> : k_trace_queue<K, true, false>;
     int e;
-    if ((e = set_smem(k_ext, smem)) != PT_OK || (e = set_smem(k_sh, smem)) != PT_OK) return e;
-    int occ_t = 0, occ_s = 0;
+    if ((e = set_smem(k_ext, smem)) != PT_OK || (e = set_smem(k_sh, smem_sh)) != PT_OK) return e;
+    int occ_t = 0, occ_s = 0, occ_h = 0;
     PT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_t, k_ext, tb, smem));
     PT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s, k_shade<false>, 256, 0));
+    PT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_h, k_sh, tb, smem_sh));
     const uint32_t grid_trace = (uint32_t)std::max(1, occ_t) * s->num_sms;
+    const uint32_t grid_shadow = (uint32_t)std::max(1, occ_h) * s->num_sms;
     const uint32_t grid_shade = (uint32_t)std::max(1, occ_s) * s->num_sms;
 
     // the array keeps the previous call's contents: clear the counters and statistics
@@ -1575,7 +1581,7 @@ int render_noalloc(pt_scene *s, const pt_render_params *p, const pt_frame_buffer
         for (uint32_t b = 0; b < max_depth; b++) {
             k_ext<<<grid_trace, tb, smem, st>>>(d, stt, Batch{}, w.frames);
             k_shade<false><<<grid_shade, 256, 0, st>>>(d, Batch{}, stt, w, out);
-            k_sh<<<grid_trace, tb, smem, st>>>(d, stt, Batch{}, w.frames);
+            k_sh<<<grid_shadow, tb, smem_sh, st>>>(d, stt, Batch{}, w.frames);
             k_advance<<<1, 1, 0, st>>>(stt.counters);
             std::swap(stt.q_in, stt.q_out);
         }
