@@ -395,7 +395,7 @@ int pt_render_get_stats(const pt_scene *scene, pt_render_stats *out);
  * from their own fixed pools or budgets, and interactive callers that must not
  * allocate per frame, since an allocation can synchronise the device).  The
  * render's path state lives in a fixed device array inside the library (about
- * 9.3 MiB, held by every GPU that loads the library until exit) instead of a
+ * 8.5 MiB, held by every GPU that loads the library until exit) instead of a
  * workspace allocated on first use; the call makes no allocation.  Limit: at
  * most 65,536 pixels (width * height) per call; larger images are rejected
  * with PT_ERR_INVALID.  The first call on a device looks up the array's device

@@ -57,17 +57,27 @@ struct Wave {
     uint32_t max_depth;
     uint32_t rng_mode;
     uint32_t accumulate;
+    uint32_t bounce;       // bounce of this launch: the depth of every path in the queue
+    uint32_t bounces;      // bounces of the wave
 };
 
+// Path state.  A slot's ray is one 32-byte sector, moved with one 256-bit
+// access: slots get sparse as paths end and are binned by material, and
+// separate 16-byte arrays then waste half of each sector.  The ray record also
+// carries the random stream's state (an extension ray's range is fixed), the
+// queue entry whether the last lobe was a delta; a path's depth is the wave's
+// bounce.
 struct State {
-    float4 *ray_o, *ray_d, *hit, *thr, *rad;
-    uint2 *rng;
-    uint32_t *meta;
-    uint32_t *q_in, *q_out;
+    float4 *ray;   // 2 per slot: (origin, stream low bits) (direction, stream high bits)
+    float4 *hit, *rad;
+    float4 *thr;   // throughput, pdf of the last BSDF sample
+    uint32_t *q_in, *q_out;  // path slot | kEntryDelta
     float4 *sh_o, *sh_d, *sh_c;
     uint32_t *counters;
     unsigned long long *stats;
 };
+constexpr uint32_t kEntryDelta = 1u << 31;  // slots are below 2^31
+PT_DI uint32_t entry_slot(uint32_t e) { return e & ~kEntryDelta; }
 
 struct Outputs {
     float4 *accum, *frame;
@@ -115,14 +125,14 @@ PT_DI uint32_t tile_pixel(uint32_t r, uint32_t width, uint32_t height) {
     return (y0 + in_band - x * rows) * width + x;
 }
 
-PT_DI void save_rng(uint2 *dst, const Sampler &s) {
-    *dst = make_uint2((uint32_t)s.state, (uint32_t)(s.state >> 32));
+PT_DI void store_ray(const State &st, uint32_t slot, float3 o, float3 d, const Sampler &r) {
+    st8(st.ray + 2 * (size_t)slot, make_float4(o.x, o.y, o.z, __uint_as_float((uint32_t)r.state)),
+        make_float4(d.x, d.y, d.z, __uint_as_float((uint32_t)(r.state >> 32))));
 }
-PT_DI Sampler load_rng(const uint2 *src, uint32_t mode, uint32_t frame_seed) {
+PT_DI Sampler load_rng(float lo, float hi, uint32_t mode, uint32_t frame_seed) {
     Sampler s;
-    uint2 v = *src;
     s.mode = mode;
-    s.state = (uint64_t)v.x | ((uint64_t)v.y << 32);
+    s.state = (uint64_t)__float_as_uint(lo) | ((uint64_t)__float_as_uint(hi) << 32);
     s.inc = (static_cast<uint64_t>(frame_seed) << 1u) | 1u;
     return s;
 }
@@ -196,12 +206,8 @@ __global__ void k_raygen(DevScene s, Batch bt, State st, Wave w) {
         } else {
             raygen_one(s, tile_pixel(r, s.width_px, s.height_px), w.seed0 + w.frame0 + fl, w.rng_mode, o, d, rng);
         }
-        st.ray_o[slot] = make_float4(o.x, o.y, o.z, 0.001f);
-        st.ray_d[slot] = make_float4(d.x, d.y, d.z, 1e16f);
-        st.thr[slot] = make_float4(1.f, 1.f, 1.f, 0.f);
-        st.rad[slot] = make_float4(0.f, 0.f, 0.f, 0.f);
-        save_rng(st.rng + slot, rng);
-        st.meta[slot] = 0;
+        store_ray(st, slot, o, d, rng);
+        if (w.bounces == 0) st.rad[slot] = make_float4(0.f, 0.f, 0.f, 0.f);  // else the first bounce starts it
         st.q_in[slot] = slot;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -228,17 +234,16 @@ PT_DI size_t smem_node_bytes(const DevScene &s) {
 }
 
 // Ray sources / result sinks of the persistent traversal.
-struct ExtendSrc {  // closest hit of the active queue (entries are path slots)
+struct ExtendSrc {  // closest hit of the active queue
     State st;
     PT_DI int root(uint32_t) const { return 0; }
     PT_DI uint32_t count() const { return st.counters[kNIn]; }
-    PT_DI void load(uint32_t i, float3 &o, float3 &d, float &tmin, float &tmax, uint32_t &tag) const {
-        uint32_t slot = ld_stream(st.q_in + i);
-        float4 o4 = ld_stream(st.ray_o + slot), d4 = ld_stream(st.ray_d + slot);
+    PT_DI void load(uint32_t i, float3 &o, float3 &d, float &, float &, uint32_t &tag) const {
+        const uint32_t slot = entry_slot(ld_stream(st.q_in + i));
+        float4 o4, d4;
+        ld_stream8(st.ray + 2 * (size_t)slot, o4, d4);
         o = xyz(o4);
         d = xyz(d4);
-        tmin = o4.w;
-        tmax = d4.w;
         tag = slot;
     }
     PT_DI void store(uint32_t, uint32_t slot, const TraceResult &r) const {
@@ -391,7 +396,7 @@ PT_DI void hit_geometry(const DevScene &s, float4 h, float3 o, float3 d, const D
 
 // One bounce of shading for every entry of the active queue.
 struct ShadeOut {
-    bool push_ext = false, push_sh = false;
+    bool push_ext = false, push_sh = false, delta = false;
     float3 hit_pos = f3s(0.f), sh_d = f3s(0.f), sh_c = f3s(0.f);
     float sh_tmax = 0.f;
 };
@@ -399,26 +404,33 @@ struct ShadeOut {
 // One path slot of k_shade: frame fl of the wave, pixel r (tile order) of scene s.
 // The radiance slot is read and written only when the bounce adds to it (a
 // miss, or a hit on an emitter): most bounces do not.
-PT_DI void shade_one(const DevScene &s, const Outputs &out, const State &st, const Wave &w, uint32_t slot, uint32_t fl,
+PT_DI void shade_one(const DevScene &s, const Outputs &out, const State &st, const Wave &w, uint32_t entry, uint32_t fl,
                      uint32_t r, float env_pdf, ShadeOut &so) {
     float3 new_d = f3s(0.f);
-    uint32_t meta = st.meta[slot];
-    uint32_t depth = meta & 0xffffu;
-    bool prev_delta = (meta >> 16) & 1u;
+    const uint32_t slot = entry_slot(entry);
+    const bool first = w.bounce == 0;  // no throughput or radiance stored yet
+    uint32_t depth = w.bounce;
+    bool prev_delta = (entry & kEntryDelta) != 0;
     uint32_t frame = w.frame0 + fl;
-    const bool first_of_last = depth == 0 && frame == w.last_frame;  // this sample writes the AOVs
+    const bool first_of_last = first && frame == w.last_frame;  // this sample writes the AOVs
     const uint32_t p = first_of_last ? tile_pixel(r, s.width_px, s.height_px) : 0u;
     float4 h = st.hit[slot];
-    float3 ro = xyz(st.ray_o[slot]), rd = xyz(st.ray_d[slot]);
-    float4 t4 = st.thr[slot];
+    float4 o4, d4;
+    ld8(st.ray + 2 * (size_t)slot, o4, d4);
+    const float3 ro = xyz(o4), rd = xyz(d4);
+    const float4 t4 = first ? make_float4(1.f, 1.f, 1.f, 0.f) : st.thr[slot];
     float3 thr = xyz(t4);
     float prev_pdf = t4.w;
+    float3 first_rad = f3s(0.f);
     const auto add_radiance = [&](float3 c) {
-        const float4 r4 = st.rad[slot];
-        const float3 rad = xyz(r4) + c;
-        st.rad[slot] = make_float4(rad.x, rad.y, rad.z, r4.w);
+        if (first) {
+            first_rad = first_rad + c;
+            return;
+        }
+        const float3 rad = xyz(st.rad[slot]) + c;
+        st.rad[slot] = make_float4(rad.x, rad.y, rad.z, 0.f);
     };
-    Sampler rng = load_rng(st.rng + slot, w.rng_mode, w.seed0 + frame);
+    Sampler rng = load_rng(o4.w, d4.w, w.rng_mode, w.seed0 + frame);
     int prim = __float_as_int(h.y);
     bool alive = prim >= 0;
     HitGeo g;
@@ -429,7 +441,7 @@ PT_DI void shade_one(const DevScene &s, const Outputs &out, const State &st, con
             float epdf = env_pdf;
             if (emitter_type(s.env) == kEmitEnvMap) envmap_eval(s.envmap, ro, normalize(rd), le, epdf);
             else le = xyz(s.env.rad);
-            add_radiance(depth == 0 ? le : le * (thr * mis_weight(prev_pdf, epdf)));
+            add_radiance(first ? le : le * (thr * mis_weight(prev_pdf, epdf)));
         }
         if (first_of_last) {
             if (out.albedo) { out.albedo[3 * p] = 0.f; out.albedo[3 * p + 1] = 0.f; out.albedo[3 * p + 2] = 0.f; }
@@ -441,7 +453,7 @@ PT_DI void shade_one(const DevScene &s, const Outputs &out, const State &st, con
         hit_geometry(s, h, ro, rd, in, m.twosided != 0, g);
         bsdf = material_local(m, g.uv);
         int ei = in.emitter_offset >= 0 ? in.emitter_offset + (prim - (int)in.prim_offset) : -1;
-        if (depth == 0) {  // main.cu:90-98
+        if (first) {  // main.cu:90-98
             if (ei >= 0) add_radiance(emitter_radiance(s.emitters[ei], s.emit_tex, g.uv));
             if (first_of_last) {
                 float3 al = bsdf.albedo();
@@ -457,7 +469,7 @@ PT_DI void shade_one(const DevScene &s, const Outputs &out, const State &st, con
             }
         }
     }
-    if (depth == 0) {  // main.cu:104
+    if (first) {  // main.cu:104
         float tv = rng.next();
         if (first_of_last && out.test) out.test[p] = tv;
     }
@@ -515,23 +527,25 @@ PT_DI void shade_one(const DevScene &s, const Outputs &out, const State &st, con
             thr = thr * (br.f * fabsf(br.wi.z) / br.pdf);
             new_d = to_world(br.wi, g.nrm);
             prev_pdf = br.pdf;
-            prev_delta = (br.type & kDelta) != 0;
+            so.delta = (br.type & kDelta) != 0;
             so.push_ext = true;
         }
     }
     if (prim >= 0) so.hit_pos = g.pos;
+    if (first) st.rad[slot] = make_float4(first_rad.x, first_rad.y, first_rad.z, 0.f);
     if (alive) {
         st.thr[slot] = make_float4(thr.x, thr.y, thr.z, prev_pdf);
-        st.meta[slot] = depth | (prev_delta ? (1u << 16) : 0u);
-        save_rng(st.rng + slot, rng);
-        st.ray_o[slot] = make_float4(so.hit_pos.x, so.hit_pos.y, so.hit_pos.z, 0.001f);
-        st.ray_d[slot] = make_float4(new_d.x, new_d.y, new_d.z, 1e16f);
+        store_ray(st, slot, so.hit_pos, new_d, rng);
     }
 }
 
+// Bound by the latency of its gathers (path state, vertices, tables): 4 blocks
+// of 256 threads per SM (64 registers, 332 bytes of spills) hide more of it
+// than 3 (80 registers) or 2 (no spills): 22.8 / 23.4 / 26.2 ms a 64-spp 1080p
+// frame of the 1M-triangle field, 0.209 / 0.226 / 0.246 ms on the Cornell box.
+// 32.7 ms with a path's ray, stream and flags in separate 4- to 16-byte arrays.
 template <bool BATCH>
-// 3 blocks of 256 threads per SM: at most 85 registers per thread.
-__global__ void __launch_bounds__(256, 3) k_shade(DevScene s, Batch bt, State st, Wave w, Outputs out) {
+__global__ void __launch_bounds__(256, 4) k_shade(DevScene s, Batch bt, State st, Wave w, Outputs out) {
     __shared__ uint32_t push_smem[72];
     const uint32_t n = st.counters[kNIn];
     const float env_pdf = 0.25f * kInvPi;  // ConstEnvEmitter::Eval (env.h:82-85)
@@ -541,18 +555,19 @@ __global__ void __launch_bounds__(256, 3) k_shade(DevScene s, Batch bt, State st
         uint32_t slot = 0;
         ShadeOut so;
         if (valid) {
-            slot = st.q_in[i];
+            const uint32_t entry = st.q_in[i];
+            slot = entry_slot(entry);
             const uint32_t r = slot / w.frames, fl = slot - r * w.frames;
             if (BATCH) {
                 const uint32_t k = batch_scene(bt, r);
-                shade_one(bt.scenes[k], bt.outs[k], st, w, slot, fl, r - bt.pix_off[k], env_pdf, so);
+                shade_one(bt.scenes[k], bt.outs[k], st, w, entry, fl, r - bt.pix_off[k], env_pdf, so);
             } else {
-                shade_one(s, out, st, w, slot, fl, r, env_pdf, so);
+                shade_one(s, out, st, w, entry, fl, r, env_pdf, so);
             }
         }
         uint32_t pos_ext, pos_sh;
         block_push2(so.push_ext, so.push_sh, st.counters + kNOut, st.counters + kNShadow, pos_ext, pos_sh, push_smem);
-        if (so.push_ext) st.q_out[pos_ext] = slot;
+        if (so.push_ext) st.q_out[pos_ext] = slot | (so.delta ? kEntryDelta : 0u);
         if (so.push_sh) {  // shadow ray from the hit point, tmin 1e-4, tmax distance - 1e-4 (main.cu:122-126)
             st.sh_o[pos_sh] = make_float4(so.hit_pos.x, so.hit_pos.y, so.hit_pos.z, 0.0001f);
             st.sh_d[pos_sh] = make_float4(so.sh_d.x, so.sh_d.y, so.sh_d.z, so.sh_tmax);
@@ -591,7 +606,7 @@ __global__ void k_bin_count(DevScene s, State st, uint8_t *keys, uint32_t *block
     uint32_t lo, hi;
     bin_stretch(st.counters[kNIn], lo, hi);
     for (uint32_t i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-        uint32_t slot = st.q_in[i];
+        const uint32_t slot = entry_slot(st.q_in[i]);
         int prim = __float_as_int(st.hit[slot].y);
         const uint32_t key = material_bin(s, prim);
         keys[i] = (uint8_t)key;
@@ -675,7 +690,7 @@ __global__ void k_bin_count_batch(Batch bt, uint32_t frames, State st, uint16_t 
     __syncthreads();
     const uint32_t n = st.counters[kNIn];
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t slot = st.q_in[i];
+        const uint32_t slot = entry_slot(st.q_in[i]);
         const int prim = __float_as_int(st.hit[slot].y);
         const uint32_t sc = batch_scene(bt, slot / frames);
         const uint32_t key = sc * kNumBins + material_bin(bt.scenes[sc], prim);
@@ -925,9 +940,9 @@ struct Launcher {
         }
         if (ws.capacity < cap) {
             int e;
-            if ((e = ws.ray_o.ensure(16 * cap)) || (e = ws.ray_d.ensure(16 * cap)) || (e = ws.hit.ensure(16 * cap)) ||
-                (e = ws.thr.ensure(16 * cap)) || (e = ws.rad.ensure(16 * cap)) || (e = ws.rng.ensure(8 * cap)) ||
-                (e = ws.meta.ensure(4 * cap)) || (e = ws.q0.ensure(4 * cap)) || (e = ws.q1.ensure(4 * cap)) ||
+            if ((e = ws.ray.ensure(32 * cap)) || (e = ws.hit.ensure(16 * cap)) ||
+                (e = ws.thr.ensure(16 * cap)) || (e = ws.rad.ensure(16 * cap)) ||
+                (e = ws.q0.ensure(4 * cap)) || (e = ws.q1.ensure(4 * cap)) ||
                 (e = ws.sh_o.ensure(16 * cap)) || (e = ws.sh_d.ensure(16 * cap)) || (e = ws.sh_c.ensure(16 * cap)))
                 return e;
             ws.capacity = cap;
@@ -935,13 +950,10 @@ struct Launcher {
         int e = ws.counters.ensure(256);
         if (e != PT_OK) return e;
         State stt;
-        stt.ray_o = ws.ray_o.as<float4>();
-        stt.ray_d = ws.ray_d.as<float4>();
+        stt.ray = ws.ray.as<float4>();
         stt.hit = ws.hit.as<float4>();
         stt.thr = ws.thr.as<float4>();
         stt.rad = ws.rad.as<float4>();
-        stt.rng = ws.rng.as<uint2>();
-        stt.meta = ws.meta.as<uint32_t>();
         stt.sh_o = ws.sh_o.as<float4>();
         stt.sh_d = ws.sh_d.as<float4>();
         stt.sh_c = ws.sh_c.as<float4>();
@@ -1006,6 +1018,8 @@ struct Launcher {
             w.max_depth = max_depth;
             w.rng_mode = p->rng;
             w.accumulate = p->accumulate;
+            w.bounce = 0;
+            w.bounces = bounces;
             stt.q_in = ws.q0.as<uint32_t>();
             stt.q_out = ws.q1.as<uint32_t>();
             const size_t slots = (size_t)w.frames * npix;
@@ -1016,6 +1030,7 @@ struct Launcher {
             }
             launches++;
             for (uint32_t b = 0; b < bounces; b++) {
+                w.bounce = b;
                 pt_nvtx::Range nv_bounce("bounce");
                 if (timing) tm.mark(0, ls);
                 {
@@ -1203,7 +1218,7 @@ void pt_batch_release(BatchWorkspace *b) {
     DevBuf *bufs[] = {&b->nodes, &b->cnodes, &b->prims, &b->scenes, &b->outs, &b->pix_off, &b->roots, &b->bins};
     for (DevBuf *d : bufs) d->release();
     RenderWorkspace &w = b->ws;
-    DevBuf *wb[] = {&w.ray_o, &w.ray_d, &w.hit, &w.thr, &w.rad, &w.rng, &w.meta, &w.q0,
+    DevBuf *wb[] = {&w.ray, &w.hit, &w.thr, &w.rad, &w.q0,
                     &w.q1, &w.sh_o, &w.sh_d, &w.sh_c, &w.mat_key, &w.counters, &w.sort_tmp, &w.bin_blocks};
     for (DevBuf *d : wb) d->release();
     if (w.exec) cudaGraphExecDestroy(w.exec);
@@ -1478,10 +1493,10 @@ namespace {
 
 constexpr uint32_t kNoAllocMaxPixels = 1u << 16;  // 65,536 path slots
 constexpr size_t kNoAllocCounterBytes = 256;
-constexpr size_t kNoAllocSlotBytes = 16 * 8 + 8 + 4 * 3;  // 8 float4 arrays, rng, meta, two queues = 148 B
+constexpr size_t kNoAllocSlotBytes = 32 + 16 * 6 + 4 * 2;  // ray, 6 float4 arrays, two queues = 136 B
 constexpr size_t kNoAllocScratchBytes = kNoAllocCounterBytes + kNoAllocSlotBytes * kNoAllocMaxPixels;
 
-// About 9.3 MiB, held by every GPU that loads the library until the process exits.
+// About 8.5 MiB, held by every GPU that loads the library until the process exits.
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
 
 std::mutex g_noalloc_mutex;
@@ -1525,16 +1540,13 @@ int render_noalloc(pt_scene *s, const pt_render_params *p, const pt_frame_buffer
     };
     stt.counters = reinterpret_cast<uint32_t *>(scratch);
     stt.stats = reinterpret_cast<unsigned long long *>(stt.counters + kStatBase);
-    stt.ray_o = reinterpret_cast<float4 *>(take(16));
-    stt.ray_d = reinterpret_cast<float4 *>(take(16));
+    stt.ray = reinterpret_cast<float4 *>(take(32));
     stt.hit = reinterpret_cast<float4 *>(take(16));
     stt.thr = reinterpret_cast<float4 *>(take(16));
     stt.rad = reinterpret_cast<float4 *>(take(16));
     stt.sh_o = reinterpret_cast<float4 *>(take(16));
     stt.sh_d = reinterpret_cast<float4 *>(take(16));
     stt.sh_c = reinterpret_cast<float4 *>(take(16));
-    stt.rng = reinterpret_cast<uint2 *>(take(8));
-    stt.meta = reinterpret_cast<uint32_t *>(take(4));
     uint32_t *q0 = reinterpret_cast<uint32_t *>(take(4));
     uint32_t *q1 = reinterpret_cast<uint32_t *>(take(4));
     Outputs out;
@@ -1575,10 +1587,13 @@ int render_noalloc(pt_scene *s, const pt_render_params *p, const pt_frame_buffer
         w.max_depth = max_depth;
         w.rng_mode = p->rng;
         w.accumulate = p->accumulate;
+        w.bounce = 0;
+        w.bounces = max_depth;
         stt.q_in = q0;
         stt.q_out = q1;
         k_raygen<false><<<nblocks((size_t)w.frames * npix, 256), 256, 0, st>>>(d, Batch{}, stt, w);
         for (uint32_t b = 0; b < max_depth; b++) {
+            w.bounce = b;
             k_ext<<<grid_trace, tb, smem, st>>>(d, stt, Batch{}, w.frames);
             k_shade<false><<<grid_shade, 256, 0, st>>>(d, Batch{}, stt, w, out);
             k_sh<<<grid_shadow, tb, smem_sh, st>>>(d, stt, Batch{}, w.frames);

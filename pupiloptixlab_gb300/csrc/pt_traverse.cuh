@@ -273,6 +273,25 @@ PT_DI void ld_bvh8(const float4 *p, float *f) {
         : "l"(p));
 }
 
+// 32 bytes of ray state, streaming (evict-first), and the same store.
+PT_DI void ld_stream8(const float4 *p, float4 &a, float4 &b) {
+    asm volatile("ld.global.L1::evict_first.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                 : "l"(p)
+                 : "memory");
+}
+PT_DI void ld8(const float4 *p, float4 &a, float4 &b) {
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                 : "l"(p)
+                 : "memory");
+}
+PT_DI void st8(float4 *p, float4 a, float4 b) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(a.z),
+                 "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+                 : "memory");
+}
+
 template <typename T>
 PT_DI T ld_stream(const T *p) {
     return __ldcs(p);
@@ -482,7 +501,8 @@ constexpr int kNodeWaitMax = 8;
 // which is re-checked against the current closest hit when popped.
 //
 // Src provides: count(), load(i, o, d, tmin, tmax, tag), root(tag) (the node
-// the ray starts at), store(i, tag, result).
+// the ray starts at), store(i, tag, result).  A load that leaves tmin and tmax
+// alone (extension rays: always 0.001 and 1e16) keeps them out of registers.
 // CURVES = false compiles the leaf test without the curve-piece branch (a
 // record with non-zero kind bits is then treated as a sphere), so that scenes
 // without curves run the smaller kernel.
@@ -504,7 +524,7 @@ PT_DI void trace_persistent(const DevScene &s, const float4 *snodes, void *sstac
     bool fma_slab = false;
     int oct = 0;  // direction octant (compressed 8-wide nodes)
     RayWT w{0, 1, 2, 0.f, 0.f, 1.f};
-    float tmin = 0.f, tmax = 0.f;
+    float tmin = 0.001f, tmax = 1e16f;  // the extension rays' range (main.cu:80-85)
     TraceResult best{0.f, -1, 0.f, 0.f};
     int item = kNoItem, leaf = kNoItem;
     uint32_t nodes = 0, prims = 0, rays = 0, ovf = 0;
