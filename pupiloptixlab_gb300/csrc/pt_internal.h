@@ -78,6 +78,10 @@ struct RenderWorkspace {
     // and before the caller's stream, and the instantiated graph.
     cudaStream_t stream = nullptr;
     cudaEvent_t ev_in = nullptr, ev_out = nullptr;
+    // the captured render's second branch: a bounce's shadow rays beside the
+    // next bounce's extension rays
+    cudaStream_t side = nullptr;
+    cudaEvent_t ev_shade = nullptr, ev_shadow = nullptr;
     cudaGraphExec_t exec = nullptr;
 };
 
@@ -92,6 +96,7 @@ struct pt_scene {
     uint32_t num_vertices = 0;
     std::vector<MeshInstanceRef> mesh_instances;
     std::vector<uint32_t> mesh_num_vertices;
+    bool one_bsdf = false;  // every instance's material is of one type
     float scene_mag = 1.f;  // max |coordinate| of the scene bounds and the camera
 
     // host copies used by refit / updates

@@ -35,16 +35,18 @@ using namespace ptd;
 // state; 64 frames of 1080p in one wave: fewer, fuller launches per bounce).
 constexpr uint32_t kDefaultWavePaths = 128u << 20;
 
+// Counters (32-bit words).  A call's: overflow, non-finite samples, statistics.
+// Then one set per bounce (a 32-byte sector each), so that the shadow rays of a
+// bounce can run beside the next bounce's extension rays; sets are cleared
+// before their wave, or, where fewer sets than bounces exist, taken in turn
+// and cleared one bounce ahead (k_advance).
 enum Counter : int {
-    kNIn = 0,
-    kNOut = 1,
-    kNShadow = 2,
-    kWorkExtend = 3,
-    kWorkShadow = 4,
     kOverflow = 5,
     kNonFinite = 6,  // samples whose radiance was NaN or infinite
-    kStatBase = 8,  // uint64 statistics start at counters + 8 (32-byte offset)
+    kStatBase = 8,   // uint64 statistics start at counters + 8 (32-byte offset)
 };
+constexpr uint32_t kFirstSet = 24, kSetWords = 8;
+enum SetCounter : int { kNIn = 0, kNShadow, kWorkExtend, kWorkShadow };
 enum Stat : int { kStatExtNodes = 0, kStatExtPrims, kStatShNodes, kStatShPrims, kStatExtRays, kStatShRays, kNumStats };
 
 struct Wave {
@@ -74,6 +76,7 @@ struct State {
     uint32_t *q_in, *q_out;  // path slot | kEntryDelta
     float4 *sh_o, *sh_d, *sh_c;
     uint32_t *counters;
+    uint32_t *cur, *next;  // counter sets of this bounce and the next
     unsigned long long *stats;
 };
 constexpr uint32_t kEntryDelta = 1u << 31;  // slots are below 2^31
@@ -210,22 +213,13 @@ __global__ void k_raygen(DevScene s, Batch bt, State st, Wave w) {
         if (w.bounces == 0) st.rad[slot] = make_float4(0.f, 0.f, 0.f, 0.f);  // else the first bounce starts it
         st.q_in[slot] = slot;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        st.counters[kNIn] = total;
-        st.counters[kNOut] = 0;
-        st.counters[kNShadow] = 0;
-        st.counters[kWorkExtend] = 0;
-        st.counters[kWorkShadow] = 0;
-    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) st.cur[kNIn] = total;
 }
 
-// Queue hand-over between bounces: the next active queue becomes the input.
-__global__ void k_advance(uint32_t *counters) {
-    counters[kNIn] = counters[kNOut];
-    counters[kNOut] = 0;
-    counters[kNShadow] = 0;
-    counters[kWorkExtend] = 0;
-    counters[kWorkShadow] = 0;
+// Clears a counter set for the bounce after this one (its last users, the
+// bounce before the previous one's, are done).
+__global__ void k_advance(uint32_t *next) {
+    if (threadIdx.x < kSetWords) next[threadIdx.x] = 0;
 }
 
 template <int K>
@@ -237,7 +231,7 @@ PT_DI size_t smem_node_bytes(const DevScene &s) {
 struct ExtendSrc {  // closest hit of the active queue
     State st;
     PT_DI int root(uint32_t) const { return 0; }
-    PT_DI uint32_t count() const { return st.counters[kNIn]; }
+    PT_DI uint32_t count() const { return st.cur[kNIn]; }
     PT_DI void load(uint32_t i, float3 &o, float3 &d, float &, float &, uint32_t &tag) const {
         const uint32_t slot = entry_slot(ld_stream(st.q_in + i));
         float4 o4, d4;
@@ -253,7 +247,7 @@ struct ExtendSrc {  // closest hit of the active queue
 struct ShadowSrc {  // any hit of the shadow queue; unoccluded rays add their NEE radiance
     State st;
     PT_DI int root(uint32_t) const { return 0; }
-    PT_DI uint32_t count() const { return st.counters[kNShadow]; }
+    PT_DI uint32_t count() const { return st.cur[kNShadow]; }
     PT_DI void load(uint32_t i, float3 &o, float3 &d, float &tmin, float &tmax, uint32_t &tag) const {
         float4 o4 = ld_stream(st.sh_o + i), d4 = ld_stream(st.sh_d + i);
         o = xyz(o4);
@@ -326,11 +320,11 @@ __global__ void __maxnreg__(K == 8 ? 96 : 72) k_trace_queue(DevScene s, State st
             src.st = st;
             src.bt = bt;
             src.frames = frames;
-            trace_persistent<K, true, COUNT, decltype(src), CURVES>(s, smem, sstack, src, st.counters + kWorkShadow, st.counters + kOverflow,
+            trace_persistent<K, true, COUNT, decltype(src), CURVES>(s, smem, sstack, src, st.cur + kWorkShadow, st.counters + kOverflow,
                                              st.stats + kStatShNodes, st.stats + kStatShPrims, st.stats + kStatShRays);
         } else {
             ShadowSrc src{st};
-            trace_persistent<K, true, COUNT, decltype(src), CURVES>(s, smem, sstack, src, st.counters + kWorkShadow, st.counters + kOverflow,
+            trace_persistent<K, true, COUNT, decltype(src), CURVES>(s, smem, sstack, src, st.cur + kWorkShadow, st.counters + kOverflow,
                                              st.stats + kStatShNodes, st.stats + kStatShPrims, st.stats + kStatShRays);
         }
     } else {
@@ -339,11 +333,11 @@ __global__ void __maxnreg__(K == 8 ? 96 : 72) k_trace_queue(DevScene s, State st
             src.st = st;
             src.bt = bt;
             src.frames = frames;
-            trace_persistent<K, false, COUNT, decltype(src), CURVES>(s, smem, sstack, src, st.counters + kWorkExtend, st.counters + kOverflow,
+            trace_persistent<K, false, COUNT, decltype(src), CURVES>(s, smem, sstack, src, st.cur + kWorkExtend, st.counters + kOverflow,
                                               st.stats + kStatExtNodes, st.stats + kStatExtPrims, st.stats + kStatExtRays);
         } else {
             ExtendSrc src{st};
-            trace_persistent<K, false, COUNT, decltype(src), CURVES>(s, smem, sstack, src, st.counters + kWorkExtend, st.counters + kOverflow,
+            trace_persistent<K, false, COUNT, decltype(src), CURVES>(s, smem, sstack, src, st.cur + kWorkExtend, st.counters + kOverflow,
                                               st.stats + kStatExtNodes, st.stats + kStatExtPrims, st.stats + kStatExtRays);
         }
     }
@@ -547,7 +541,7 @@ PT_DI void shade_one(const DevScene &s, const Outputs &out, const State &st, con
 template <bool BATCH>
 __global__ void __launch_bounds__(256, 4) k_shade(DevScene s, Batch bt, State st, Wave w, Outputs out) {
     __shared__ uint32_t push_smem[72];
-    const uint32_t n = st.counters[kNIn];
+    const uint32_t n = st.cur[kNIn];
     const float env_pdf = 0.25f * kInvPi;  // ConstEnvEmitter::Eval (env.h:82-85)
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
         uint32_t i = base + threadIdx.x;
@@ -566,7 +560,7 @@ __global__ void __launch_bounds__(256, 4) k_shade(DevScene s, Batch bt, State st
             }
         }
         uint32_t pos_ext, pos_sh;
-        block_push2(so.push_ext, so.push_sh, st.counters + kNOut, st.counters + kNShadow, pos_ext, pos_sh, push_smem);
+        block_push2(so.push_ext, so.push_sh, st.next + kNIn, st.cur + kNShadow, pos_ext, pos_sh, push_smem);
         if (so.push_ext) st.q_out[pos_ext] = slot | (so.delta ? kEntryDelta : 0u);
         if (so.push_sh) {  // shadow ray from the hit point, tmin 1e-4, tmax distance - 1e-4 (main.cu:122-126)
             st.sh_o[pos_sh] = make_float4(so.hit_pos.x, so.hit_pos.y, so.hit_pos.z, 0.0001f);
@@ -604,7 +598,7 @@ __global__ void k_bin_count(DevScene s, State st, uint8_t *keys, uint32_t *block
     if (threadIdx.x < kNumBins) h[threadIdx.x] = 0;
     __syncthreads();
     uint32_t lo, hi;
-    bin_stretch(st.counters[kNIn], lo, hi);
+    bin_stretch(st.cur[kNIn], lo, hi);
     for (uint32_t i = lo + threadIdx.x; i < hi; i += blockDim.x) {
         const uint32_t slot = entry_slot(st.q_in[i]);
         int prim = __float_as_int(st.hit[slot].y);
@@ -655,7 +649,7 @@ __global__ void k_bin_scatter(State st, const uint8_t *keys, const uint32_t *blo
     if (threadIdx.x < kWarps * kNumBins) wc[threadIdx.x / kNumBins][threadIdx.x % kNumBins] = 0;
     __syncthreads();
     uint32_t lo, hi;
-    bin_stretch(st.counters[kNIn], lo, hi);
+    bin_stretch(st.cur[kNIn], lo, hi);
     for (uint32_t base = lo; base < hi; base += blockDim.x) {  // uniform per block
         const uint32_t i = base + threadIdx.x;
         const bool valid = i < hi;
@@ -688,7 +682,7 @@ __global__ void k_bin_count_batch(Batch bt, uint32_t frames, State st, uint16_t 
     extern __shared__ uint32_t hb[];
     for (uint32_t k = threadIdx.x; k < bt.nbins; k += blockDim.x) hb[k] = 0;
     __syncthreads();
-    const uint32_t n = st.counters[kNIn];
+    const uint32_t n = st.cur[kNIn];
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t slot = entry_slot(st.q_in[i]);
         const int prim = __float_as_int(st.hit[slot].y);
@@ -738,7 +732,7 @@ __global__ void k_bin_scatter_batch(Batch bt, State st, const uint16_t *keys, ui
     uint32_t *cnt = sbins, *start = sbins + bt.nbins;
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    const uint32_t n = st.counters[kNIn];
+    const uint32_t n = st.cur[kNIn];
     uint32_t *cursor = bt.bins + bt.nbins;
     for (uint32_t blk = blockIdx.x * blockDim.x; blk < n; blk += gridDim.x * blockDim.x) {  // uniform per block
         for (uint32_t k = threadIdx.x; k < bt.nbins; k += blockDim.x) cnt[k] = 0;
@@ -892,6 +886,7 @@ struct RunTarget {
     int num_sms;
     uint32_t tuned_block, tuned_wave_paths;
     pt_render_stats *rs;
+    bool one_bsdf;  // one material type: binning by material orders nothing
     bool curves;  // some scene has curve pieces: use the traversal with the curve test
 };
 
@@ -910,7 +905,7 @@ template <int K>
 struct Launcher {
     static int run(pt_scene *s, const pt_render_params *p, const pt_frame_buffers *fb, cudaStream_t st) {
         RunTarget t{&s->ws, s->ev0, s->ev1, s->num_sms, s->tuned_block, s->tuned_wave_paths, &s->render_stats,
-                    s->num_curve_pieces > 0};
+                    s->one_bsdf, s->num_curve_pieces > 0};
         const uint32_t max_depth = p->max_depth ? p->max_depth : s->desc_shallow.max_depth;
         const uint32_t npix = s->dev.width_px * s->dev.height_px;
         return run_waves<false>(t, s->dev, Batch{}, npix, max_depth, max_depth, p, make_outputs(fb, p->flags), st);
@@ -947,7 +942,9 @@ struct Launcher {
                 return e;
             ws.capacity = cap;
         }
-        int e = ws.counters.ensure(256);
+        const size_t set_bytes = 4 * (size_t)kSetWords * (bounces + 1);
+        const size_t counter_bytes = 4 * kFirstSet + set_bytes;
+        int e = ws.counters.ensure(std::max<size_t>(counter_bytes, 256));
         if (e != PT_OK) return e;
         State stt;
         stt.ray = ws.ray.as<float4>();
@@ -976,7 +973,7 @@ struct Launcher {
         const uint32_t grid_shadow = (uint32_t)std::max(1, occ_h) * t.num_sms;
         const uint32_t grid_shade = (uint32_t)std::max(1, occ_s) * t.num_sms;
 
-        const bool sort = (p->flags & PT_RENDER_NO_MATERIAL_SORT) == 0;
+        const bool sort = (p->flags & PT_RENDER_NO_MATERIAL_SORT) == 0 && !t.one_bsdf;
         if (sort && ws.sort_capacity < cap) {
             if ((e = ws.mat_key.ensure(2 * cap)) != PT_OK || (e = ws.sort_tmp.ensure(4 * cap)) != PT_OK) return e;
             ws.sort_capacity = cap;
@@ -988,12 +985,21 @@ struct Launcher {
 
         // The whole render is captured into a CUDA graph on the scene's own
         // stream (ordered after and before the caller's stream by events) and
-        // replayed; later calls update the instantiated graph in place.
+        // replayed; later calls update the instantiated graph in place.  The
+        // graph has a second branch: a bounce's shadow rays run beside the next
+        // bounce's extension rays and binning (they meet before shading, which
+        // adds to the same radiance), so that the last long rays of one kernel
+        // do not leave the chip idle: 1M-triangle field at 1080p, 1 spp 4.27 ->
+        // 3.56 ms, 13-launch Cornell preview 0.23 -> 0.135 ms.  Two halves of a
+        // wave as parallel chains were slower (4.78 ms), stream priorities equal.
         const bool graph = (p->flags & (PT_RENDER_NO_GRAPH | PT_RENDER_KERNEL_TIMING)) == 0;
         if (graph && !ws.stream) {
             PT_CUDA_TRY(cudaStreamCreateWithFlags(&ws.stream, cudaStreamNonBlocking));
             PT_CUDA_TRY(cudaEventCreateWithFlags(&ws.ev_in, cudaEventDisableTiming));
             PT_CUDA_TRY(cudaEventCreateWithFlags(&ws.ev_out, cudaEventDisableTiming));
+            PT_CUDA_TRY(cudaStreamCreateWithFlags(&ws.side, cudaStreamNonBlocking));
+            PT_CUDA_TRY(cudaEventCreateWithFlags(&ws.ev_shade, cudaEventDisableTiming));
+            PT_CUDA_TRY(cudaEventCreateWithFlags(&ws.ev_shadow, cudaEventDisableTiming));
         }
         cudaStream_t ls = graph ? ws.stream : st;
         if (graph) {
@@ -1006,7 +1012,12 @@ struct Launcher {
         uint32_t waves = 0;
         pt_nvtx::Range nv_render(graph ? "pt_render: capture" : "pt_render: launches");
         if (!graph) PT_CUDA_TRY(cudaEventRecord(t.ev0, st));
-        cudaError_t enq = cudaMemsetAsync(ws.counters.ptr, 0, 256, ls);
+        cudaError_t enq = cudaMemsetAsync(ws.counters.ptr, 0, counter_bytes, ls);
+        const auto order = [&](cudaStream_t from, cudaStream_t to, cudaEvent_t ev) {  // `to` continues after `from`
+            if (from == to || enq != cudaSuccess) return;
+            enq = cudaEventRecord(ev, from);
+            if (enq == cudaSuccess) enq = cudaStreamWaitEvent(to, ev, 0);
+        };
         for (uint32_t f0 = 0; f0 < p->spp && enq == cudaSuccess; f0 += frames_per_wave) {
             Wave w;
             w.npix = npix;
@@ -1020,17 +1031,26 @@ struct Launcher {
             w.accumulate = p->accumulate;
             w.bounce = 0;
             w.bounces = bounces;
+            const size_t slots = (size_t)w.frames * npix;
+            uint32_t *sets = stt.counters + kFirstSet;
             stt.q_in = ws.q0.as<uint32_t>();
             stt.q_out = ws.q1.as<uint32_t>();
-            const size_t slots = (size_t)w.frames * npix;
+            stt.cur = sets;
+            stt.next = sets;
             pt_nvtx::Range nv_wave("wave");
+            if (f0) enq = cudaMemsetAsync(sets, 0, set_bytes, ls);
             {
                 pt_nvtx::Range r("raygen");
                 k_raygen<BATCH><<<nblocks(slots, 256), 256, 0, ls>>>(d, bt, stt, w);
             }
             launches++;
-            for (uint32_t b = 0; b < bounces; b++) {
+            cudaStream_t ss = graph ? ws.side : ls;  // the shadow rays' branch
+            uint32_t *q_sorted = ws.sort_tmp.as<uint32_t>(), *bin_blocks = ws.bin_blocks.as<uint32_t>();
+            for (uint32_t b = 0; b < bounces && enq == cudaSuccess; b++) {
                 w.bounce = b;
+                stt.cur = sets + (size_t)kSetWords * b;
+                stt.next = stt.cur + kSetWords;
+                const bool last_bounce = b + 1 == bounces;
                 pt_nvtx::Range nv_bounce("bounce");
                 if (timing) tm.mark(0, ls);
                 {
@@ -1038,35 +1058,42 @@ struct Launcher {
                     k_ext<<<grid_trace, tb, smem, ls>>>(d, stt, bt, w.frames);
                 }
                 if (timing) tm.mark(0, ls);
+                launches++;
                 State shade_st = stt;
-                if (sort && BATCH) {
-                    k_bin_count_batch<<<grid_bin, 256, bt.nbins * 4, ls>>>(bt, w.frames, stt, ws.mat_key.as<uint16_t>());
-                    k_bin_scan_batch<<<1, 1024, 0, ls>>>(bt);
-                    k_bin_scatter_batch<<<grid_bin, 256, 2 * bt.nbins * 4, ls>>>(bt, stt, ws.mat_key.as<uint16_t>(),
-                                                                  ws.sort_tmp.as<uint32_t>());
-                    shade_st.q_in = ws.sort_tmp.as<uint32_t>();
-                    launches += 3;
-                } else if (sort) {
-                    k_bin_count<<<grid_bin, 256, 0, ls>>>(d, stt, ws.mat_key.as<uint8_t>(), ws.bin_blocks.as<uint32_t>());
-                    k_bin_scan<<<1, 32 * kNumBins, 0, ls>>>(ws.bin_blocks.as<uint32_t>(), grid_bin);
-                    k_bin_scatter<<<grid_bin, 256, 0, ls>>>(stt, ws.mat_key.as<uint8_t>(), ws.bin_blocks.as<uint32_t>(),
-                                                            ws.sort_tmp.as<uint32_t>());
-                    shade_st.q_in = ws.sort_tmp.as<uint32_t>();
+                if (sort && !last_bounce) {  // the last bounce evaluates no BSDF
+                    if (BATCH) {
+                        uint16_t *keys = ws.mat_key.as<uint16_t>();
+                        k_bin_count_batch<<<grid_bin, 256, bt.nbins * 4, ls>>>(bt, w.frames, stt, keys);
+                        k_bin_scan_batch<<<1, 1024, 0, ls>>>(bt);
+                        k_bin_scatter_batch<<<grid_bin, 256, 2 * bt.nbins * 4, ls>>>(bt, stt, keys, q_sorted);
+                    } else {
+                        uint8_t *keys = ws.mat_key.as<uint8_t>();
+                        k_bin_count<<<grid_bin, 256, 0, ls>>>(d, stt, keys, bin_blocks);
+                        k_bin_scan<<<1, 32 * kNumBins, 0, ls>>>(bin_blocks, grid_bin);
+                        k_bin_scatter<<<grid_bin, 256, 0, ls>>>(stt, keys, bin_blocks, q_sorted);
+                    }
+                    shade_st.q_in = q_sorted;
                     launches += 3;
                 }
+                // the previous bounce's shadow rays add to the radiance and read the shadow queue
+                if (b > 0) order(ss, ls, ws.ev_shadow);
                 if (timing) tm.mark(2, ls);
                 {
                     pt_nvtx::Range r("shade (MIS, NEE, BSDF sample)");
                     k_shade<BATCH><<<grid_shade, 256, 0, ls>>>(d, bt, shade_st, w, out);
                 }
-                if (timing) { tm.mark(2, ls); tm.mark(1, ls); }
-                {
-                    pt_nvtx::Range r("shadow (any hit)");
-                    k_sh<<<grid_shadow, tb, smem_sh, ls>>>(d, stt, bt, w.frames);
+                launches++;
+                if (timing) tm.mark(2, ls);
+                if (!last_bounce) {  // the last bounce casts no shadow rays
+                    order(ls, ss, ws.ev_shade);
+                    if (timing) tm.mark(1, ss);
+                    {
+                        pt_nvtx::Range r("shadow (any hit)");
+                        k_sh<<<grid_shadow, tb, smem_sh, ss>>>(d, stt, bt, w.frames);
+                    }
+                    if (timing) tm.mark(1, ss);
+                    launches++;
                 }
-                if (timing) tm.mark(1, ls);
-                k_advance<<<1, 1, 0, ls>>>(stt.counters);
-                launches += 4;
                 std::swap(stt.q_in, stt.q_out);
             }
             {
@@ -1075,7 +1102,7 @@ struct Launcher {
             }
             launches++;
             waves++;
-            enq = cudaGetLastError();
+            if (enq == cudaSuccess) enq = cudaGetLastError();
         }
         if (graph) {
             cudaGraph_t g = nullptr;
@@ -1173,7 +1200,7 @@ struct Launcher {
         uint32_t *c = s->ws.counters.as<uint32_t>();
         PT_CUDA_TRY(cudaMemsetAsync(c, 0, 256, st));
         if (n) kern<<<(uint32_t)std::max(1, occ) * s->num_sms, tb, smem, st>>>(
-            d, reinterpret_cast<const float4 *>(rays), reinterpret_cast<float4 *>(hits), n, c + kWorkExtend, c + kOverflow);
+            d, reinterpret_cast<const float4 *>(rays), reinterpret_cast<float4 *>(hits), n, c + kFirstSet + kWorkExtend, c + kOverflow);
         PT_CUDA_TRY(cudaGetLastError());
         uint32_t ovf = 0;
         PT_CUDA_TRY(cudaMemcpyAsync(&ovf, c + kOverflow, 4, cudaMemcpyDeviceToHost, st));
@@ -1225,6 +1252,9 @@ void pt_batch_release(BatchWorkspace *b) {
     if (w.ev_in) cudaEventDestroy(w.ev_in);
     if (w.ev_out) cudaEventDestroy(w.ev_out);
     if (w.stream) cudaStreamDestroy(w.stream);
+    if (w.side) cudaStreamDestroy(w.side);
+    if (w.ev_shade) cudaEventDestroy(w.ev_shade);
+    if (w.ev_shadow) cudaEventDestroy(w.ev_shadow);
     if (b->ev0) cudaEventDestroy(b->ev0);
     if (b->ev1) cudaEventDestroy(b->ev1);
     delete b;
@@ -1324,7 +1354,7 @@ int render_batch(pt_context *ctx, pt_scene *const *scenes, const pt_render_param
         for (uint32_t k = 0; k < n; k++) bounces = std::max(bounces, scenes[k]->dev.max_depth);
     bool curves = false;
     for (uint32_t k = 0; k < n; k++) curves = curves || scenes[k]->num_curve_pieces > 0;
-    RunTarget t{&b.ws, b.ev0, b.ev1, ctx->num_sms, 0, 0, &b.stats, curves};
+    RunTarget t{&b.ws, b.ev0, b.ev1, ctx->num_sms, 0, 0, &b.stats, false, curves};
     Outputs none{};
     return Launcher<K>::template run_waves<true>(t, dt, bt, static_cast<uint32_t>(total_pix), max_depth, bounces, p,
                                                  none, st);
@@ -1591,13 +1621,17 @@ int render_noalloc(pt_scene *s, const pt_render_params *p, const pt_frame_buffer
         w.bounces = max_depth;
         stt.q_in = q0;
         stt.q_out = q1;
+        stt.cur = stt.counters + kFirstSet;
+        if (f0) PT_CUDA_TRY(cudaMemsetAsync(stt.cur, 0, 3 * kSetWords * 4, st));
         k_raygen<false><<<nblocks((size_t)w.frames * npix, 256), 256, 0, st>>>(d, Batch{}, stt, w);
         for (uint32_t b = 0; b < max_depth; b++) {
             w.bounce = b;
+            stt.cur = stt.counters + kFirstSet + kSetWords * (b % 3);
+            stt.next = stt.counters + kFirstSet + kSetWords * ((b + 1) % 3);
+            if (b > 0) k_advance<<<1, 32, 0, st>>>(stt.next);  // sets 0 and 1 start clear
             k_ext<<<grid_trace, tb, smem, st>>>(d, stt, Batch{}, w.frames);
             k_shade<false><<<grid_shade, 256, 0, st>>>(d, Batch{}, stt, w, out);
-            k_sh<<<grid_shadow, tb, smem_sh, st>>>(d, stt, Batch{}, w.frames);
-            k_advance<<<1, 1, 0, st>>>(stt.counters);
+            if (b + 1 < max_depth) k_sh<<<grid_shadow, tb, smem_sh, st>>>(d, stt, Batch{}, w.frames);  // the last bounce casts none
             std::swap(stt.q_in, stt.q_out);
         }
         k_accumulate<false><<<nblocks(npix, 256), 256, 0, st>>>(stt, w, out, Batch{}, d.width_px, d.height_px);

@@ -578,6 +578,10 @@ int build_scene(pt_scene *s, const pt_scene_desc *d) {
         }
     }
 
+    uint32_t types = 0;  // of the materials that instances use
+    for (uint32_t ii = 0; ii < d->num_instances; ii++) types |= 1u << (mats[insts[ii].material].type & 31u);
+    s->one_bsdf = (types & (types - 1)) == 0;
+
     // emissive instances in instance order (world/emitter.cpp:169-263)
     std::vector<DevTexture> emit_tex;
     s->emitter_sources.clear();
@@ -835,6 +839,9 @@ pt_scene::~pt_scene() {
     if (ws.ev_in) cudaEventDestroy(ws.ev_in);
     if (ws.ev_out) cudaEventDestroy(ws.ev_out);
     if (ws.stream) cudaStreamDestroy(ws.stream);
+    if (ws.side) cudaStreamDestroy(ws.side);
+    if (ws.ev_shade) cudaEventDestroy(ws.ev_shade);
+    if (ws.ev_shadow) cudaEventDestroy(ws.ev_shadow);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
 }
