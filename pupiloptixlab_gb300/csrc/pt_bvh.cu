@@ -6,17 +6,18 @@
 //   1. primitive boxes and centroid bounds (block reduction + ordered atomics)
 //   2. 63-bit Morton codes (21 bits per axis)
 //   3. stable LSD radix sort of (code, primitive) pairs, 8 passes of 8 bits:
-//      tile histogram -> one-block exclusive scan -> warp-multisplit scatter
-//      (__match_any_sync ranks, per-warp digit counts in shared memory)
+//      tile histogram -> exclusive scan per digit over the tiles -> scatter
+//      (warp-private digit counters, __match_any_sync ranks)
 //   4. binary tree: PLOC clustering (default) or the Karras (HPG 2012)
 //      binary radix tree, equal codes split by index
-//   5. bottom-up boxes with an SAH cost per node (leaf vs split decision,
-//      leaves of at most max_leaf_size primitives)
-//   6. SAH-optimal assignment of the binary subtrees to the slots of 2/4/8-wide
-//      nodes (dynamic programming, bottom up), then a top-down,
-//      level-synchronous collapse that follows it; nodes come out in
-//      breadth-first order.
-//   7. primitive records gathered into leaf order
+//   5. with each binary node, when it forms: box, primitive count and the
+//      SAH-optimal assignment of its subtree to the slots of 2/4/8-wide nodes
+//      (dynamic programming, leaves of at most max_leaf_size primitives)
+//   6. top-down, level-synchronous collapse that follows those choices; nodes
+//      come out in breadth-first order
+//   7. primitive records gathered into leaf order (depth first)
+// The level and cluster counts stay on the device; the host reads them back a
+// few times a build.
 // Child boxes are padded outward (relative to the box and scene magnitude) so
 // that the conservative slab test never rejects a primitive the exact test
 // would hit.
@@ -27,6 +28,8 @@
 
 #include <algorithm>
 #include <cfloat>
+#include <cstddef>
+#include <type_traits>
 
 namespace {
 
@@ -71,18 +74,25 @@ __device__ __forceinline__ void prim_box(const float4 *prims, uint32_t p, float3
     }
 }
 
-// 1. per-primitive boxes (SoA float4) + centroid bounds into 6 ordered uints.
-__global__ void k_prim_bounds(const float4 *prims, uint32_t n, float4 *plo, float4 *phi, uint32_t *cb) {
+// 1. per-primitive box records + centroid bounds into 6 ordered uints.  A grid
+// of a few blocks per SM: one atomic per block and bound (16,033 blocks spent
+// most of their 174 us on six addresses).
+__global__ void k_prim_bounds(const float4 *prims, uint32_t n, float4 *pbox, uint32_t *cb) {
     __shared__ float red[6][32];
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     float v[6] = {FLT_MAX, FLT_MAX, FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX};
-    if (i < n) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         float3 lo, hi;
         prim_box(prims, i, lo, hi);
-        plo[i] = make_float4(lo.x, lo.y, lo.z, 0.f);
-        phi[i] = make_float4(hi.x, hi.y, hi.z, 0.f);
-        float cx = 0.5f * (lo.x + hi.x), cy = 0.5f * (lo.y + hi.y), cz = 0.5f * (lo.z + hi.z);
-        v[0] = cx; v[1] = cy; v[2] = cz; v[3] = cx; v[4] = cy; v[5] = cz;
+        // box record: (low, cost weight) (high, primitive count)
+        ptd::st8(pbox + 2 * (size_t)i, make_float4(lo.x, lo.y, lo.z, prim_cost(prims, i)),
+                 make_float4(hi.x, hi.y, hi.z, __int_as_float(1)));
+        const float cx = 0.5f * (lo.x + hi.x), cy = 0.5f * (lo.y + hi.y), cz = 0.5f * (lo.z + hi.z);
+        v[0] = fminf(v[0], cx);
+        v[1] = fminf(v[1], cy);
+        v[2] = fminf(v[2], cz);
+        v[3] = fmaxf(v[3], cx);
+        v[4] = fmaxf(v[4], cy);
+        v[5] = fmaxf(v[5], cz);
     }
     int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
@@ -123,12 +133,13 @@ __device__ __forceinline__ uint64_t split3(uint32_t a) {
 }
 
 // 2. Morton codes of the box centroids.
-__global__ void k_morton(const float4 *plo, const float4 *phi, uint32_t n, const uint32_t *cb, uint64_t *keys, uint32_t *vals) {
+__global__ void k_morton(const float4 *pbox, uint32_t n, const uint32_t *cb, uint64_t *keys, uint32_t *vals) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float mn[3] = {ord2f(cb[0]), ord2f(cb[1]), ord2f(cb[2])};
     float mx[3] = {ord2f(cb[3]), ord2f(cb[4]), ord2f(cb[5])};
-    float4 lo = plo[i], hi = phi[i];
+    float4 lo, hi;
+    ptd::ld8(pbox + 2 * (size_t)i, lo, hi);
     float c[3] = {0.5f * (lo.x + hi.x), 0.5f * (lo.y + hi.y), 0.5f * (lo.z + hi.z)};
     uint32_t q[3];
 #pragma unroll
@@ -157,71 +168,126 @@ __global__ void k_radix_hist(const uint64_t *keys, uint32_t n, int shift, uint32
     hist[(size_t)threadIdx.x * tiles + blockIdx.x] = h[threadIdx.x];
 }
 
-// 3b. in-place exclusive scan of m values with one block of 1024 threads.
-__global__ void k_scan_excl(uint32_t *data, uint32_t m) {
-    __shared__ uint32_t part[1024];
-    uint32_t per = (m + 1023) / 1024;
-    uint32_t b = threadIdx.x * per, e = min(m, b + per);
-    uint32_t sum = 0;
-    for (uint32_t i = b; i < e; i++) sum += data[i];
-    part[threadIdx.x] = sum;
-    __syncthreads();
-    for (int o = 1; o < 1024; o <<= 1) {
-        uint32_t v = threadIdx.x >= (uint32_t)o ? part[threadIdx.x - o] : 0;
+// 3b. one block per digit: exclusive scan of its tile counts, in place, and
+// their total.  (One block over all 256 * tiles counts took about 100 us a pass
+// at 4 million primitives.)
+__global__ void __launch_bounds__(256) k_radix_scan(uint32_t *hist, uint32_t tiles, uint32_t *total) {
+    __shared__ uint32_t wsum[8];
+    uint32_t *row = hist + (size_t)blockIdx.x * tiles;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t carry = 0;
+    for (uint32_t b = 0; b < tiles; b += 256) {
+        const uint32_t i = b + threadIdx.x;
+        const uint32_t v = i < tiles ? row[i] : 0u;
+        uint32_t x = v;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= (uint32_t)o) x += y;
+        }
+        if (lane == 31) wsum[warp] = x;
         __syncthreads();
-        part[threadIdx.x] += v;
+        uint32_t before = 0, all = 0;
+        for (uint32_t w = 0; w < 8; w++) {
+            if (w < warp) before += wsum[w];
+            all += wsum[w];
+        }
+        if (i < tiles) row[i] = carry + before + x - v;
+        carry += all;
         __syncthreads();
     }
-    uint32_t run = part[threadIdx.x] - sum;
-    for (uint32_t i = b; i < e; i++) {
-        uint32_t v = data[i];
-        data[i] = run;
-        run += v;
-    }
+    if (threadIdx.x == 0) total[blockIdx.x] = carry;
 }
 
-// 3c. stable scatter: ranks within a tile come from warp multisplit.
-__global__ void __launch_bounds__(kSortThreads) k_radix_scatter(const uint64_t *kin, const uint32_t *vin, uint64_t *kout,
+// 3c. stable scatter.  Each warp owns a contiguous eighth of the tile and
+// counts its digits in order (the rank of an entry = its warp's count so far +
+// its rank among the equal digits of its 32).  The tile is put in digit order
+// in shared memory first, so that runs of equal digits are written together
+// (written straight from the registers: 98 us a pass at 4.1 million pairs).
+constexpr int kScatterSmem = kSortTile * 12;
+__global__ void __launch_bounds__(kSortThreads, 3) k_radix_scatter(const uint64_t *kin, const uint32_t *vin, uint64_t *kout,
                                                                 uint32_t *vout, uint32_t n, int shift,
-                                                                const uint32_t *hist, uint32_t tiles) {
-    __shared__ uint32_t base_off[256];
-    __shared__ uint32_t wcnt[kSortThreads / 32][256];
-    __shared__ uint32_t tot[256];
+                                                                const uint32_t *hist, uint32_t tiles,
+                                                                const uint32_t *total) {
+    constexpr int kWarps = kSortThreads / 32;
+    extern __shared__ uint64_t sort_smem[];
+    uint64_t *skey = sort_smem;
+    uint32_t *sval = reinterpret_cast<uint32_t *>(skey + kSortTile);
+    __shared__ uint32_t wcnt[kWarps][256];
+    __shared__ uint32_t gbase[256];  // output position of a digit's first entry, minus its place in the tile
+    __shared__ uint32_t wsum[2][kWarps];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    base_off[tid] = hist[(size_t)tid * tiles + blockIdx.x];
     const uint32_t lt = (1u << lane) - 1u;
-    size_t base = (size_t)blockIdx.x * kSortTile;
+    for (int d = lane; d < 256; d += 32) wcnt[warp][d] = 0;
+    __syncwarp();
+    const uint32_t t0 = blockIdx.x * kSortTile;
+    const uint32_t base = warp * (32 * kSortItems) + lane;
+    uint64_t key[kSortItems];
+    uint32_t rank[kSortItems];
+#pragma unroll
     for (int k = 0; k < kSortItems; k++) {
+        const uint32_t i = base + k * 32;
+        key[k] = t0 + i < n ? kin[t0 + i] : ~0ull;
+    }
 #pragma unroll
-        for (int w = 0; w < kSortThreads / 32; w++) wcnt[w][tid] = 0;
-        __syncthreads();
-        size_t idx = base + (size_t)k * kSortThreads + tid;
-        bool valid = idx < n;
-        uint64_t key = valid ? kin[idx] : 0;
-        uint32_t val = valid ? vin[idx] : 0;
-        uint32_t digit = valid ? (uint32_t)((key >> shift) & 255u) : 256u;
-        uint32_t peers = __match_any_sync(0xffffffffu, digit);
-        uint32_t lrank = __popc(peers & lt);
-        if (valid && lrank == 0) wcnt[warp][digit] = __popc(peers);
-        __syncthreads();
-        {
-            uint32_t run = 0;
-#pragma unroll
-            for (int w = 0; w < kSortThreads / 32; w++) {
-                uint32_t c = wcnt[w][tid];
-                wcnt[w][tid] = run;
-                run += c;
+    for (int k = 0; k < kSortItems; k++) {
+        const bool valid = t0 + base + k * 32 < n;
+        const uint32_t digit = (uint32_t)(key[k] >> shift) & 255u;
+        const uint32_t peers = __match_any_sync(0xffffffffu, valid ? digit : 256u);
+        uint32_t old = 0;
+        if (valid) old = wcnt[warp][digit];
+        __syncwarp();
+        if (valid && (peers & lt) == 0) wcnt[warp][digit] = old + __popc(peers);
+        __syncwarp();
+        rank[k] = old + __popc(peers & lt);
+    }
+    __syncthreads();
+    {  // thread = digit: starts of the digits in the output (over the totals) and in the tile
+        uint32_t mine = 0;
+        for (int w = 0; w < kWarps; w++) mine += wcnt[w][tid];
+        const uint32_t tot = total[tid];
+        uint32_t a = tot, b = mine;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t ya = __shfl_up_sync(0xffffffffu, a, o), yb = __shfl_up_sync(0xffffffffu, b, o);
+            if (lane >= o) {
+                a += ya;
+                b += yb;
             }
-            tot[tid] = run;
+        }
+        if (lane == 31) {
+            wsum[0][warp] = a;
+            wsum[1][warp] = b;
         }
         __syncthreads();
-        if (valid) {
-            uint32_t pos = base_off[digit] + wcnt[warp][digit] + lrank;
-            kout[pos] = key;
-            vout[pos] = val;
+        a -= tot;
+        b -= mine;
+        for (int w = 0; w < warp; w++) {
+            a += wsum[0][w];
+            b += wsum[1][w];
         }
-        __syncthreads();
-        base_off[tid] += tot[tid];
+        gbase[tid] = a + hist[(size_t)tid * tiles + blockIdx.x] - b;
+        uint32_t run = b;
+        for (int w = 0; w < kWarps; w++) {
+            const uint32_t c = wcnt[w][tid];
+            wcnt[w][tid] = run;
+            run += c;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kSortItems; k++) {
+        const uint32_t i = t0 + base + k * 32;
+        if (i >= n) continue;
+        const uint32_t at = wcnt[warp][(uint32_t)(key[k] >> shift) & 255u] + rank[k];
+        skey[at] = key[k];
+        sval[at] = vin[i];
+    }
+    __syncthreads();
+    const uint32_t count = min((uint32_t)kSortTile, n - t0);
+    for (uint32_t i = tid; i < count; i += kSortThreads) {
+        const uint64_t key_i = skey[i];
+        const uint32_t pos = gbase[(uint32_t)(key_i >> shift) & 255u] + i;
+        kout[pos] = key_i;
+        vout[pos] = sval[i];
     }
 }
 
@@ -233,7 +299,7 @@ __device__ __forceinline__ int delta(const uint64_t *keys, int n, int i, int j) 
 }
 
 // 4. Karras binary radix tree.  Internal nodes 0..n-2, leaf k is node n-1+k.
-__global__ void k_karras(const uint64_t *keys, int n, int *left, int *right, int *parent, int *rfirst) {
+__global__ void k_karras(const uint64_t *keys, int n, int4 *links, int *parent) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n - 1) return;
     int d = (delta(keys, n, i, i + 1) - delta(keys, n, i, i - 1)) >= 0 ? 1 : -1;
@@ -256,11 +322,9 @@ __global__ void k_karras(const uint64_t *keys, int n, int *left, int *right, int
     int first = min(i, j), last = max(i, j);
     int lc = (first == gamma) ? (n - 1 + gamma) : gamma;
     int rc = (last == gamma + 1) ? (n - 1 + gamma + 1) : gamma + 1;
-    left[i] = lc;
-    right[i] = rc;
+    links[i] = make_int4(lc, rc, 0, 0);
     parent[lc] = i;
     parent[rc] = i;
-    rfirst[i] = first;
 }
 
 __device__ __forceinline__ float half_area(float4 lo, float4 hi) {
@@ -268,234 +332,398 @@ __device__ __forceinline__ float half_area(float4 lo, float4 hi) {
     return ex * ey + ey * ez + ez * ex;
 }
 
-// 5. bottom-up boxes, counts and SAH costs (second arrival processes a node).
-__global__ void k_bottom_up(int n, const int *left, const int *right, const int *parent, const uint32_t *order,
-                            const float4 *prims, const float4 *plo, const float4 *phi, float4 *nlo, float4 *nhi,
-                            int *ncount, float *ncost, float *nwt, int *nleaf, int *flags, int max_leaf) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
+// A binary node's box record: (low, summed cost weight) (high, primitive count).
+struct NodeBox {
+    float4 lo, hi;
+    __device__ __forceinline__ float area() const { return half_area(lo, hi); }
+    __device__ __forceinline__ float weight() const { return lo.w; }
+    __device__ __forceinline__ int count() const { return __float_as_int(hi.w); }
+};
+__device__ __forceinline__ NodeBox load_box(const float4 *nb, int x) {
+    NodeBox b;
+    ptd::ld8(nb + 2 * (size_t)x, b.lo, b.hi);
+    return b;
+}
+__device__ __forceinline__ NodeBox merged(const NodeBox &a, const NodeBox &b) {
+    NodeBox u;
+    u.lo = make_float4(fminf(a.lo.x, b.lo.x), fminf(a.lo.y, b.lo.y), fminf(a.lo.z, b.lo.z), a.lo.w + b.lo.w);
+    u.hi = make_float4(fmaxf(a.hi.x, b.hi.x), fmaxf(a.hi.y, b.hi.y), fmaxf(a.hi.z, b.hi.z),
+                       __int_as_float(a.count() + b.count()));
+    return u;
+}
+
+// The binary tree: internal nodes 0..n-2, leaf k (sorted primitive k) is node
+// n-1+k.
+struct Tree {
+    int n, max_leaf;
+    int4 *links;   // per internal node: left, right, the choices (below), the left child's primitive count
+    float4 *nb;    // 2 per node
+    float *dval;   // K per internal node: S(x, 1..K) below
+};
+
+// 5. SAH-optimal wide collapse (Ylitie, Karras and Laine, HPG 2017): for
+// every binary node x and i = 1..K, S(x, i) is the cheapest way to represent
+// its subtree with at most i slots of a wide parent:
+//   S(x, 1) = min(leaf: area * primitive weight (if count <= max_leaf),
+//                 wide node: 1.2 * area + min_j S(l, j) + S(r, K - j))
+//   S(x, i) = min(S(x, i - 1), min_j S(l, j) + S(r, i - j))
+// Formed with the node itself, when its children are complete.  The choices, 3
+// bits each: 0 the wide node's split j, i - 1 the split for i = 2..K slots (0:
+// use i - 1 slots); bit 31: leaf.
+constexpr uint32_t kSelLeaf = 1u << 31;
+__device__ __forceinline__ int sel_of(int sel, int i) { return (sel >> (3 * i)) & 7; }
+
+template <int K>
+__device__ __forceinline__ void load_costs(const Tree &t, int x, const NodeBox &b, float *c) {
+    if (x >= t.n - 1) {
+        const float v = b.area() * b.weight();
+#pragma unroll
+        for (int i = 0; i < K; i++) c[i] = v;
+    } else {
+#pragma unroll
+        for (int i = 0; i < K; i++) c[i] = __ldcg(t.dval + (size_t)x * K + i);
+    }
+}
+
+// Node `id` over children l and r (boxes bl, br): links, box, costs, choices.
+template <int K>
+__device__ __forceinline__ NodeBox form_node(const Tree &t, int id, int l, int r, const NodeBox &bl, const NodeBox &br) {
+    const NodeBox u = merged(bl, br);
+    float sl[K], sr[K], sx[K];
+    load_costs<K>(t, l, bl, sl);
+    load_costs<K>(t, r, br, sr);
+    const float area = u.area();
+    float best = FLT_MAX;
+    int jw = 1;
+#pragma unroll
+    for (int j = 1; j < K; j++) {
+        const float c = sl[j - 1] + sr[K - j - 1];
+        if (c < best) {
+            best = c;
+            jw = j;
+        }
+    }
+    const float c_wide = kCostNode * area + best;
+    const float c_leaf = u.count() <= t.max_leaf ? area * u.weight() : FLT_MAX;
+    const bool mk_leaf = c_leaf <= c_wide;
+    sx[0] = mk_leaf ? c_leaf : c_wide;
+    uint32_t sel = (uint32_t)jw | (mk_leaf ? kSelLeaf : 0);
+#pragma unroll
+    for (int i = 2; i <= K; i++) {
+        float v = sx[i - 2];
+        int pick = 0;
+#pragma unroll
+        for (int j = 1; j < i; j++) {
+            const float c = sl[j - 1] + sr[i - j - 1];
+            if (c < v) {
+                v = c;
+                pick = j;
+            }
+        }
+        sx[i - 1] = v;
+        sel |= (uint32_t)pick << (3 * (i - 1));
+    }
+#pragma unroll
+    for (int i = 0; i < K; i++) t.dval[(size_t)id * K + i] = sx[i];
+    t.links[id] = make_int4(l, r, (int)sel, bl.count());
+    ptd::st8(t.nb + 2 * (size_t)id, u.lo, u.hi);
+    return u;
+}
+
+// The sorted primitives as leaves.
+__global__ void k_leaf_boxes(int n, const uint32_t *order, const float4 *pbox, float4 *nb, int *cl) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
-    int leaf = n - 1 + k;
-    uint32_t p = order[k];
-    float4 lo = plo[p], hi = phi[p];
-    const float w = prim_cost(prims, p);
-    nlo[leaf] = lo;
-    nhi[leaf] = hi;
-    ncount[leaf] = 1;
-    ncost[leaf] = w * half_area(lo, hi);
-    nwt[leaf] = w;
-    nleaf[leaf] = 1;
-    int cur = parent[leaf];
+    const NodeBox b = load_box(pbox, (int)order[k]);
+    ptd::st8(nb + 2 * (size_t)(n - 1 + k), b.lo, b.hi);
+    cl[k] = n - 1 + k;
+}
+
+// Radix tree, bottom up (second arrival forms a node).
+template <int K>
+__global__ void k_bottom_up(const Tree t, const int *parent, int *flags) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= t.n) return;
+    int cur = parent[t.n - 1 + k];
     while (cur >= 0) {
         __threadfence();
         if (atomicAdd(&flags[cur], 1) == 0) return;
         __threadfence();
-        int l = left[cur], r = right[cur];
-        float4 llo = __ldcg(&nlo[l]), lhi = __ldcg(&nhi[l]), rlo = __ldcg(&nlo[r]), rhi = __ldcg(&nhi[r]);
-        float4 blo = make_float4(fminf(llo.x, rlo.x), fminf(llo.y, rlo.y), fminf(llo.z, rlo.z), 0.f);
-        float4 bhi = make_float4(fmaxf(lhi.x, rhi.x), fmaxf(lhi.y, rhi.y), fmaxf(lhi.z, rhi.z), 0.f);
-        int cnt = __ldcg(&ncount[l]) + __ldcg(&ncount[r]);
-        float wsum = __ldcg(&nwt[l]) + __ldcg(&nwt[r]);
-        float a = half_area(blo, bhi);
-        float c_split = kCostNode * a + __ldcg(&ncost[l]) + __ldcg(&ncost[r]);
-        float c_leaf = cnt <= max_leaf ? a * wsum : FLT_MAX;
-        bool mk_leaf = c_leaf <= c_split;
-        nlo[cur] = blo;
-        nhi[cur] = bhi;
-        ncount[cur] = cnt;
-        nwt[cur] = wsum;
-        ncost[cur] = mk_leaf ? c_leaf : c_split;
-        nleaf[cur] = mk_leaf ? 1 : 0;
+        const int l = t.links[cur].x, r = t.links[cur].y;
+        NodeBox bl, br;
+        bl.lo = __ldcg(t.nb + 2 * (size_t)l);
+        bl.hi = __ldcg(t.nb + 2 * (size_t)l + 1);
+        br.lo = __ldcg(t.nb + 2 * (size_t)r);
+        br.hi = __ldcg(t.nb + 2 * (size_t)r + 1);
+        form_node<K>(t, cur, l, r, bl, br);
         cur = parent[cur];
     }
 }
 
-// 4'/5'. PLOC: parallel locally-ordered clustering (Meister and Bittner,
+// 4'. PLOC: parallel locally-ordered clustering (Meister and Bittner,
 // IEEE TVCG 2018), the default build.  The Morton-sorted primitives start as
-// clusters (leaf k = node n-1+k); each pass every cluster finds the cluster
-// within kPlocRadius positions whose union has the smallest surface area,
-// mutual nearest neighbours merge into a new internal node (id from a
-// counter, 0..n-2) that takes the lower position, and the array is compacted.
-// Boxes, counts and the SAH leaf-or-split decision of a node are made when it
-// forms (its children are complete by then).  Subtrees are then laid out
-// depth first so that every subtree covers a contiguous range of the
-// primitive order, as the wide collapse expects.
+// clusters; each pass every cluster finds the cluster within kPlocRadius
+// positions whose union has the smallest surface area (ties to the lower
+// position, so the closest pair is always mutual), mutual nearest neighbours
+// merge into a new internal node (id from a counter, 0..n-2) that takes the
+// lower position, and the array is compacted.  A pass is two launches: neighbours
+// and merging share a tile with a halo of two radii, and each compaction tile
+// sums the survivor counts of the tiles before it.  The counts stay on the
+// device: the host bounds the grids by the count it last read.  The last
+// kPlocTail clusters are merged by one block in shared memory.
+// The neighbour search is bound by shared-memory reads (64 128-bit loads a
+// position, 181 us for 4.1 million), so a thread searches for PER = 4
+// consecutive positions, whose windows share 28 of 36 boxes; where few tiles
+// are left the time is one thread's chain (20 us at PER = 4), so PER = 1.
 constexpr int kPlocRadius = 16;
-constexpr int kPlocBlock = 256;
-constexpr int kPlocMaxDepth = 256;  // a deeper binary tree makes the build fall back to the radix tree
+constexpr int kPlocThreads = 288;
+__host__ __device__ constexpr int ploc_tile(int per) { return kPlocThreads * per - 2 * kPlocRadius; }  // every thread searches once
+constexpr int kPlocTail = 2048;
+constexpr int kPlocMaxPasses = 64 + 8 * 28;
+constexpr int kPlocPassesPerRead = 8;  // clusters shrink by about a quarter a pass
+constexpr uint32_t kPlocWide = 300000;  // clusters from which PER = 4 is used (about two tiles an SM)
 
-__global__ void k_ploc_init(int n, const uint32_t *order, const float4 *prims, const float4 *plo, const float4 *phi,
-                            float4 *nlo, float4 *nhi, int *ncount, float *ncost, float *nwt, int *nleaf, int *cl) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    int leaf = n - 1 + k;
-    uint32_t p = order[k];
-    float4 lo = plo[p], hi = phi[p];
-    const float w = prim_cost(prims, p);
-    nlo[leaf] = lo;
-    nhi[leaf] = hi;
-    ncount[leaf] = 1;
-    ncost[leaf] = w * half_area(lo, hi);
-    nwt[leaf] = w;
-    nleaf[leaf] = 1;
-    cl[k] = leaf;
+// Device-side counts of a build.
+constexpr int kMaxLevels = 128;
+struct BuildCounts {
+    uint32_t centroid[6];   // ordered-float bounds
+    uint32_t nodes;         // PLOC internal nodes formed
+    uint32_t fail;
+    double sah, root_area;
+    uint32_t level[kMaxLevels + 1];            // wide nodes per level
+    uint32_t clusters[kPlocMaxPasses + 2];     // PLOC clusters before pass p
+};
+
+// Nearest neighbours of the positions i..i+PER-1 among the boxes lo/hi in shared
+// memory (box of position i + o at place(o); out of range: an unbounded box).
+template <int PER, class Place>
+__device__ __forceinline__ void nearest(const float4 *lo, const float4 *hi, const Place &place, int i, int *bj) {
+    float4 al[PER], ah[PER];
+    float best[PER];
+#pragma unroll
+    for (int q = 0; q < PER; q++) {
+        al[q] = lo[place(q)];
+        ah[q] = hi[place(q)];
+        best[q] = FLT_MAX;
+        bj[q] = -1;
+    }
+#pragma unroll
+    for (int o = -kPlocRadius; o < PER + kPlocRadius; o++) {
+        const float4 bl = lo[place(o)], bh = hi[place(o)];
+#pragma unroll
+        for (int q = 0; q < PER; q++) {
+            if (o == q || o - q > kPlocRadius || q - o > kPlocRadius) continue;
+            const float4 ul = make_float4(fminf(al[q].x, bl.x), fminf(al[q].y, bl.y), fminf(al[q].z, bl.z), 0.f);
+            const float4 uh = make_float4(fmaxf(ah[q].x, bh.x), fmaxf(ah[q].y, bh.y), fmaxf(ah[q].z, bh.z), 0.f);
+            const float a = half_area(ul, uh);
+            if (a < best[q]) {  // positions are visited in increasing order: ties keep the lower one
+                best[q] = a;
+                bj[q] = i + o;
+            }
+        }
+    }
+}
+__device__ __forceinline__ void unbounded(float4 &lo, float4 &hi) {
+    lo = make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, 0.f);
+    hi = make_float4(FLT_MAX, FLT_MAX, FLT_MAX, 0.f);
 }
 
-// Nearest neighbour of every cluster: smallest union area, ties to the lower
-// position (so the closest pair overall is always mutual).
-__global__ void __launch_bounds__(kPlocBlock) k_ploc_nn(int m, const int *cl, const float4 *nlo, const float4 *nhi,
-                                                        int *nn) {
-    __shared__ float4 slo[kPlocBlock + 2 * kPlocRadius], shi[kPlocBlock + 2 * kPlocRadius];
-    const int b0 = blockIdx.x * kPlocBlock;
-    for (int t = threadIdx.x; t < kPlocBlock + 2 * kPlocRadius; t += blockDim.x) {
-        const int g = b0 - kPlocRadius + t;
+template <int K, int PER>
+__global__ void __launch_bounds__(kPlocThreads) k_ploc_merge(const Tree t, BuildCounts *bc, int pass, const int *cl,
+                                                             int *out_id, uint32_t *tile_count) {
+    constexpr int R = kPlocRadius, kTile = ploc_tile(PER);
+    // boxes of the positions [t0 - 2R, t0 + kTile + 2R), PER rows: the boxes a
+    // warp reads together are neighbours in a row (no bank conflicts)
+    constexpr int kCols = kPlocThreads + 2 * R / PER + (PER > 1 ? 1 : 0);
+    __shared__ float4 slo[PER * kCols], shi[PER * kCols];
+    __shared__ int snn[kTile + 2 * R];
+    __shared__ uint32_t kept;
+    const auto at = [](int k) { return PER == 1 ? k : (k % PER) * kCols + k / PER; };  // place of position t0 - 2R + k
+    const int m = (int)bc->clusters[pass];
+    const int t0 = blockIdx.x * kTile;
+    if (t0 >= m) return;  // uniform
+    if (threadIdx.x == 0) kept = 0;
+    for (int k = threadIdx.x; k < kTile + 4 * R; k += kPlocThreads) {
+        const int g = t0 - 2 * R + k;
         if (g >= 0 && g < m) {
-            const int id = cl[g];
-            slo[t] = nlo[id];
-            shi[t] = nhi[id];
+            const NodeBox b = load_box(t.nb, cl[g]);
+            slo[at(k)] = b.lo;
+            shi[at(k)] = b.hi;
+        } else {
+            unbounded(slo[at(k)], shi[at(k)]);
         }
     }
     __syncthreads();
-    const int i = b0 + threadIdx.x;
-    if (i >= m) return;
-    const float4 lo = slo[threadIdx.x + kPlocRadius], hi = shi[threadIdx.x + kPlocRadius];
-    float best = FLT_MAX;
-    int bj = -1;
-    for (int o = -kPlocRadius; o <= kPlocRadius; o++) {
-        const int j = i + o;
-        if (o == 0 || j < 0 || j >= m) continue;
-        const float4 l2 = slo[threadIdx.x + kPlocRadius + o], h2 = shi[threadIdx.x + kPlocRadius + o];
-        const float4 ulo = make_float4(fminf(lo.x, l2.x), fminf(lo.y, l2.y), fminf(lo.z, l2.z), 0.f);
-        const float4 uhi = make_float4(fmaxf(hi.x, h2.x), fmaxf(hi.y, h2.y), fmaxf(hi.z, h2.z), 0.f);
-        const float a = half_area(ulo, uhi);
-        if (a < best) {  // positions are visited in increasing order: ties keep the lower one
-            best = a;
-            bj = j;
+    {
+        const int c = threadIdx.x * PER;  // positions t0 - R + c ...
+        int bj[PER];
+        // place of position t0 - R + c + o (c a multiple of PER)
+        const auto place = [](int o) { return (R + o) % PER * kCols + (int)threadIdx.x + (R + o) / PER; };
+        nearest<PER>(slo, shi, place, t0 - R + c, bj);
+#pragma unroll
+        for (int q = 0; q < PER; q++) {
+            const int g = t0 - R + c + q;
+            snn[c + q] = g >= 0 && g < m ? bj[q] : -1;
         }
     }
-    nn[i] = bj;
+    __syncthreads();
+    uint32_t mine = 0;
+    for (int k = threadIdx.x; k < kTile; k += kPlocThreads) {
+        const int i = t0 + k;
+        if (i >= m) break;
+        const int j = snn[k + R];
+        const bool mutual = j >= 0 && snn[j - t0 + R] == i;
+        int out = -1;
+        if (!mutual) {
+            out = cl[i];
+        } else if (i < j) {
+            NodeBox a, b;
+            a.lo = slo[at(k + 2 * R)];
+            a.hi = shi[at(k + 2 * R)];
+            b.lo = slo[at(j - t0 + 2 * R)];
+            b.hi = shi[at(j - t0 + 2 * R)];
+            out = (int)atomicAdd(&bc->nodes, 1u);
+            form_node<K>(t, out, cl[i], cl[j], a, b);
+        }
+        out_id[i] = out;
+        mine += out >= 0 ? 1u : 0u;
+    }
+    for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
+    if ((threadIdx.x & 31) == 0) atomicAdd(&kept, mine);
+    __syncthreads();
+    if (threadIdx.x == 0) tile_count[blockIdx.x] = kept;
 }
 
-// Merge mutual pairs: keep[i] = 1 where position i survives, out_id[i] its node.
-__global__ void k_ploc_merge(int m, const int *cl, const int *nn, uint32_t *keep, int *out_id, uint32_t *node_ctr,
-                             int *left, int *right, int *parent, float4 *nlo, float4 *nhi, int *ncount, float *ncost,
-                             float *nwt, int *nleaf, int max_leaf) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m) return;
-    const int j = nn[i];
-    const bool mutual = j >= 0 && nn[j] == i;
-    if (!mutual) {
-        keep[i] = 1;
-        out_id[i] = cl[i];
+// Order-preserving compaction of a tile's survivors behind those of the tiles
+// before it; the last tile records the next pass's counts.
+template <int PER>
+__global__ void __launch_bounds__(kPlocThreads) k_ploc_compact(BuildCounts *bc, int pass, const int *out_id,
+                                                               const uint32_t *tile_count, int *cl_next) {
+    constexpr int kWarps = kPlocThreads / 32, kTile = ploc_tile(PER);
+    constexpr int kRounds = (kTile + kPlocThreads - 1) / kPlocThreads;
+    __shared__ uint32_t before[kWarps];
+    __shared__ uint32_t wc[kRounds * kWarps];
+    const int m = (int)bc->clusters[pass];
+    const int t0 = blockIdx.x * kTile;
+    if (t0 >= m) return;  // uniform
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t sum = 0;
+    for (uint32_t b = threadIdx.x; b < blockIdx.x; b += kPlocThreads) sum += tile_count[b];
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane == 0) before[warp] = sum;
+    int id[kRounds];
+    unsigned bal[kRounds];
+#pragma unroll
+    for (int k = 0; k < kRounds; k++) {
+        const int at = k * kPlocThreads + (int)threadIdx.x;
+        id[k] = at < kTile && t0 + at < m ? out_id[t0 + at] : -1;
+        bal[k] = __ballot_sync(0xffffffffu, id[k] >= 0);
+        if (lane == 0) wc[k * kWarps + warp] = __popc(bal[k]);
+    }
+    __syncthreads();
+    uint32_t start = 0;
+    for (int w = 0; w < kWarps; w++) start += before[w];
+#pragma unroll
+    for (int k = 0; k < kRounds; k++) {
+        uint32_t at = start;
+        for (uint32_t w = 0; w < kWarps; w++) {
+            if (w < warp) at += wc[k * kWarps + w];
+            start += wc[k * kWarps + w];
+        }
+        if (id[k] >= 0) cl_next[at + __popc(bal[k] & ((1u << lane) - 1u))] = id[k];
+    }
+    if (t0 + kTile >= m && threadIdx.x == 0) bc->clusters[pass + 1] = start;
+}
+
+// The passes from `pass` on, at most kPlocTail clusters, in one block.
+template <int K>
+__global__ void __launch_bounds__(1024) k_ploc_tail(const Tree t, BuildCounts *bc, int pass, const int *cl) {
+    constexpr int R = kPlocRadius, kPer = kPlocTail / 1024;
+    extern __shared__ float4 tail_smem[];
+    float4 *slo = tail_smem, *shi = slo + kPlocTail + 2 * R;
+    int *sid = reinterpret_cast<int *>(shi + kPlocTail + 2 * R), *snn = sid + kPlocTail;
+    __shared__ uint32_t wc[kPer * 32];
+    __shared__ uint32_t ctr, survivors;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int m = (int)bc->clusters[pass];
+    if (m > kPlocTail || m < 1) {  // uniform: the host starts this kernel only below the limit
+        if (tid == 0) bc->fail = 1;
         return;
     }
-    if (i > j) {
-        keep[i] = 0;
-        return;
-    }
-    const int a = cl[i], b = cl[j];
-    const int id = (int)atomicAdd(node_ctr, 1u);
-    const float4 la = nlo[a], ha = nhi[a], lb = nlo[b], hb = nhi[b];
-    const float4 blo = make_float4(fminf(la.x, lb.x), fminf(la.y, lb.y), fminf(la.z, lb.z), 0.f);
-    const float4 bhi = make_float4(fmaxf(ha.x, hb.x), fmaxf(ha.y, hb.y), fmaxf(ha.z, hb.z), 0.f);
-    const int cnt = ncount[a] + ncount[b];
-    const float wsum = nwt[a] + nwt[b];
-    const float area = half_area(blo, bhi);
-    const float c_split = kCostNode * area + ncost[a] + ncost[b];
-    const float c_leaf = cnt <= max_leaf ? area * wsum : FLT_MAX;
-    const bool mk_leaf = c_leaf <= c_split;
-    left[id] = a;
-    right[id] = b;
-    parent[a] = id;
-    parent[b] = id;
-    nlo[id] = blo;
-    nhi[id] = bhi;
-    ncount[id] = cnt;
-    nwt[id] = wsum;
-    ncost[id] = mk_leaf ? c_leaf : c_split;
-    nleaf[id] = mk_leaf ? 1 : 0;
-    keep[i] = 1;
-    out_id[i] = id;
-}
-
-// Order-preserving compaction of the surviving positions in blocks of
-// kCompactBlock: survivors per block (warp ballots), an exclusive scan of the
-// block counts, then each survivor's rank = block offset + warp offset + its
-// rank among the warp's survivors.
-constexpr int kCompactBlock = 1024;
-
-__global__ void __launch_bounds__(kCompactBlock) k_ploc_block_counts(int m, const uint32_t *keep, uint32_t *bsum) {
-    __shared__ uint32_t wc[kCompactBlock / 32];
-    const int i = blockIdx.x * kCompactBlock + threadIdx.x;
-    const unsigned b = __ballot_sync(0xffffffffu, i < m && keep[i] != 0);
-    if ((threadIdx.x & 31) == 0) wc[threadIdx.x >> 5] = __popc(b);
+    if (tid == 0) ctr = bc->nodes;
+    for (int i = tid; i < kPlocTail + 2 * R; i += 1024) unbounded(slo[i], shi[i]);
     __syncthreads();
-    if (threadIdx.x < 32) {
-        uint32_t v = wc[threadIdx.x];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (threadIdx.x == 0) bsum[blockIdx.x] = v;
+    for (int i = tid; i < m; i += 1024) {
+        const int id = cl[i];
+        const NodeBox b = load_box(t.nb, id);
+        sid[i] = id;
+        slo[i + R] = b.lo;
+        shi[i + R] = b.hi;
     }
-}
-
-__global__ void __launch_bounds__(kCompactBlock) k_ploc_compact(int m, const uint32_t *keep, const uint32_t *boff,
-                                                                const int *out_id, int *cl_next) {
-    __shared__ uint32_t woff[kCompactBlock / 32];
-    const int i = blockIdx.x * kCompactBlock + threadIdx.x;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const bool k = i < m && keep[i] != 0;
-    const unsigned b = __ballot_sync(0xffffffffu, k);
-    if (lane == 0) woff[warp] = __popc(b);
     __syncthreads();
-    if (warp == 0) {  // exclusive scan of the per-warp counts
-        const uint32_t v = woff[lane];
-        uint32_t x = v;
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
+    while (m > 1 && pass < kPlocMaxPasses) {
+        for (int i = tid; i < m; i += 1024) nearest<1>(slo, shi, [&](int o) { return i + R + o; }, i, snn + i);
+        __syncthreads();
+        int id[kPer];
+        NodeBox box[kPer];
+        unsigned bal[kPer];
+#pragma unroll
+        for (int k = 0; k < kPer; k++) {
+            const int i = k * 1024 + tid;
+            id[k] = -1;
+            if (i < m) {
+                const int j = snn[i];
+                const bool mutual = j >= 0 && snn[j] == i;
+                box[k].lo = slo[i + R];
+                box[k].hi = shi[i + R];
+                if (!mutual) {
+                    id[k] = sid[i];
+                } else if (i < j) {
+                    NodeBox b;
+                    b.lo = slo[j + R];
+                    b.hi = shi[j + R];
+                    id[k] = (int)atomicAdd(&ctr, 1u);
+                    box[k] = form_node<K>(t, id[k], sid[i], sid[j], box[k], b);
+                }
+            }
+            bal[k] = __ballot_sync(0xffffffffu, id[k] >= 0);
+            if (lane == 0) wc[k * 32 + warp] = __popc(bal[k]);
         }
-        woff[lane] = x - v;
-    }
-    __syncthreads();
-    if (k) cl_next[boff[blockIdx.x] + woff[warp] + __popc(b & ((1u << lane) - 1u))] = out_id[i];
-}
-
-// Depth-first position of every node (leftmost leaf of its subtree): the sum
-// of the left siblings' primitive counts along the path to the root.  A path
-// longer than kPlocMaxDepth raises the failure flag.
-__global__ void k_ploc_offsets(int n, const int *left, const int *right, const int *parent, const int *ncount,
-                               int *offs, uint32_t *fail) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= 2 * n - 1) return;
-    int cur = x, off = 0, steps = 0;
-    for (int p = parent[cur]; p >= 0; p = parent[cur]) {
-        if (right[p] == cur) off += ncount[left[p]];
-        cur = p;
-        if (++steps > kPlocMaxDepth) {
-            atomicOr(fail, 1u);
-            break;
+        __syncthreads();  // boxes and ids are read, nodes are formed
+        if (warp == 0) {
+            uint32_t carry = 0;
+            for (int k = 0; k < kPer; k++) {
+                const uint32_t v = wc[k * 32 + lane];
+                uint32_t x = v;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+                    if (lane >= o) x += y;
+                }
+                wc[k * 32 + lane] = carry + x - v;
+                carry += __shfl_sync(0xffffffffu, x, 31);
+            }
+            if (lane == 0) survivors = carry;
         }
+        __syncthreads();
+        const int next = (int)survivors;
+#pragma unroll
+        for (int k = 0; k < kPer; k++) {
+            if (id[k] < 0) continue;
+            const int at = (int)(wc[k * 32 + warp] + __popc(bal[k] & ((1u << lane) - 1u)));
+            sid[at] = id[k];
+            slo[at + R] = box[k].lo;
+            shi[at + R] = box[k].hi;
+        }
+        __syncthreads();
+        for (int i = next + tid; i < m; i += 1024) unbounded(slo[i + R], shi[i + R]);
+        __syncthreads();
+        pass++;
+        if (next >= m) break;  // uniform: no pair merged (boxes without a finite area)
+        m = next;
     }
-    offs[x] = off;
-}
-
-// Renumber leaves to their depth-first positions (leaf at position q is node
-// n-1+q), record every internal node's first position, permute the order.
-__global__ void k_ploc_finish(int n, const int *offs, const uint32_t *order, const float4 *nlo, const float4 *nhi,
-                              const int *parent, int *left, int *right, int *rfirst, uint32_t *order_out,
-                              float4 *leaf_lo, float4 *leaf_hi, int *parent_out) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= 2 * n - 1) return;
-    if (x >= n - 1) {
-        const int q = offs[x];
-        order_out[q] = order[x - (n - 1)];
-        leaf_lo[q] = nlo[x];
-        leaf_hi[q] = nhi[x];
-        parent_out[n - 1 + q] = parent[x];
-    } else {
-        parent_out[x] = parent[x];
-        rfirst[x] = offs[x];
-        const int l = left[x], r = right[x];
-        left[x] = l >= n - 1 ? n - 1 + offs[l] : l;
-        right[x] = r >= n - 1 ? n - 1 + offs[r] : r;
+    if (tid == 0) {
+        bc->nodes = ctr;
+        if (m != 1 || ctr != (uint32_t)(t.n - 1)) bc->fail = 1;
     }
 }
 
@@ -518,165 +746,175 @@ __device__ __forceinline__ void write_slot(float *node, int c, float3 lo, float3
     node[6 * K + c] = __int_as_float(count > 0 ? ptd::make_leaf(child, count) : child);
 }
 __device__ __forceinline__ int item_count(int item) { return ptd::is_leaf(item) ? ptd::leaf_count(item) : 0; }
-template <int K>
-__device__ __forceinline__ void write_empty(float *node, int c) {
-    write_slot<K>(node, c, f3(1e30f, 1e30f, 1e30f), f3(1e30f, 1e30f, 1e30f), ptd::kNoItem, 0);
+// The primitives of leaf x (at most 15), depth first, from position `first` on.
+__device__ __forceinline__ void leaf_positions(const Tree &t, int x, int first, const uint32_t *order,
+                                               uint32_t *leaf_order) {
+    int st[16];
+    int sp = 0;
+    for (;;) {
+        if (x >= t.n - 1) {
+            leaf_order[first++] = order[x - (t.n - 1)];
+            if (sp == 0) return;
+            x = st[--sp];
+        } else {
+            const int4 l = t.links[x];
+            if (sp < 16) st[sp++] = l.y;  // (15 primitives: at most 14 pending)
+            x = l.x;
+        }
+    }
 }
 
-// 6. SAH-optimal wide collapse (Ylitie, Karras and Laine, HPG 2017): for
-// every binary node x and i = 1..K, S(x, i) is the cheapest way to represent
-// its subtree with at most i slots of a wide parent:
-//   S(x, 1) = min(leaf: area * primitive weight (if count <= max_leaf),
-//                 wide node: 1.2 * area + min_j S(l, j) + S(r, K - j))
-//   S(x, i) = min(S(x, i - 1), min_j S(l, j) + S(r, i - j))
-// computed bottom up (second arrival processes a node).  dsel[8x] keeps the
-// wide node's split j, dsel[8x + i - 1] the split for i = 2..K slots (0: use
-// i - 1 slots), and nleaf[x] the leaf-or-wide choice; the collapse below
-// follows them.
+// 6. one level of the collapse, following the choices of form_node: the wide
+// node of binary node b gets the slots of left(b) (choice 0 of them) and
+// right(b) (the rest), each expanded while its choice splits it further.  The
+// wide nodes of level L are [start, start + level[L]); their inner children,
+// appended by one atomic per warp, follow them.  wide[w]: binary node of wide
+// node w and the position of its first primitive in leaf order (depth first:
+// a right subtree follows its left one), which the leaves found here get.
+// Also sums the SAH cost of what it writes.  A small level's time is the chain
+// of one thread's dependent loads, hence one 16-byte record per binary node.
 template <int K>
-__global__ void k_wide_dp(int n, const int *left, const int *right, const int *parent, const float4 *nlo,
-                          const float4 *nhi, const int *ncount, const float *nwt, float *dval, uint8_t *dsel,
-                          int *nleaf, int *flags, int max_leaf) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    const int leaf = n - 1 + k;
-    const float v = half_area(nlo[leaf], nhi[leaf]) * nwt[leaf];
-#pragma unroll
-    for (int i = 0; i < K; i++) dval[(size_t)leaf * 8 + i] = v;
-    int cur = parent[leaf];
-    while (cur >= 0) {
-        __threadfence();
-        if (atomicAdd(&flags[cur], 1) == 0) return;
-        __threadfence();
-        const int l = left[cur], r = right[cur];
-        float sl[K + 1], sr[K + 1], sx[K + 1];
-#pragma unroll
-        for (int i = 1; i <= K; i++) {
-            sl[i] = __ldcg(&dval[(size_t)l * 8 + i - 1]);
-            sr[i] = __ldcg(&dval[(size_t)r * 8 + i - 1]);
-        }
-        const float area = half_area(nlo[cur], nhi[cur]);
-        float best = FLT_MAX;
-        int jw = 1;
-#pragma unroll
-        for (int j = 1; j < K; j++) {
-            const float c = sl[j] + sr[K - j];
-            if (c < best) {
-                best = c;
-                jw = j;
-            }
-        }
-        const float c_wide = kCostNode * area + best;
-        const float c_leaf = ncount[cur] <= max_leaf ? area * nwt[cur] : FLT_MAX;
-        const bool mk_leaf = c_leaf <= c_wide;
-        sx[1] = mk_leaf ? c_leaf : c_wide;
-        dsel[(size_t)cur * 8] = (uint8_t)jw;
-#pragma unroll
-        for (int i = 2; i <= K; i++) {
-            float vi = sx[i - 1];
-            int sel = 0;
-#pragma unroll
-            for (int j = 1; j < i; j++) {
-                const float c = sl[j] + sr[i - j];
-                if (c < vi) {
-                    vi = c;
-                    sel = j;
+__global__ void __launch_bounds__(128) k_collapse(const Tree t, BuildCounts *bc, int level, int root, int2 *wide,
+                                                  float *nodes, float scene_mag, const uint32_t *order,
+                                                  uint32_t *leaf_order) {
+    __shared__ uint32_t s_start;
+    __shared__ double s_sah;
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    if (bc->fail) return;  // uniform
+    const uint32_t count = bc->level[level];
+    if (blockIdx.x * blockDim.x >= count) return;  // uniform
+    if (threadIdx.x == 0) s_sah = 0.0;
+    if (threadIdx.x < 32) {
+        uint32_t v = 0;
+        for (int l = lane; l < level; l += 32) v += bc->level[l];
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
+        if (lane == 0) s_start = v;
+    }
+    __syncthreads();
+    const uint32_t start = s_start;
+    const int n = t.n;
+    double sah = 0.0;
+    for (uint32_t k0 = blockIdx.x * blockDim.x; k0 < count; k0 += gridDim.x * blockDim.x) {  // uniform per block
+        const uint32_t k = k0 + threadIdx.x;
+        const bool valid = k < count;
+        int slot[K], first[K];  // binary node and first position of each slot
+        int ns = 0;
+        uint32_t inner = 0;  // bit c: slot c is an inner node
+        if (valid) {
+            const int2 w = level == 0 ? make_int2(root, 0) : wide[start + k];
+            const int4 lb = w.x < n - 1 ? t.links[w.x] : make_int4(0, 0, (int)kSelLeaf, 0);
+            if (level == 0 && (lb.z & (int)kSelLeaf)) {  // the whole scene is one leaf
+                slot[0] = w.x;
+                first[0] = 0;
+                ns = 1;
+            } else {
+                int stn[K], sti[K], stf[K];  // pending (node, slots, first position); their slots sum to at most K
+                int sp = 0;
+                const int jw = sel_of(lb.z, 0);
+                stn[sp] = lb.y;
+                stf[sp] = w.y + lb.w;
+                sti[sp++] = K - jw;
+                stn[sp] = lb.x;
+                stf[sp] = w.y;
+                sti[sp++] = jw;
+                while (sp > 0) {
+                    --sp;
+                    const int x = stn[sp], f0 = stf[sp];
+                    int si = sti[sp];
+                    const int4 lx = x < n - 1 ? t.links[x] : make_int4(0, 0, (int)kSelLeaf, 0);
+                    while (si > 1 && sel_of(lx.z, si - 1) == 0) si--;
+                    if (si <= 1 || sp + 2 > K) {  // (the stack cannot overflow: its slots sum to at most K)
+                        if (ns < K) {
+                            if (!(lx.z & (int)kSelLeaf)) inner |= 1u << ns;
+                            first[ns] = f0;
+                            slot[ns++] = x;
+                        }
+                        continue;
+                    }
+                    const int pick = sel_of(lx.z, si - 1);
+                    stn[sp] = lx.y;
+                    stf[sp] = f0 + lx.w;
+                    sti[sp++] = si - pick;
+                    stn[sp] = lx.x;
+                    stf[sp] = f0;
+                    sti[sp++] = pick;
                 }
             }
-            sx[i] = vi;
-            dsel[(size_t)cur * 8 + i - 1] = (uint8_t)sel;
         }
+        // ids of the inner children
+        const uint32_t mine = __popc(inner);
+        uint32_t x = mine;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(FULL, x, o);
+            if (lane >= o) x += y;
+        }
+        uint32_t at = 0;
+        if (lane == 31 && x) at = atomicAdd(&bc->level[level + 1], x);
+        uint32_t child = start + count + __shfl_sync(FULL, at, 31) + x - mine;
+        if (!valid) continue;
+        float f[8 * K];
+        float3 rlo = f3(FLT_MAX, FLT_MAX, FLT_MAX), rhi = f3(-FLT_MAX, -FLT_MAX, -FLT_MAX);
 #pragma unroll
-        for (int i = 1; i <= K; i++) dval[(size_t)cur * 8 + i - 1] = sx[i];
-        nleaf[cur] = mk_leaf ? 1 : 0;
-        cur = parent[cur];
+        for (int c = 0; c < K; c++) {
+            float3 lo = f3(1e30f, 1e30f, 1e30f), hi = lo;  // empty slot: a point box far away
+            int item = ptd::kNoItem;
+            if (c < ns) {
+                const int y = slot[c];
+                const NodeBox b = load_box(t.nb, y);
+                padded(b.lo, b.hi, scene_mag, lo, hi);
+                const float ex = hi.x - lo.x, ey = hi.y - lo.y, ez = hi.z - lo.z;
+                const float a = ex * ey + ey * ez + ez * ex;
+                if ((inner >> c) & 1u) {
+                    item = (int)child;
+                    wide[child++] = make_int2(y, first[c]);
+                    sah += (double)a * (double)kCostNode;
+                } else {
+                    item = ptd::make_leaf(first[c], b.count());
+                    leaf_positions(t, y, first[c], order, leaf_order);
+                    sah += (double)a * (double)kCostPrim * b.count();
+                }
+                rlo = f3(fminf(rlo.x, lo.x), fminf(rlo.y, lo.y), fminf(rlo.z, lo.z));
+                rhi = f3(fmaxf(rhi.x, hi.x), fmaxf(rhi.y, hi.y), fmaxf(rhi.z, hi.z));
+            }
+            f[c] = lo.x;
+            f[K + c] = hi.x;
+            f[2 * K + c] = lo.y;
+            f[3 * K + c] = hi.y;
+            f[4 * K + c] = lo.z;
+            f[5 * K + c] = hi.z;
+            f[6 * K + c] = __int_as_float(item);
+            f[7 * K + c] = 0.f;
+        }
+        float4 *node = reinterpret_cast<float4 *>(nodes) + (size_t)(start + k) * 2 * K;
+#pragma unroll
+        for (int i = 0; i < K; i++)
+            ptd::st8(node + 2 * i, make_float4(f[8 * i], f[8 * i + 1], f[8 * i + 2], f[8 * i + 3]),
+                     make_float4(f[8 * i + 4], f[8 * i + 5], f[8 * i + 6], f[8 * i + 7]));
+        if (level == 0) {
+            const double ex = rhi.x - rlo.x, ey = rhi.y - rlo.y, ez = rhi.z - rlo.z;
+            bc->root_area = ex * ey + ey * ez + ez * ex;
+        }
     }
+    for (int o = 16; o > 0; o >>= 1) sah += __shfl_xor_sync(FULL, sah, o);
+    if (lane == 0) atomicAdd(&s_sah, sah);
+    __syncthreads();
+    if (threadIdx.x == 0) atomicAdd(&bc->sah, s_sah);
 }
 
-// 6'. one level of the collapse, following the choices of k_wide_dp: the
-// wide node of binary node b gets the slots of left(b) (dsel[8b] of them) and
-// right(b) (the rest), each expanded while its choice splits it further.
+// A scene without primitives: one node of empty slots.
 template <int K>
-__global__ void k_collapse_dp(int n, const int2 *items_in, const uint32_t *n_in_ptr, int2 *items_out, uint32_t *n_out,
-                              uint32_t *n_wide, float *nodes, const int *left, const int *right, const int *rfirst,
-                              const float4 *nlo, const float4 *nhi, const int *ncount, const int *nleaf,
-                              const uint8_t *dsel, float scene_mag) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= *n_in_ptr) return;
-    const int2 it = items_in[t];
-    const int b = it.y;
-    int slot[K];
-    int ns = 0;
-    int stn[K], sti[K];  // pending (node, slots); their slots sum to at most K
-    int sp = 0;
-    const int jw = dsel[(size_t)b * 8];
-    stn[sp] = right[b];
-    sti[sp++] = K - jw;
-    stn[sp] = left[b];
-    sti[sp++] = jw;
-    while (sp > 0) {
-        --sp;
-        const int x = stn[sp];
-        int si = sti[sp];
-        if (x < n - 1) {
-            while (si > 1 && dsel[(size_t)x * 8 + si - 1] == 0) si--;
-        }
-        if (x >= n - 1 || si <= 1) {
-            if (ns < K) slot[ns++] = x;
-            continue;
-        }
-        const int sel = dsel[(size_t)x * 8 + si - 1];
-        if (sp + 2 > K) {  // cannot happen (slots on the stack sum to at most K)
-            if (ns < K) slot[ns++] = x;
-            continue;
-        }
-        stn[sp] = right[x];
-        sti[sp++] = si - sel;
-        stn[sp] = left[x];
-        sti[sp++] = sel;
-    }
-    float *node = nodes + (size_t)it.x * 8 * K;
-    for (int c = 0; c < K; c++) {
-        if (c >= ns) {
-            write_empty<K>(node, c);
-            continue;
-        }
-        const int x = slot[c];
-        float3 lo, hi;
-        padded(nlo[x], nhi[x], scene_mag, lo, hi);
-        if (x >= n - 1) {
-            write_slot<K>(node, c, lo, hi, x - (n - 1), 1);
-        } else if (nleaf[x]) {
-            write_slot<K>(node, c, lo, hi, rfirst[x], ncount[x]);
-        } else {
-            const uint32_t w = atomicAdd(n_wide, 1u);
-            const uint32_t q = atomicAdd(n_out, 1u);
-            items_out[q] = make_int2((int)w, x);
-            write_slot<K>(node, c, lo, hi, (int)w, 0);
-        }
-    }
+__global__ void k_empty_root(float *nodes) {
+    if (threadIdx.x < 8 * K)
+        nodes[threadIdx.x] = threadIdx.x < 6 * K ? 1e30f : threadIdx.x < 7 * K ? __int_as_float(ptd::kNoItem) : 0.f;
 }
 
-// Root that is a single leaf (tiny scenes): one wide node, slot 0 = all primitives.
-template <int K>
-__global__ void k_leaf_root(float *nodes, int n, const float4 *nlo, const float4 *nhi, int root, float scene_mag) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    for (int c = 0; c < K; c++) write_empty<K>(nodes, c);
-    if (n > 0) {
-        float3 lo, hi;
-        padded(nlo[root], nhi[root], scene_mag, lo, hi);
-        write_slot<K>(nodes, 0, lo, hi, 0, n);
-    }
-}
-
-// 7. primitive records into leaf order.
+// 7. primitive records into leaf order, one float4 a thread.
 __global__ void k_gather_prims(const float4 *src, const uint32_t *order, uint32_t n, float4 *dst) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    uint32_t p = order[i];
-    dst[3 * (size_t)i] = src[3 * (size_t)p];
-    dst[3 * (size_t)i + 1] = src[3 * (size_t)p + 1];
-    dst[3 * (size_t)i + 2] = src[3 * (size_t)p + 2];
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t k = i / 3, j = i - 3 * k;
+    if (k >= n) return;
+    dst[3 * (size_t)k + j] = src[3 * (size_t)order[k] + j];
 }
 
 // SAH cost of the wide tree: sum over slots of area * (node or primitive cost).
@@ -903,98 +1141,105 @@ __global__ void k_compress8(const float *nodes, uint32_t n, float4 *out) {
     }
 }
 
+// Scratch of a build: one allocation, carved.
 struct Scratch {
     uint64_t *keys[2];
     uint32_t *vals[2];
-    uint32_t *hist;
-    float4 *plo, *phi;
-    int *left, *right, *parent, *rfirst, *ncount, *nleaf, *flags;
-    float4 *nlo, *nhi;
-    float *ncost, *nwt;  // SAH cost and summed primitive cost weight of each binary node
-    int2 *items[2];
-    uint32_t *counters;  // [0..5] centroid bounds, [6] n_wide, [7] n_out0, [8] n_out1, [9] PLOC nodes, [10] PLOC failure
-    double *sah;
-    int *cl[2], *nn, *out_id, *offs;  // PLOC clusters, neighbours, merge results, depth-first positions
-    uint32_t *keep, *order2, *bsum;  // survival flags, permuted order, per-block survivor counts
-    int *par2;                       // parents renumbered with the leaves
-    float *dval;                     // wide-collapse costs S(x, 1..8)
-    uint8_t *dsel;                   // wide-collapse choices
-    float4 *leaf_lo, *leaf_hi;
+    uint32_t *hist, *digit_total;
+    float4 *pbox;
+    int *parent, *flags;  // radix tree only
+    int *cl[2], *out_id;  // PLOC
+    uint32_t *tile_count;
+    int2 *wide;           // of each wide node: its binary node, its first primitive's position
+    Tree tree;
+    BuildCounts *counts;
 };
 
-template <class T>
-T *carve(char *&p, size_t count) {
-    T *r = reinterpret_cast<T *>(p);
-    size_t bytes = (count * sizeof(T) + 255) & ~size_t(255);
-    p += bytes;
-    return r;
-}
-size_t carve_size(size_t n, uint32_t tiles) {
-    size_t t = 0;
-    auto add = [&](size_t bytes) { t += (bytes + 255) & ~size_t(255); };
-    add(8 * n); add(8 * n); add(4 * n); add(4 * n);
-    add(4 * (size_t)256 * tiles);
-    add(16 * n); add(16 * n);
-    add(4 * n); add(4 * n); add(4 * 2 * n); add(4 * n); add(4 * 2 * n); add(4 * 2 * n); add(4 * n);
-    add(16 * 2 * n); add(16 * 2 * n);
-    add(4 * 2 * n);
-    add(8 * n); add(8 * n);
-    add(64); add(64);
-    add(4 * n); add(4 * n); add(4 * n); add(4 * n); add(4 * 2 * n);
-    add(4 * (n + 1)); add(4 * n);
-    add(16 * n); add(16 * n);
-    add(4 * 2 * n);
-    add(4 * (n / 1024 + 2));
-    add(4 * 2 * n); add(4 * 8 * 2 * n); add(8 * 2 * n);
-    return t;
+// Carves the scratch for n primitives from base; returns the bytes taken.
+size_t carve(Scratch &sc, char *base, size_t n, uint32_t tiles, int K) {
+    size_t at = 0;
+    auto take = [&](auto *&p, size_t count) {
+        using T = std::remove_reference_t<decltype(*p)>;
+        p = reinterpret_cast<T *>(base + at);
+        at += (count * sizeof(T) + 255) & ~size_t(255);
+    };
+    take(sc.counts, 1);
+    take(sc.keys[0], n);
+    take(sc.keys[1], n);
+    take(sc.vals[0], n);
+    take(sc.vals[1], n);
+    take(sc.hist, (size_t)256 * tiles);
+    take(sc.digit_total, 256);
+    take(sc.pbox, 2 * n);
+    take(sc.parent, 2 * n);
+    take(sc.flags, n);
+    take(sc.cl[0], n);
+    take(sc.cl[1], n);
+    take(sc.out_id, n);
+    take(sc.tile_count, n / ploc_tile(1) + 1);
+    take(sc.wide, n);
+    take(sc.tree.links, n);
+    take(sc.tree.nb, 4 * n);
+    take(sc.tree.dval, (size_t)K * n);
+    return at;
 }
 
+// The collapse, the records in leaf order and the counts (level_start, SAH
+// cost, *sah) read back.  *ok = false: clustering failed, or the wide tree is
+// deeper than max_levels.
 template <int K>
-int build_wide(pt_scene *s, const Scratch &sc, uint32_t n, int root, int max_leaf, cudaStream_t st) {
+int build_wide(pt_scene *s, const Scratch &sc, uint32_t n, int root, uint32_t max_levels, float *sah, bool *ok,
+               cudaStream_t st) {
+    *ok = true;
     s->level_start.clear();
-    size_t node_bytes = (size_t)std::max<uint32_t>(1, n > 1 ? n - 1 : 1) * 32 * K;
-    int e = s->nodes.ensure(node_bytes);
+    int e = s->nodes.ensure((size_t)std::max<uint32_t>(1, n > 1 ? n - 1 : 1) * 32 * K);
     if (e != PT_OK) return e;
     float *nodes = s->nodes.as<float>();
-    const int tb = 256;
-    if (n > 1) {  // SAH-optimal slot assignment for this width (also the final leaf decisions)
-        PT_CUDA_TRY(cudaMemsetAsync(sc.flags, 0, 4 * (size_t)n, st));
-        k_wide_dp<K><<<blocks(n, tb), tb, 0, st>>>((int)n, sc.left, sc.right, sc.parent, sc.nlo, sc.nhi, sc.ncount,
-                                                   sc.nwt, sc.dval, sc.dsel, sc.nleaf, sc.flags, max_leaf);
+    if (n == 0) {
+        k_empty_root<K><<<1, 64, 0, st>>>(nodes);
         PT_CUDA_TRY(cudaGetLastError());
-    }
-    // root: binary node `root` (internal), or the single leaf (node 0 when n == 1)
-    int root_leaf = 0;
-    if (n > 1) PT_CUDA_TRY(cudaMemcpyAsync(&root_leaf, sc.nleaf + root, sizeof(int), cudaMemcpyDeviceToHost, st));
-    PT_CUDA_TRY(cudaStreamSynchronize(st));
-    if (n <= 1 || root_leaf) {
-        k_leaf_root<K><<<1, 32, 0, st>>>(nodes, (int)n, sc.nlo, sc.nhi, n > 1 ? root : 0, s->scene_mag);
         s->level_start = {0, 1};
+        *sah = 0.f;
         return PT_OK;
     }
-    uint32_t h_init[3] = {1, 1, 0};  // n_wide = 1 (root), n_out0 = 1 (root item), n_out1 = 0
-    PT_CUDA_TRY(cudaMemcpyAsync(sc.counters + 6, h_init, sizeof(h_init), cudaMemcpyHostToDevice, st));
-    int2 root_item = make_int2(0, root);
-    PT_CUDA_TRY(cudaMemcpyAsync(sc.items[0], &root_item, sizeof(int2), cudaMemcpyHostToDevice, st));
-    uint32_t level_count = 1, start = 0;
-    int cur = 0;
-    while (level_count > 0) {
-        s->level_start.push_back(start);
-        uint32_t *n_in = sc.counters + 7 + cur, *n_out = sc.counters + 7 + (cur ^ 1);
-        PT_CUDA_TRY(cudaMemsetAsync(n_out, 0, sizeof(uint32_t), st));
-        k_collapse_dp<K><<<blocks(level_count, tb), tb, 0, st>>>((int)n, sc.items[cur], n_in, sc.items[cur ^ 1], n_out,
-                                                                sc.counters + 6, nodes, sc.left, sc.right, sc.rfirst,
-                                                                sc.nlo, sc.nhi, sc.ncount, sc.nleaf, sc.dsel,
-                                                                s->scene_mag);
+    BuildCounts *bc = sc.counts;
+    PT_CUDA_TRY(cudaMemsetAsync(&bc->sah, 0, 2 * sizeof(double) + sizeof(bc->level), st));
+    const uint32_t one = 1;
+    PT_CUDA_TRY(cudaMemcpyAsync(bc->level, &one, sizeof(one), cudaMemcpyHostToDevice, st));
+    // levels in batches; a launch past the last level returns at once
+    constexpr int kBatch = 20;
+    BuildCounts h;
+    const size_t head = offsetof(BuildCounts, clusters);
+    const uint32_t most = std::min<uint32_t>(blocks(n, 128), (uint32_t)s->num_sms * 16u);
+    uint32_t bound = 1;  // nodes of a level: at most K times the level above, and n - 1
+    int level = 0;
+    for (bool more = true; more && level < kMaxLevels;) {
+        const int end = std::min(level + (level ? 8 : kBatch), kMaxLevels);
+        for (; level < end; level++) {
+            k_collapse<K><<<std::min(most, blocks(bound, 128)), 128, 0, st>>>(sc.tree, bc, level, root, sc.wide, nodes,
+                                                                             s->scene_mag, sc.vals[0],
+                                                                             s->bvh_order.as<uint32_t>());
+            bound = std::min<uint32_t>(n, bound * K);
+        }
         PT_CUDA_TRY(cudaGetLastError());
-        uint32_t nxt = 0;
-        PT_CUDA_TRY(cudaMemcpyAsync(&nxt, n_out, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+        PT_CUDA_TRY(cudaMemcpyAsync(&h, bc, head, cudaMemcpyDeviceToHost, st));
         PT_CUDA_TRY(cudaStreamSynchronize(st));
-        start += level_count;
-        level_count = nxt;
-        cur ^= 1;
+        more = !h.fail && h.level[end] != 0;
+    }
+    uint32_t start = 0;
+    for (int l = 0; l <= kMaxLevels && h.level[l]; l++) {
+        s->level_start.push_back(start);
+        start += h.level[l];
     }
     s->level_start.push_back(start);
+    if (h.fail || h.level[kMaxLevels] || s->level_start.size() - 1 > max_levels) {
+        *ok = false;
+        return PT_OK;
+    }
+    k_gather_prims<<<blocks(3 * (size_t)n, 256), 256, 0, st>>>(s->prims_world.as<float4>(), s->bvh_order.as<uint32_t>(),
+                                                               n, s->prims_bvh.as<float4>());
+    PT_CUDA_TRY(cudaGetLastError());
+    *sah = h.root_area > 0 ? (float)((kCostNode * h.root_area + h.sah) / h.root_area) : 0.f;
     return PT_OK;
 }
 
@@ -1030,60 +1275,117 @@ int compute_sah(pt_scene *s, double *scratch2, cudaStream_t st, float &out) {
     return PT_OK;
 }
 
-// PLOC over the sorted order in s->bvh_order (n >= 2).  Returns PT_OK with
-// the binary root in *root, or PT_OK with *root = -1 when clustering stalls
-// (ties in degenerate scenes) or the tree is deeper than the traversal can
-// handle; the caller then builds the radix tree instead.
-int ploc_build(pt_scene *s, const Scratch &sc, uint32_t n, int max_leaf, cudaStream_t st, int *root) {
-    *root = -1;
-    const int tb = 256;
-    uint32_t *order = s->bvh_order.as<uint32_t>();
-    PT_CUDA_TRY(cudaMemsetAsync(sc.parent, 0xff, 4 * (2 * (size_t)n - 1), st));
-    PT_CUDA_TRY(cudaMemsetAsync(sc.counters + 9, 0, 2 * sizeof(uint32_t), st));
-    k_ploc_init<<<blocks(n, tb), tb, 0, st>>>((int)n, order, s->prims_world.as<float4>(), sc.plo, sc.phi, sc.nlo,
-                                              sc.nhi, sc.ncount, sc.ncost, sc.nwt, sc.nleaf, sc.cl[0]);
-    PT_CUDA_TRY(cudaGetLastError());
-    uint32_t m = n;
-    int cur = 0;
-    int log2n = 0;
-    while ((1u << log2n) < n) log2n++;
-    const int max_passes = 64 + 8 * log2n;
-    for (int pass = 0; m > 1; pass++) {
-        if (pass >= max_passes) return PT_OK;  // too slow to converge: radix tree
-        k_ploc_nn<<<blocks(m, kPlocBlock), kPlocBlock, 0, st>>>((int)m, sc.cl[cur], sc.nlo, sc.nhi, sc.nn);
-        k_ploc_merge<<<blocks(m, tb), tb, 0, st>>>((int)m, sc.cl[cur], sc.nn, sc.keep, sc.out_id, sc.counters + 9,
-                                                   sc.left, sc.right, sc.parent, sc.nlo, sc.nhi, sc.ncount, sc.ncost,
-                                                   sc.nwt, sc.nleaf, max_leaf);
-        const uint32_t nb = (m + kCompactBlock - 1) / kCompactBlock;
-        k_ploc_block_counts<<<nb, kCompactBlock, 0, st>>>((int)m, sc.keep, sc.bsum);
-        PT_CUDA_TRY(cudaMemsetAsync(sc.bsum + nb, 0, sizeof(uint32_t), st));
-        k_scan_excl<<<1, 1024, 0, st>>>(sc.bsum, nb + 1);
-        k_ploc_compact<<<nb, kCompactBlock, 0, st>>>((int)m, sc.keep, sc.bsum, sc.out_id, sc.cl[cur ^ 1]);
+// PLOC over the sorted order in sc.vals[0] (n >= 2); the root is node n - 2.
+// *stalled: clustering made no progress (boxes without a finite area); the
+// caller then builds the radix tree.
+template <int K>
+int ploc_build(const Scratch &sc, uint32_t n, bool *stalled, cudaStream_t st) {
+    *stalled = false;
+    BuildCounts *bc = sc.counts;
+    PT_CUDA_TRY(cudaMemcpyAsync(bc->clusters, &n, sizeof(n), cudaMemcpyHostToDevice, st));
+    uint32_t bound = n;  // clusters, at most
+    int cur = 0, pass = 0;
+    while (bound > (uint32_t)kPlocTail) {
+        if (pass + kPlocPassesPerRead > kPlocMaxPasses) {
+            *stalled = true;
+            return PT_OK;
+        }
+        const bool wide = bound >= kPlocWide;
+        const uint32_t tile = (uint32_t)ploc_tile(wide ? 4 : 1), tiles = (bound + tile - 1) / tile;
+        for (int k = 0; k < kPlocPassesPerRead; k++, pass++, cur ^= 1) {
+            if (wide) {
+                k_ploc_merge<K, 4><<<tiles, kPlocThreads, 0, st>>>(sc.tree, bc, pass, sc.cl[cur], sc.out_id,
+                                                                  sc.tile_count);
+                k_ploc_compact<4><<<tiles, kPlocThreads, 0, st>>>(bc, pass, sc.out_id, sc.tile_count, sc.cl[cur ^ 1]);
+            } else {
+                k_ploc_merge<K, 1><<<tiles, kPlocThreads, 0, st>>>(sc.tree, bc, pass, sc.cl[cur], sc.out_id,
+                                                                  sc.tile_count);
+                k_ploc_compact<1><<<tiles, kPlocThreads, 0, st>>>(bc, pass, sc.out_id, sc.tile_count, sc.cl[cur ^ 1]);
+            }
+        }
         PT_CUDA_TRY(cudaGetLastError());
-        uint32_t next = 0;
-        PT_CUDA_TRY(cudaMemcpyAsync(&next, sc.bsum + nb, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+        uint32_t m = 0;
+        PT_CUDA_TRY(cudaMemcpyAsync(&m, bc->clusters + pass, sizeof(m), cudaMemcpyDeviceToHost, st));
         PT_CUDA_TRY(cudaStreamSynchronize(st));
-        if (next == 0 || next >= m) return PT_OK;  // cannot happen (the closest pair always merges)
-        m = next;
-        cur ^= 1;
+        if (m == 0 || m >= bound) {
+            *stalled = true;
+            return PT_OK;
+        }
+        bound = m;
     }
-    const uint32_t nodes2 = 2 * n - 1;
-    k_ploc_offsets<<<blocks(nodes2, tb), tb, 0, st>>>((int)n, sc.left, sc.right, sc.parent, sc.ncount, sc.offs,
-                                                     sc.counters + 10);
-    k_ploc_finish<<<blocks(nodes2, tb), tb, 0, st>>>((int)n, sc.offs, order, sc.nlo, sc.nhi, sc.parent, sc.left,
-                                                    sc.right, sc.rfirst, sc.order2, sc.leaf_lo, sc.leaf_hi, sc.par2);
+    constexpr int smem = (kPlocTail + 2 * kPlocRadius) * 32 + kPlocTail * 8;
+    PT_CUDA_TRY(cudaFuncSetAttribute(k_ploc_tail<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    k_ploc_tail<K><<<1, 1024, smem, st>>>(sc.tree, bc, pass, sc.cl[cur]);
     PT_CUDA_TRY(cudaGetLastError());
-    PT_CUDA_TRY(cudaMemcpyAsync(sc.parent, sc.par2, 4 * (size_t)nodes2, cudaMemcpyDeviceToDevice, st));
-    PT_CUDA_TRY(cudaMemcpyAsync(order, sc.order2, 4 * (size_t)n, cudaMemcpyDeviceToDevice, st));
-    PT_CUDA_TRY(cudaMemcpyAsync(sc.nlo + (n - 1), sc.leaf_lo, 16 * (size_t)n, cudaMemcpyDeviceToDevice, st));
-    PT_CUDA_TRY(cudaMemcpyAsync(sc.nhi + (n - 1), sc.leaf_hi, 16 * (size_t)n, cudaMemcpyDeviceToDevice, st));
-    uint32_t h[2] = {0, 0};
-    int r = -1;
-    PT_CUDA_TRY(cudaMemcpyAsync(h, sc.counters + 9, sizeof(h), cudaMemcpyDeviceToHost, st));
-    PT_CUDA_TRY(cudaMemcpyAsync(&r, sc.cl[cur], sizeof(int), cudaMemcpyDeviceToHost, st));
-    PT_CUDA_TRY(cudaStreamSynchronize(st));
-    if (h[1] != 0 || h[0] != n - 1) return PT_OK;  // too deep (or incomplete): radix tree
-    *root = r;
+    return PT_OK;
+}
+
+template <int K>
+int build_tree(pt_scene *s, const pt_bvh_opts *o, cudaStream_t st, float *sah, bool *clustered) {
+    const uint32_t n = s->num_prims;
+    const uint32_t tiles = std::max<uint32_t>(1, (n + kSortTile - 1) / kSortTile);
+    const size_t nn = std::max<uint32_t>(n, 2);
+    Scratch sc;
+    int e = s->bvh_scratch.ensure(carve(sc, nullptr, nn, tiles, K));
+    if (e != PT_OK) return e;
+    carve(sc, static_cast<char *>(s->bvh_scratch.ptr), nn, tiles, K);
+    sc.tree.n = (int)n;
+    sc.tree.max_leaf = (int)o->max_leaf_size;
+    if ((e = s->bvh_order.ensure(std::max<size_t>(4 * (size_t)n, 16))) != PT_OK) return e;
+    if ((e = s->prims_bvh.ensure(std::max<size_t>(48 * (size_t)n, 48))) != PT_OK) return e;
+
+    const int tb = 256;
+    PT_CUDA_TRY(cudaMemsetAsync(sc.counts, 0, sizeof(BuildCounts), st));
+    PT_CUDA_TRY(cudaMemsetAsync(sc.counts->centroid, 0xff, 3 * sizeof(uint32_t), st));
+    if (n > 0) {
+        k_prim_bounds<<<std::min<uint32_t>(blocks(n, tb), (uint32_t)s->num_sms * 8u), tb, 0, st>>>(s->prims_world.as<float4>(), n, sc.pbox, sc.counts->centroid);
+        k_morton<<<blocks(n, tb), tb, 0, st>>>(sc.pbox, n, sc.counts->centroid, sc.keys[0], sc.vals[0]);
+        PT_CUDA_TRY(cudaFuncSetAttribute(k_radix_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, kScatterSmem));
+        for (int pass = 0, cur = 0; pass < 8; pass++, cur ^= 1) {  // back in buffer 0 after 8 passes
+            const int shift = pass * 8;
+            k_radix_hist<<<tiles, kSortThreads, 0, st>>>(sc.keys[cur], n, shift, sc.hist, tiles);
+            k_radix_scan<<<256, 256, 0, st>>>(sc.hist, tiles, sc.digit_total);
+            k_radix_scatter<<<tiles, kSortThreads, kScatterSmem, st>>>(sc.keys[cur], sc.vals[cur], sc.keys[cur ^ 1], sc.vals[cur ^ 1],
+                                                             n, shift, sc.hist, tiles, sc.digit_total);
+        }
+        k_leaf_boxes<<<blocks(n, tb), tb, 0, st>>>((int)n, sc.vals[0], sc.pbox, sc.tree.nb, sc.cl[0]);
+        PT_CUDA_TRY(cudaGetLastError());
+    }
+    // binary tree: PLOC by default, the radix tree for PT_BVH_FAST_BUILD, for
+    // a PLOC build that did not converge, or one whose wide tree is deeper
+    // than the traversal stack covers (kShortStack + kSpillStack entries)
+    const auto radix_tree = [&]() -> int {
+        PT_CUDA_TRY(cudaMemsetAsync(&sc.counts->fail, 0, sizeof(uint32_t), st));
+        if (n == 0) return PT_OK;  // no primitives: nothing to sort or link (2n - 1 would wrap)
+        PT_CUDA_TRY(cudaMemsetAsync(sc.parent, 0xff, 4 * (2 * (size_t)n - 1), st));
+        PT_CUDA_TRY(cudaMemsetAsync(sc.flags, 0, 4 * (size_t)n, st));
+        if (n > 1)
+            k_karras<<<blocks(n - 1, tb), tb, 0, st>>>(sc.keys[0], (int)n, sc.tree.links, sc.parent);
+        k_bottom_up<K><<<blocks(n, tb), tb, 0, st>>>(sc.tree, sc.parent, sc.flags);
+        PT_CUDA_TRY(cudaGetLastError());
+        return PT_OK;
+    };
+    // curve pieces (long, thin, often diagonal) trace faster under the radix
+    // tree although PLOC gives them a lower SAH cost (50 k-strand hair at
+    // 1080p: 341 vs 320 Msamples/s), so curve-dominated scenes use it
+    const bool curve_heavy = 2ull * s->num_curve_pieces > n;
+    *clustered = n > 1 && !(o->flags & PT_BVH_FAST_BUILD) && !curve_heavy;
+    if (*clustered) {
+        bool stalled = false;
+        if ((e = ploc_build<K>(sc, n, &stalled, st)) != PT_OK) return e;
+        bool ok = false;
+        const uint32_t stack_levels = (uint32_t)ptd::kTraversalStackEntries / (uint32_t)(K - 1);
+        if (!stalled && (e = build_wide<K>(s, sc, n, (int)n - 2, stack_levels, sah, &ok, st)) != PT_OK) return e;
+        if (ok) return PT_OK;
+        *clustered = false;
+    }
+    if ((e = radix_tree()) != PT_OK) return e;
+    bool ok = false;
+    if ((e = build_wide<K>(s, sc, n, 0, kMaxLevels, sah, &ok, st)) != PT_OK) return e;
+    if (!ok) {
+        pt_set_error("pt_bvh_build: the tree is deeper than %d levels", kMaxLevels);
+        return PT_ERR_UNSUPPORTED;
+    }
     return PT_OK;
 }
 
@@ -1092,118 +1394,17 @@ int ploc_build(pt_scene *s, const Scratch &sc, uint32_t n, int max_leaf, cudaStr
 int pt_bvh_build_impl(pt_scene *s, const pt_bvh_opts *o, cudaStream_t st) {
     pt_nvtx::Range nv("pt_bvh_build");
     const uint32_t n = s->num_prims;
-    const uint32_t tiles = std::max<uint32_t>(1, (n + kSortTile - 1) / kSortTile);
     const int K = (int)o->width;
     PT_CUDA_TRY(cudaEventRecord(s->ev0, st));
-    int e = s->bvh_scratch.ensure(carve_size(std::max<uint32_t>(n, 2), tiles));
+    float sah = 0.f;
+    bool clustered = false;
+    int e;
+    switch (K) {
+        case 2: e = build_tree<2>(s, o, st, &sah, &clustered); break;
+        case 4: e = build_tree<4>(s, o, st, &sah, &clustered); break;
+        default: e = build_tree<8>(s, o, st, &sah, &clustered); break;
+    }
     if (e != PT_OK) return e;
-    Scratch sc;
-    char *p = static_cast<char *>(s->bvh_scratch.ptr);
-    size_t nn = std::max<uint32_t>(n, 2);
-    sc.keys[0] = carve<uint64_t>(p, nn);
-    sc.keys[1] = carve<uint64_t>(p, nn);
-    sc.vals[0] = carve<uint32_t>(p, nn);
-    sc.vals[1] = carve<uint32_t>(p, nn);
-    sc.hist = carve<uint32_t>(p, (size_t)256 * tiles);
-    sc.plo = carve<float4>(p, nn);
-    sc.phi = carve<float4>(p, nn);
-    sc.left = carve<int>(p, nn);
-    sc.right = carve<int>(p, nn);
-    sc.parent = carve<int>(p, 2 * nn);
-    sc.rfirst = carve<int>(p, nn);
-    sc.ncount = carve<int>(p, 2 * nn);
-    sc.nleaf = carve<int>(p, 2 * nn);
-    sc.flags = carve<int>(p, nn);
-    sc.nlo = carve<float4>(p, 2 * nn);
-    sc.nhi = carve<float4>(p, 2 * nn);
-    sc.ncost = carve<float>(p, 2 * nn);
-    sc.items[0] = carve<int2>(p, nn);
-    sc.items[1] = carve<int2>(p, nn);
-    sc.counters = carve<uint32_t>(p, 16);
-    sc.sah = carve<double>(p, 8);
-    sc.cl[0] = carve<int>(p, nn);
-    sc.cl[1] = carve<int>(p, nn);
-    sc.nn = carve<int>(p, nn);
-    sc.out_id = carve<int>(p, nn);
-    sc.offs = carve<int>(p, 2 * nn);
-    sc.keep = carve<uint32_t>(p, nn + 1);
-    sc.order2 = carve<uint32_t>(p, nn);
-    sc.leaf_lo = carve<float4>(p, nn);
-    sc.leaf_hi = carve<float4>(p, nn);
-    sc.nwt = carve<float>(p, 2 * nn);
-    sc.bsum = carve<uint32_t>(p, nn / 1024 + 2);
-    sc.par2 = carve<int>(p, 2 * nn);
-    sc.dval = carve<float>(p, 8 * 2 * nn);
-    sc.dsel = carve<uint8_t>(p, 8 * 2 * nn);
-    if ((e = s->bvh_order.ensure(std::max<size_t>(4 * (size_t)n, 16))) != PT_OK) return e;
-    if ((e = s->prims_bvh.ensure(std::max<size_t>(48 * (size_t)n, 48))) != PT_OK) return e;
-
-    const int tb = 256;
-    uint32_t cb_init[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
-    PT_CUDA_TRY(cudaMemcpyAsync(sc.counters, cb_init, sizeof(cb_init), cudaMemcpyHostToDevice, st));
-    int cur = 0;  // sort buffer holding the sorted (code, primitive) pairs
-    if (n > 0) {
-        const float4 *prims = s->prims_world.as<float4>();
-        k_prim_bounds<<<blocks(n, tb), tb, 0, st>>>(prims, n, sc.plo, sc.phi, sc.counters);
-        k_morton<<<blocks(n, tb), tb, 0, st>>>(sc.plo, sc.phi, n, sc.counters, sc.keys[0], sc.vals[0]);
-        for (int pass = 0; pass < 8; pass++) {
-            int shift = pass * 8;
-            k_radix_hist<<<tiles, kSortThreads, 0, st>>>(sc.keys[cur], n, shift, sc.hist, tiles);
-            k_scan_excl<<<1, 1024, 0, st>>>(sc.hist, 256 * tiles);
-            k_radix_scatter<<<tiles, kSortThreads, 0, st>>>(sc.keys[cur], sc.vals[cur], sc.keys[cur ^ 1], sc.vals[cur ^ 1],
-                                                             n, shift, sc.hist, tiles);
-            cur ^= 1;
-        }
-        PT_CUDA_TRY(cudaGetLastError());
-        // after 8 passes the sorted pairs are back in buffer 0
-        PT_CUDA_TRY(cudaMemcpyAsync(s->bvh_order.ptr, sc.vals[cur], 4 * (size_t)n, cudaMemcpyDeviceToDevice, st));
-    }
-    // binary tree: PLOC by default, the radix tree for PT_BVH_FAST_BUILD, for
-    // a PLOC build that did not converge, or one whose wide tree is deeper
-    // than the traversal stack covers (kShortStack + kSpillStack entries)
-    const auto radix_tree = [&]() -> int {
-        if (n == 0) return PT_OK;  // no primitives: nothing to sort or link (2n - 1 would wrap)
-        PT_CUDA_TRY(cudaMemcpyAsync(s->bvh_order.ptr, sc.vals[cur], 4 * (size_t)n, cudaMemcpyDeviceToDevice, st));
-        PT_CUDA_TRY(cudaMemsetAsync(sc.parent, 0xff, 4 * (2 * (size_t)n - 1), st));
-        PT_CUDA_TRY(cudaMemsetAsync(sc.flags, 0, 4 * (size_t)n, st));
-        if (n > 1) k_karras<<<blocks(n - 1, tb), tb, 0, st>>>(sc.keys[cur], (int)n, sc.left, sc.right, sc.parent, sc.rfirst);
-        k_bottom_up<<<blocks(n, tb), tb, 0, st>>>((int)n, sc.left, sc.right, sc.parent, s->bvh_order.as<uint32_t>(),
-                                                  s->prims_world.as<float4>(), sc.plo, sc.phi, sc.nlo, sc.nhi, sc.ncount,
-                                                  sc.ncost, sc.nwt, sc.nleaf, sc.flags, (int)o->max_leaf_size);
-        PT_CUDA_TRY(cudaGetLastError());
-        return PT_OK;
-    };
-    const auto wide = [&](int root) -> int {
-        if (n > 0) {
-            k_gather_prims<<<blocks(n, tb), tb, 0, st>>>(s->prims_world.as<float4>(), s->bvh_order.as<uint32_t>(), n,
-                                                         s->prims_bvh.as<float4>());
-            PT_CUDA_TRY(cudaGetLastError());
-        }
-        switch (K) {
-            case 2: return build_wide<2>(s, sc, n, root, (int)o->max_leaf_size, st);
-            case 4: return build_wide<4>(s, sc, n, root, (int)o->max_leaf_size, st);
-            default: return build_wide<8>(s, sc, n, root, (int)o->max_leaf_size, st);
-        }
-    };
-    // curve pieces (long, thin, often diagonal) trace faster under the radix
-    // tree although PLOC gives them a lower SAH cost (50 k-strand hair at
-    // 1080p: 341 vs 320 Msamples/s), so curve-dominated scenes use it
-    const bool curve_heavy = 2ull * s->num_curve_pieces > n;
-    int root = -1;
-    if (n > 1 && !(o->flags & PT_BVH_FAST_BUILD) && !curve_heavy)
-        if ((e = ploc_build(s, sc, n, (int)o->max_leaf_size, st, &root)) != PT_OK) return e;
-    bool clustered = root >= 0;
-    if (!clustered) {
-        if ((e = radix_tree()) != PT_OK) return e;
-        root = 0;
-    }
-    if ((e = wide(root)) != PT_OK) return e;
-    const uint32_t stack_levels = (uint32_t)ptd::kTraversalStackEntries / (uint32_t)(K - 1);
-    if (clustered && s->level_start.size() - 1 > stack_levels) {
-        clustered = false;
-        if ((e = radix_tree()) != PT_OK) return e;
-        if ((e = wide(0)) != PT_OK) return e;
-    }
     if (o->width == 8) {  // the traversal reads compressed copies of the 8-wide nodes
         const uint32_t nn = s->level_start.back();
         if ((e = s->cnodes.ensure((size_t)std::max<uint32_t>(nn, 1) * 16 * ptd::kCwFloat4)) != PT_OK) return e;
@@ -1214,9 +1415,6 @@ int pt_bvh_build_impl(pt_scene *s, const pt_bvh_opts *o, cudaStream_t st) {
     float ms = 0.f;
     PT_CUDA_TRY(cudaEventElapsedTime(&ms, s->ev0, s->ev1));
     s->bvh_opts = *o;
-    float sah = 0.f;
-    if ((e = s->sah_scratch.ensure(64)) != PT_OK) return e;
-    if ((e = compute_sah(s, s->sah_scratch.as<double>(), st, sah)) != PT_OK) return e;
 
     pt_bvh_stats &bs = s->bvh_stats;
     bs.width = o->width;
@@ -1254,7 +1452,7 @@ int pt_bvh_refit_impl(pt_scene *s, cudaStream_t st) {
     const uint32_t n = s->num_prims;
     PT_CUDA_TRY(cudaEventRecord(s->ev0, st));
     if (n > 0)
-        k_gather_prims<<<blocks(n, 256), 256, 0, st>>>(s->prims_world.as<float4>(), s->bvh_order.as<uint32_t>(), n,
+        k_gather_prims<<<blocks(3 * (size_t)n, 256), 256, 0, st>>>(s->prims_world.as<float4>(), s->bvh_order.as<uint32_t>(), n,
                                                         s->prims_bvh.as<float4>());
     switch (s->bvh_opts.width) {
         case 2: refit_levels<2>(s, st); break;
