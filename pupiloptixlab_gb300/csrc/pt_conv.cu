@@ -56,11 +56,6 @@ constexpr uint64_t kWaitNs = 2000000000ull;
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
-__device__ __forceinline__ uint64_t gtimer() {
-    uint64_t t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
@@ -85,18 +80,22 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 // Bounded wait for the phase with the given parity to complete: false after
-// limit_ns of %globaltimer, or as soon as *abort is set (another warp of the
-// CTA gave up), so that a failing CTA leaves within one limit.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, bool backoff = false,
-                                          uint64_t limit_ns = kWaitNs, const volatile int *abort = nullptr) {
+// limit_ns (in SM cycles at two per nanosecond, so at least that long), or as
+// soon as *abort is set (another warp of the CTA gave up), so that a failing CTA
+// leaves within one limit.  try_wait itself suspends the thread until the phase
+// completes or a short hardware limit passes.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint64_t limit_ns = kWaitNs,
+                                          const volatile int *abort = nullptr) {
     if (mbar_try(bar, parity)) return true;
-    const uint64_t t0 = gtimer();
-    while (!mbar_try(bar, parity)) {
-        if (backoff) __nanosleep(128);
-        if (gtimer() - t0 > limit_ns) return false;
+    const long long t0 = clock64();
+    const long long limit = static_cast<long long>(limit_ns * 2);
+    for (;;) {
+#pragma unroll 1
+        for (int i = 0; i < 8; i++)
+            if (mbar_try(bar, parity)) return true;
+        if (clock64() - t0 > limit) return false;
         if (abort && *abort) return false;
     }
-    return true;
 }
 __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0, int c1, int c2,
                                             int c3) {
@@ -122,29 +121,49 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+// Issued by a whole warp, in the lane with `elected` set: the operands then stay
+// in uniform registers.  One lane of a diverged warp, forming its descriptors
+// per MMA, took 95 cycles for an MMA of 128 x 32 x 16 that runs in 40.
 __device__ __forceinline__ void umma_bf16(uint32_t dtmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                          uint32_t accumulate) {
+                                          uint32_t accumulate, uint32_t elected) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p, q;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(dtmem),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(dtmem),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(elected)
         : "memory");
 }
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+__device__ __forceinline__ void umma_commit(uint32_t bar, uint32_t elected) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar),
+        "r"(elected)
+        : "memory");
+}
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+    return e;
 }
 // 32 lanes x 16 consecutive 32-bit columns: thread t of the warp gets lane
-// (warp base + t), columns col..col+15.
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
-    uint32_t r[16];
+// (warp base + t), columns col..col+15.  tmem_ld16 starts the load, tmem_wait
+// makes v valid; loads put between the two overlap it.
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
         "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
           "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_wait(uint32_t (&r)[16], float (&v)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+                 :
+                 : "memory");
 #pragma unroll
     for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
@@ -189,81 +208,103 @@ __device__ __forceinline__ void st_global_v8(uint16_t *p, uint4 a, uint4 b) {
                  : "memory");
 }
 
-// Forward epilogue: accumulator row `tid` = pixel (x0 + tid % tile_w,
-// y0 + tid / tile_w); warp w reads TMEM lanes 32w..32w+31, 16 columns at a time.
-__device__ __forceinline__ void fwd_epilogue(const FwdArgs &a, uint32_t tmem, int tid, int warp, int img, int x0, int y0,
-                                             int n0, bool ok) {
-    const int px = tid % a.tile_w, py = tid / a.tile_w;
-    const int x = x0 + px, y = y0 + py;
-    const bool valid = ok && py < a.tile_rows && x < a.W && y < a.H;
-    const size_t pix = ((size_t)img * a.H + (valid ? y : 0)) * a.W + (valid ? x : 0);
-    const uint32_t trow = tmem + (static_cast<uint32_t>(warp * 32) << 16);
-    for (int c = 0; c < a.n_tile; c += 16) {
-        float v[16];
-        tmem_ld16(trow + c, v);
-        const int ch0 = n0 + c;
-        if (!valid || ch0 >= a.cout) continue;
-        const int nvalid = min(16, a.cout - ch0);
-        if (a.epi == EPI_F32) {
-            float *o = static_cast<float *>(a.out) + pix * a.out_ctot + a.out_coff + ch0;
-            for (int i = 0; i < nvalid; i++) o[i] = v[i] + (a.bias ? a.bias[ch0 + i] : 0.f);
-            continue;
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t *>(&h);
+}
+// 16 biases from channel ch0 on (of which nvalid exist), or zeros.
+__device__ __forceinline__ void load_bias(const FwdArgs &a, int ch0, int nvalid, float (&b)[16]) {
+    if (a.bias && nvalid == 16 && a.bias16) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const float4 q = __ldg(reinterpret_cast<const float4 *>(a.bias + ch0) + i);
+            b[4 * i] = q.x;
+            b[4 * i + 1] = q.y;
+            b[4 * i + 2] = q.z;
+            b[4 * i + 3] = q.w;
         }
-        if (a.epi == EPI_BF16) {
-            float b[16];
-            if (a.bias && nvalid == 16 && a.bias16) {  // 16 biases in four 16-byte loads
+    } else {
 #pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const float4 q = __ldg(reinterpret_cast<const float4 *>(a.bias + ch0) + i);
-                    b[4 * i] = q.x;
-                    b[4 * i + 1] = q.y;
-                    b[4 * i + 2] = q.z;
-                    b[4 * i + 3] = q.w;
-                }
-            } else {
-#pragma unroll
-                for (int i = 0; i < 16; i++) b[i] = (a.bias && i < nvalid) ? a.bias[ch0 + i] : 0.f;
-            }
-#pragma unroll
-            for (int i = 0; i < 16; i++) {
-                const float f = v[i] + b[i];
-                v[i] = a.relu ? fmaxf(f, 0.f) : f;
-            }
-        } else {
+        for (int i = 0; i < 16; i++) b[i] = (a.bias && i < nvalid) ? __ldg(a.bias + ch0 + i) : 0.f;
+    }
+}
+
+// Forward epilogue of the columns c0, c0 + cstep, ... (16 channels each):
+// accumulator row `tid` = pixel (x0 + tid % tile_w, y0 + tid / tile_w); warp
+// quadrant w reads TMEM lanes 32w..32w+31.  Bias and mask are loaded while the
+// accumulator is.
+__device__ __forceinline__ void fwd_epilogue(const FwdArgs &a, uint32_t tmem, int tid, int quad, int img, int x0, int y0,
+                                             int n0, int c0, int cstep) {
+    int px = tid, py = 0;
+    if (a.tile_w != 128) {
+        py = tid / a.tile_w;
+        px = tid - py * a.tile_w;
+    }
+    const int x = x0 + px, y = y0 + py;
+    const bool valid = py < a.tile_rows && x < a.W && y < a.H;
+    const size_t pix = ((size_t)img * a.H + (valid ? y : 0)) * a.W + (valid ? x : 0);
+    const uint32_t trow = tmem + (static_cast<uint32_t>(quad * 32) << 16);
+    for (int c = c0; c < a.n_tile; c += cstep) {
+        uint32_t raw[16];
+        tmem_ld16(trow + c, raw);
+        const int ch0 = n0 + c;
+        const int nvalid = min(16, a.cout - ch0);
+        float v[16];
+        if (a.epi == EPI_BF16_MASK) {
+            uint4 q0 = make_uint4(0, 0, 0, 0), q1 = q0;
             const uint16_t *m = a.mask + pix * a.mask_ctot + a.mask_coff + ch0;
-            if (nvalid == 16) {
-                uint4 q0, q1;
+            if (valid && nvalid == 16) {
                 if (a.wide_io) {
                     ld_global_v8(m, q0, q1);
                 } else {
                     q0 = *reinterpret_cast<const uint4 *>(m);
                     q1 = *reinterpret_cast<const uint4 *>(m + 8);
                 }
-                const uint16_t *h0 = reinterpret_cast<const uint16_t *>(&q0), *h1 = reinterpret_cast<const uint16_t *>(&q1);
+            } else if (valid) {
+                uint16_t *h0 = reinterpret_cast<uint16_t *>(&q0), *h1 = reinterpret_cast<uint16_t *>(&q1);
 #pragma unroll
                 for (int i = 0; i < 8; i++) {
-                    if (!(h0[i] != 0 && (h0[i] & 0x8000u) == 0)) v[i] = 0.f;
-                    if (!(h1[i] != 0 && (h1[i] & 0x8000u) == 0)) v[i + 8] = 0.f;
+                    if (i < nvalid) h0[i] = m[i];
+                    if (i + 8 < nvalid) h1[i] = m[i + 8];
                 }
-            } else {
-                for (int i = 0; i < nvalid; i++)
-                    if (!(m[i] != 0 && (m[i] & 0x8000u) == 0)) v[i] = 0.f;
             }
+            tmem_wait(raw, v);
+            const uint16_t *h0 = reinterpret_cast<const uint16_t *>(&q0), *h1 = reinterpret_cast<const uint16_t *>(&q1);
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                if (!(h0[i] != 0 && (h0[i] & 0x8000u) == 0)) v[i] = 0.f;
+                if (!(h1[i] != 0 && (h1[i] & 0x8000u) == 0)) v[i + 8] = 0.f;
+            }
+        } else {
+            float b[16];
+            load_bias(a, ch0, nvalid, b);
+            tmem_wait(raw, v);
+#pragma unroll
+            for (int i = 0; i < 16; i++) v[i] += b[i];
         }
-        uint16_t *o = static_cast<uint16_t *>(a.out) + pix * a.out_ctot + a.out_coff + ch0;
+        if (!valid || nvalid <= 0) continue;
+        if (a.epi == EPI_F32) {
+            float *o = static_cast<float *>(a.out) + pix * a.out_ctot + a.out_coff + ch0;
+#pragma unroll
+            for (int i = 0; i < 16; i++)
+                if (i < nvalid) o[i] = v[i];
+            continue;
+        }
+        if (a.epi == EPI_BF16 && a.relu) {
+#pragma unroll
+            for (int i = 0; i < 16; i++) v[i] = fmaxf(v[i], 0.f);
+        }
+        uint32_t w[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) w[i] = pack_bf16(v[2 * i], v[2 * i + 1]);
+        const uint4 q0 = make_uint4(w[0], w[1], w[2], w[3]), q1 = make_uint4(w[4], w[5], w[6], w[7]);
+        uint16_t *o = a.out ? static_cast<uint16_t *>(a.out) + pix * a.out_ctot + a.out_coff + ch0 : nullptr;
         // the four up-sampled copies (pixel (2y + i, 2x + j) of the 2H x 2W tensor)
         uint16_t *u = a.up ? a.up + (((size_t)img * 2 * a.H + 2 * y) * 2 * a.W + 2 * x) * a.up_ctot + ch0 : nullptr;
         const size_t urow = static_cast<size_t>(2 * a.W) * a.up_ctot;
         if (nvalid == 16) {
-            uint4 q0, q1;
-            uint32_t *w0 = reinterpret_cast<uint32_t *>(&q0), *w1 = reinterpret_cast<uint32_t *>(&q1);
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                w0[i] = f2bf(v[2 * i]) | (static_cast<uint32_t>(f2bf(v[2 * i + 1])) << 16);
-                w1[i] = f2bf(v[8 + 2 * i]) | (static_cast<uint32_t>(f2bf(v[8 + 2 * i + 1])) << 16);
-            }
             if (a.wide_io) {
-                st_global_v8(o, q0, q1);
+                if (o) st_global_v8(o, q0, q1);
                 if (u) {
                     st_global_v8(u, q0, q1);
                     st_global_v8(u + a.up_ctot, q0, q1);
@@ -271,8 +312,10 @@ __device__ __forceinline__ void fwd_epilogue(const FwdArgs &a, uint32_t tmem, in
                     st_global_v8(u + urow + a.up_ctot, q0, q1);
                 }
             } else {
-                reinterpret_cast<uint4 *>(o)[0] = q0;
-                reinterpret_cast<uint4 *>(o)[1] = q1;
+                if (o) {
+                    reinterpret_cast<uint4 *>(o)[0] = q0;
+                    reinterpret_cast<uint4 *>(o)[1] = q1;
+                }
                 for (int k = 0; u && k < 4; k++) {
                     uint16_t *uk = u + (k >> 1) * urow + (k & 1) * a.up_ctot;
                     reinterpret_cast<uint4 *>(uk)[0] = q0;
@@ -280,49 +323,41 @@ __device__ __forceinline__ void fwd_epilogue(const FwdArgs &a, uint32_t tmem, in
                 }
             }
         } else {
-            for (int i = 0; i < nvalid; i++) {
-                const uint16_t b = f2bf(v[i]);
-                o[i] = b;
-                for (int k = 0; u && k < 4; k++) u[(k >> 1) * urow + (k & 1) * a.up_ctot + i] = b;
+#pragma unroll
+            for (int i = 0; i < 16; i++) {
+                if (i >= nvalid) continue;
+                const uint16_t h = static_cast<uint16_t>(w[i >> 1] >> (16 * (i & 1)));
+                if (o) o[i] = h;
+                for (int k = 0; u && k < 4; k++) u[(k >> 1) * urow + (k & 1) * a.up_ctot + i] = h;
             }
         }
     }
-
 }
 
-// Two-row halo tile with the pooled output (EPI_BF16, cout a multiple of 16,
-// 32-byte aligned rows): thread `tid` holds pixel x = x0 + tid of rows y0 and
-// y0 + 1 (accumulators tmem and tmem + n_tile), its neighbour lane x ^ 1.
+// Rows y0 and y0 + 1 of a halo tile with the pooled output (EPI_BF16, cout a
+// multiple of 16, 32-byte aligned rows): thread `tid` holds pixel x = x0 + tid of
+// both rows (accumulators tmem and tmem + n_tile), its neighbour lane x ^ 1.
 // Each row is written as fwd_epilogue writes it; the even lane of each pair
 // writes the average of the four BF16 outputs, summed in the order
 // (y0, x), (y0, x + 1), (y0 + 1, x), (y0 + 1, x + 1).
-__device__ __forceinline__ void fwd_epilogue_pool2(const FwdArgs &a, uint32_t tmem, int tid, int warp, int img, int x0,
-                                                   int y0, int n0) {
+__device__ __forceinline__ void fwd_epilogue_pool2(const FwdArgs &a, uint32_t tmem, int tid, int quad, int img, int x0,
+                                                   int y0, int n0, int c0, int cstep) {
     const int x = x0 + tid;
     const bool valid = x < a.W && y0 < a.H;
     const size_t pix0 = ((size_t)img * a.H + (valid ? y0 : 0)) * a.W + (valid ? x : 0);
     const size_t ppix = ((size_t)img * (a.H / 2) + (valid ? y0 / 2 : 0)) * (a.W / 2) + (valid ? x / 2 : 0);
-    const uint32_t trow = tmem + (static_cast<uint32_t>(warp * 32) << 16);
-    for (int c = 0; c < a.n_tile; c += 16) {
-        float v[2][16];
-        tmem_ld16(trow + c, v[0]);
-        tmem_ld16(trow + a.n_tile + c, v[1]);
+    const uint32_t trow = tmem + (static_cast<uint32_t>(quad * 32) << 16);
+    for (int c = c0; c < a.n_tile; c += cstep) {
+        uint32_t raw0[16], raw1[16];
+        tmem_ld16(trow + c, raw0);
+        tmem_ld16(trow + a.n_tile + c, raw1);
         const int ch0 = n0 + c;
-        if (ch0 >= a.cout) continue;  // uniform across the warp
         float b[16];
-        if (a.bias && a.bias16) {
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const float4 q = __ldg(reinterpret_cast<const float4 *>(a.bias + ch0) + i);
-                b[4 * i] = q.x;
-                b[4 * i + 1] = q.y;
-                b[4 * i + 2] = q.z;
-                b[4 * i + 3] = q.w;
-            }
-        } else {
-#pragma unroll
-            for (int i = 0; i < 16; i++) b[i] = a.bias ? a.bias[ch0 + i] : 0.f;
-        }
+        load_bias(a, ch0, min(16, a.cout - ch0), b);
+        float v[2][16];
+        tmem_wait(raw0, v[0]);
+        tmem_wait(raw1, v[1]);
+        if (ch0 >= a.cout) continue;  // uniform across the warp
         uint32_t w[2][8];
 #pragma unroll
         for (int r = 0; r < 2; r++)
@@ -333,21 +368,22 @@ __device__ __forceinline__ void fwd_epilogue_pool2(const FwdArgs &a, uint32_t tm
                     f0 = fmaxf(f0, 0.f);
                     f1 = fmaxf(f1, 0.f);
                 }
-                w[r][i] = f2bf(f0) | (static_cast<uint32_t>(f2bf(f1)) << 16);
+                w[r][i] = pack_bf16(f0, f1);
             }
         uint32_t pw[8];
 #pragma unroll
         for (int i = 0; i < 8; i++) {
+            const uint32_t n0w = __shfl_xor_sync(0xffffffffu, w[0][i], 1), n1w = __shfl_xor_sync(0xffffffffu, w[1][i], 1);
             float acc[2];
 #pragma unroll
             for (int h = 0; h < 2; h++) {
                 const float own0 = __uint_as_float((w[0][i] >> (16 * h)) << 16);
                 const float own1 = __uint_as_float((w[1][i] >> (16 * h)) << 16);
-                const float nb0 = __shfl_xor_sync(0xffffffffu, own0, 1);
-                const float nb1 = __shfl_xor_sync(0xffffffffu, own1, 1);
+                const float nb0 = __uint_as_float((n0w >> (16 * h)) << 16);
+                const float nb1 = __uint_as_float((n1w >> (16 * h)) << 16);
                 acc[h] = 0.25f * ((((0.f + own0) + nb0) + own1) + nb1);  // k_pool's order, from 0
             }
-            pw[i] = f2bf(acc[0]) | (static_cast<uint32_t>(f2bf(acc[1])) << 16);
+            pw[i] = pack_bf16(acc[0], acc[1]);
         }
         if (!valid) continue;
 #pragma unroll
@@ -365,30 +401,28 @@ __device__ __forceinline__ void fwd_epilogue_pool2(const FwdArgs &a, uint32_t tm
 // ---------------------------------------------------------------------------
 // halo operand layout (forward / data gradient, images at least 128 pixels wide)
 // ---------------------------------------------------------------------------
-// The pixel tile is a 128-pixel row segment.  Per 16-channel chunk one TMA box
-// brings its 3 x 130-pixel neighbourhood (the segment and a one-pixel border,
-// zero outside the image) as 32-byte pixel rows in the 32-byte-swizzled
-// K-major layout, pixels in row-major order.  The A operand of tap (dy, dx) is
-// the same box read from pixel row dy * 130 + dx on (stride byte offset =
-// 256 B between 8-row groups): the tensor cores apply the swizzle to the
-// absolute shared-memory address, as the TMA wrote it, so a start at any
-// 32-byte row reads the right data.  The input is thus read from L2 once per
-// chunk instead of once per tap.  (PT_CONV_HALO_PLANES=1 selects the earlier
-// layout: two TMA boxes per chunk into non-swizzled planes of 8 channels,
-// 16 bytes per pixel, leading byte offset = plane size.)  B holds the chunk's weights for all nine
-// taps (32-byte swizzle, one TMA box per tap).  When one channel tile covers
-// every output channel and all (chunk, tap) weight boxes fit in
-// kMaxResidentWeights bytes, they are loaded once per CTA ahead of the ring
-// (on their own barrier) and the stages carry only the A box.
-// A tile may cover two output rows (halo_rows = 2: a 4-row box, two M = 128
-// accumulators sharing each B operand), so that every input row crosses L2
-// twice per pass instead of three times; the second row's A operand is the
-// same box read one box row (130 pixels) further on.
+// The pixel tile is a 128-pixel row segment of R output rows.  Per 16-channel
+// chunk one TMA box brings its (R + 2) x 130-pixel neighbourhood (the segment
+// and a one-pixel border, zero outside the image) as 32-byte pixel rows in the
+// 32-byte-swizzled K-major layout, pixels in row-major order.  The A operand of
+// input row i shifted by dx is the same box read from pixel row i * 130 + dx on
+// (stride byte offset = 256 B between 8-row groups): the tensor cores apply the
+// swizzle to the absolute shared-memory address, as the TMA wrote it, so a start
+// at any 32-byte row reads the right data.
+// Input row i adds to the output rows i - 2 .. i (taps dy = 2, 1, 0), whose
+// accumulators are neighbours in tensor memory: one MMA of N = (up to three) x
+// n_tile covers them, its B operand the chunk's weights for dx with dy falling.
+// An MMA of 128 x N x 16 takes 32 + N / 4 cycles for N < 128 (measured; the A
+// operand's 4 KiB is read either way), so three row taps cost 57 cycles instead
+// of three times 40 at N = 32.  Each output row still gets its taps in the order
+// dy, dx and is the same sum for every R.
+// B holds the chunk's weights for all nine taps ([dx][2 - dy] blocks of n_tile
+// rows, 32-byte swizzle, one TMA box per tap).  When one channel tile covers
+// every output channel and all weights fit beside the ring, they are loaded once
+// per CTA (on their own barrier) and the stages carry only the A box.
 constexpr int kHaloW = 130;
-__host__ __device__ constexpr int halo_box_bytes(int rows) { return kHaloW * (rows + 2) * 16; }
-__host__ __device__ constexpr int halo_plane_bytes(int rows) { return (halo_box_bytes(rows) + 1023) / 1024 * 1024; }
-__host__ __device__ constexpr int halo_b_tap_bytes(int n_tile) { return (n_tile * 32 + 1023) / 1024 * 1024; }
-constexpr int kMaxResidentWeights = 64 * 1024;
+__host__ __device__ constexpr int halo_box_bytes(int rows) { return kHaloW * (rows + 2) * 32; }
+__host__ __device__ constexpr int halo_b_bytes(int n_tile) { return (9 * n_tile * 32 + 1023) / 1024 * 1024; }
 
 // ---------------------------------------------------------------------------
 // persistent forward / data-gradient kernel
@@ -396,16 +430,23 @@ constexpr int kMaxResidentWeights = 64 * 1024;
 // One CTA per SM slot walks the output tiles (pixel tile x output-channel
 // tile) with a stride of gridDim.x.  Warp 0 streams operands into a ring of
 // `stages` buffers across tile boundaries, warp 1 issues the MMAs into one of
-// two accumulators in tensor memory (2 x n_tile columns), and warps 2-5 run
-// the epilogue of tile i from one accumulator while the MMAs of tile i + 1
-// fill the other.  Warp w of the epilogue reads TMEM lanes 32 * (w % 4) + 0..31.
-// HALO: the A operand comes from one 3 x 130-pixel halo box per 16-channel
-// chunk (width >= 128, see above); otherwise one box per (tap, chunk).
-template <int KC, bool HALO>
-__global__ void __launch_bounds__(192, 1)
+// two accumulators in tensor memory (2 x rows x n_tile columns), and warps 2-9
+// run the epilogue of tile i from one accumulator while the MMAs of tile i + 1
+// fill the other.  Epilogue warp w reads TMEM lanes 32 * (w % 4) + 0..31; the
+// two warps of a quadrant share a tile's rows or column groups.
+// R > 0: the A operand comes from one (R + 2) x 130-pixel halo box per
+// 16-channel chunk (width >= 128, see above); R = 0: one box per (tap, chunk).
+// At 1920 x 1088 the layers were bound by the MMA issue (80 -> 32 channels 263
+// us, of which 242 without loads and epilogue) and by the epilogue (16 -> 32: 84
+// of 119 us).
+constexpr int kFwdThreads = 320;
+template <int KC, int R>
+__global__ void __launch_bounds__(kFwdThreads, 2)
     k_conv_fwd_persistent(const __grid_constant__ CUtensorMap act, const __grid_constant__ CUtensorMap wgt,
-                          const FwdArgs a) {
-    constexpr int R = KC * 2;
+                          const __grid_constant__ FwdArgs a) {
+    constexpr bool HALO = R > 0;
+    constexpr int ROWB = KC * 2;
+    constexpr int kRows = HALO ? R : 1;  // output rows (accumulators) per tile
     constexpr uint32_t SWZ = swz_mode<KC>();
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t bars[2 * kMaxStages + 7];
@@ -421,11 +462,11 @@ __global__ void __launch_bounds__(192, 1)
     const int n_n = a.n_tiles_n;
     const int total = a.n_img * tiles_img * n_n;
     const int nk = HALO ? a.nchunks : 9 * a.nchunks;  // stages per tile
-    const int a_bytes = HALO ? a.halo_a_bytes : 128 * R;
-    const int b_tap = HALO ? halo_b_tap_bytes(a.n_tile) : 0;
-    const int hrows = HALO ? a.halo_rows : 1;  // output rows (accumulators) per tile
-    const uint32_t tx_bytes = HALO ? static_cast<uint32_t>(a.halo_a_tx + (wres ? 0 : 9 * a.n_tile * R))
-                                   : static_cast<uint32_t>(a.tile_w * a.tile_rows * R + a.n_tile * R);
+    const int a_bytes = HALO ? a.halo_a_bytes : 128 * ROWB;
+    const uint32_t chunk_b = HALO ? static_cast<uint32_t>(halo_b_bytes(a.n_tile)) : 0u;
+    const uint32_t tap_b = static_cast<uint32_t>(a.n_tile) * 32u;  // one tap's weights of a chunk (halo)
+    const uint32_t tx_bytes = HALO ? static_cast<uint32_t>(halo_box_bytes(R) + (wres ? 0 : 9 * a.n_tile * ROWB))
+                                   : static_cast<uint32_t>(a.tile_w * a.tile_rows * ROWB + a.n_tile * ROWB);
     const uint32_t bar0 = smem_u32(bars);
     auto full = [&](int s) { return bar0 + 8u * s; };
     auto empty = [&](int s) { return bar0 + 8u * (kMaxStages + s); };
@@ -440,8 +481,9 @@ __global__ void __launch_bounds__(192, 1)
         n0 = (t - pt * n_n) * a.n_tile;
         img = pt / tiles_img;
         const int r = pt - img * tiles_img;
-        x0 = (r % a.tiles_x) * a.tile_w;
-        y0 = (r / a.tiles_x) * a.tile_rows;
+        const int ty = r / a.tiles_x;
+        x0 = (r - ty * a.tiles_x) * a.tile_w;
+        y0 = ty * a.tile_rows;
     };
 
     if (warp == 0) tmem_alloc(smem_u32(&tmem_slot), a.tmem_cols);
@@ -452,7 +494,7 @@ __global__ void __launch_bounds__(192, 1)
         }
         for (int b = 0; b < 2; b++) {
             mbar_init(acc_full(b), 1);
-            mbar_init(acc_empty(b), 128);
+            mbar_init(acc_empty(b), 256);
         }
         mbar_init(wbar, 1);
         mbar_init(sbar, 1);
@@ -468,20 +510,25 @@ __global__ void __launch_bounds__(192, 1)
 
     if (warp == 0) {
         if (lane == 0) {  // producer
-            if (wres) {  // every (chunk, tap) weight box once: b_tap apart, chunk-major
-                mbar_expect_tx(wbar, static_cast<uint32_t>(a.nchunks * 9 * a.n_tile * R));
-                for (int k = 0; k < a.nchunks; k++)
-                    for (int tap = 0; tap < 9; tap++)
-                        tma_load_2d(wbase + static_cast<uint32_t>((k * 9 + tap) * b_tap), &wgt, wbar,
-                                    tap * a.cin + k * 16, 0);
+            // the nine weight boxes of a chunk: [dx][2 - dy] blocks (tap = 3 dy + dx)
+            const auto load_weights = [&](uint32_t dst, uint32_t bar, int k, int n0) {
+                for (int tap = 0; tap < 9; tap++) {
+                    const int dy = tap / 3, dx = tap - 3 * dy;
+                    tma_load_2d(dst + static_cast<uint32_t>(dx * 3 + 2 - dy) * tap_b, &wgt, bar, tap * a.cin + k * 16, n0);
+                }
+            };
+            if (wres) {
+                mbar_expect_tx(wbar, static_cast<uint32_t>(a.nchunks * 9 * a.n_tile * ROWB));
+                for (int k = 0; k < a.nchunks; k++) load_weights(wbase + static_cast<uint32_t>(k) * chunk_b, wbar, k, 0);
             }
             int kg = 0;  // stages issued so far (ring position and phase)
+            int s = 0;
+            uint32_t phase = 0;
             for (int t = blockIdx.x; t < total && !*fail; t += gridDim.x) {
                 int img, x0, y0, n0;
                 tile_of(t, img, x0, y0, n0);
                 for (int k = 0; k < nk; k++, kg++) {
-                    const int s = kg % S;
-                    if (kg >= S && !mbar_wait(empty(s), ((kg / S) - 1) & 1, false, lim, fail)) {
+                    if (kg >= S && !mbar_wait(empty(s), phase ^ 1u, lim, fail)) {
                         record_error(a.err, 1u);
                         *fail = 1;
                         break;
@@ -494,20 +541,17 @@ __global__ void __launch_bounds__(192, 1)
                     }
                     mbar_expect_tx(full(s), tx_bytes);
                     if (HALO) {
-                        if (a.halo_sw32) {
-                            tma_load_4d(sa, &act, full(s), k * 16, x0 - 1, y0 - 1, img);
-                        } else {
-                            tma_load_4d(sa, &act, full(s), k * 16, x0 - 1, y0 - 1, img);
-                            tma_load_4d(sa + a.halo_plane_bytes, &act, full(s), k * 16 + 8, x0 - 1, y0 - 1, img);
-                        }
-                        if (!wres)
-                            for (int tap = 0; tap < 9; tap++)
-                                tma_load_2d(sb + tap * b_tap, &wgt, full(s), tap * a.cin + k * 16, n0);
+                        tma_load_4d(sa, &act, full(s), k * 16, x0 - 1, y0 - 1, img);
+                        if (!wres) load_weights(sb, full(s), k, n0);
                     } else {
                         const int tap = k / a.nchunks, ch = k - tap * a.nchunks;
                         const int dy = tap / 3, dx = tap - dy * 3;
                         tma_load_4d(sa, &act, full(s), ch * KC, x0 + dx - 1, y0 + dy - 1, img);
                         tma_load_2d(sb, &wgt, full(s), tap * a.cin + ch * KC, n0);
+                    }
+                    if (++s == S) {
+                        s = 0;
+                        phase ^= 1u;
                     }
                 }
             }
@@ -515,95 +559,103 @@ __global__ void __launch_bounds__(192, 1)
             // leaves (the last issue on each ring slot, and the resident
             // weights), also when another warp gave up; within the normal limit
             for (int k = kg - S; k < kg; k++)
-                if (k >= 0) (void)mbar_wait(full(k % S), (k / S) & 1, true);
-            if (wres) (void)mbar_wait(wbar, 0, true);
+                if (k >= 0) (void)mbar_wait(full(k % S), (k / S) & 1);
+            if (wres) (void)mbar_wait(wbar, 0);
         }
-    } else if (warp == 1) {
-        if (lane == 0) {  // MMA issuer
-            const uint32_t idesc = idesc_bf16(128, a.n_tile, false, false);
-            if (a.stall && !mbar_wait(sbar, 0, true, lim)) {  // the stall test: this wait always runs out
+    } else if (warp == 1) {  // MMA issuer: the whole warp, so that descriptors stay uniform
+        const uint32_t elected = elect_one();
+        const auto wait = [&](uint32_t bar, uint32_t parity) {  // every lane, one answer
+            if (__all_sync(0xffffffffu, mbar_wait(bar, parity, lim, fail))) return true;
+            if (lane == 0) {
                 record_error(a.err, 2u);
                 *fail = 1;
             }
-            if (wres && !*fail && !mbar_wait(wbar, 0, false, lim, fail)) {
-                record_error(a.err, 2u);
-                *fail = 1;
-            }
-            int kg = 0, j = 0;
-            for (int t = blockIdx.x; t < total && !*fail; t += gridDim.x, j++) {
-                const int buf = j & 1;
-                if (!mbar_wait(acc_empty(buf), ((j >> 1) & 1) ^ 1, false, lim, fail)) {  // epilogue of tile j - 2 done
-                    record_error(a.err, 2u);
-                    *fail = 1;
-                    break;
-                }
+            return false;
+        };
+        const uint32_t idesc0 = idesc_bf16(128, 0, false, false);
+        const uint32_t n_desc = static_cast<uint32_t>(a.n_tile >> 3) << 17;  // N = n_tile
+        bool ok = true;
+        if (a.stall) ok = wait(sbar, 0);  // the stall test: this wait always runs out
+        if (ok && wres) ok = wait(wbar, 0);
+        int kg = 0, j = 0, s = 0;
+        uint32_t phase = 0;
+        for (int t = blockIdx.x; t < total && ok; t += gridDim.x, j++) {
+            const int buf = j & 1;
+            if (!(ok = wait(acc_empty(buf), ((j >> 1) & 1) ^ 1))) break;  // epilogue of tile j - 2 done
+            tc_fence_after();
+            const uint32_t d = tmem + static_cast<uint32_t>(buf * kRows * a.n_tile);
+            for (int k = 0; k < nk; k++, kg++) {
+                if (!(ok = wait(full(s), phase))) break;
                 tc_fence_after();
-                const uint32_t d = tmem + static_cast<uint32_t>(buf * hrows * a.n_tile);
-                for (int k = 0; k < nk; k++, kg++) {
-                    const int s = kg % S;
-                    if (!mbar_wait(full(s), (kg / S) & 1, false, lim, fail)) {
-                        record_error(a.err, 2u);
-                        *fail = 1;
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint32_t sa = base + s * a.stage_bytes;
-                    const uint32_t sb = wres ? wbase + static_cast<uint32_t>(k * 9 * b_tap) : sa + a_bytes;
-                    if (HALO) {
+                const uint32_t sa = base + s * a.stage_bytes;
+                const uint32_t sb = wres ? wbase + static_cast<uint32_t>(k) * chunk_b : sa + a_bytes;
+                if constexpr (HALO) {
+                    const uint64_t da0 = sdesc(sa, 16u, 256u, SWZ), db0 = sdesc(sb, 16u, 256u, SWZ);
+                    const uint64_t tap_d = tap_b >> 4;
+                    // rows r0..r1 of the tile from input row i shifted by dx
+                    const auto mma = [&](int i, int dx, int r0, int r1, uint32_t accumulate) {
+                        umma_bf16(d + static_cast<uint32_t>(r0 * a.n_tile), da0 + 2u * (i * kHaloW + dx),
+                                  db0 + tap_d * (dx * 3 + 2 - (i - r0)), idesc0 + n_desc * (r1 - r0 + 1), accumulate,
+                                  elected);
+                    };
 #pragma unroll
-                        for (int tap = 0; tap < 9; tap++) {
-                            const int dy = tap / 3, dx = tap - 3 * (tap / 3);
-                            const uint64_t db = sdesc(sb + tap * b_tap, 16u, 8u * R, SWZ);
-                            for (int r = 0; r < hrows; r++) {
-                                uint64_t da;
-                                if (a.halo_sw32) {  // 32-byte rows, 32-byte swizzle, 8-row groups 256 B apart
-                                    da = sdesc(sa + 32u * ((dy + r) * kHaloW + dx), 16u, 256u, 6u);
-                                } else {
-                                    da = sdesc(sa + 16u * ((dy + r) * kHaloW + dx),
-                                               static_cast<uint32_t>(a.halo_plane_bytes), 128u, 0u);
-                                }
-                                umma_bf16(d + static_cast<uint32_t>(r * a.n_tile), da, db, idesc,
-                                          (k | tap) != 0 ? 1u : 0u);
+                    for (int i = 0; i < R + 2; i++) {
+                        const int r0 = i >= 2 ? i - 2 : 0, r1 = i < R ? i : R - 1;
+#pragma unroll
+                        for (int dx = 0; dx < 3; dx++) {
+                            if (dx == 0 && i < R && k == 0) {  // row i of the tile starts here
+                                if (r0 < i) mma(i, dx, r0, i - 1, 1u);
+                                mma(i, dx, i, i, 0u);
+                            } else {
+                                mma(i, dx, r0, r1, 1u);
                             }
                         }
-                    } else {
-#pragma unroll
-                        for (int q = 0; q < KC / 16; q++) {
-                            const uint64_t da = sdesc(sa + 32u * q, 16u, 8u * R, SWZ);
-                            const uint64_t db = sdesc(sb + 32u * q, 16u, 8u * R, SWZ);
-                            umma_bf16(d, da, db, idesc, (k | q) != 0 ? 1u : 0u);
-                        }
                     }
-                    umma_commit(empty(s));
+                } else {
+                    const uint64_t da0 = sdesc(sa, 16u, 8u * ROWB, SWZ), db0 = sdesc(sb, 16u, 8u * ROWB, SWZ);
+#pragma unroll
+                    for (int q = 0; q < KC / 16; q++)
+                        umma_bf16(d, da0 + 2u * q, db0 + 2u * q, idesc0 + n_desc, (k | q) != 0 ? 1u : 0u, elected);
                 }
-                if (*fail) break;
-                umma_commit(acc_full(buf));
+                umma_commit(empty(s), elected);
+                if (++s == S) {
+                    s = 0;
+                    phase ^= 1u;
+                }
             }
-            if (*fail && kg > 0) {  // let the MMAs already issued finish before tensor memory is freed
-                umma_commit(mdone);
-                (void)mbar_wait(mdone, 0, true);
-            }
+            if (!ok) break;
+            umma_commit(acc_full(buf), elected);
         }
-    } else {  // epilogue warps 2-5
-        const int quad = warp & 3;
+        if (!ok && kg > 0) {  // let the MMAs already issued finish before tensor memory is freed
+            umma_commit(mdone, elected);
+            (void)mbar_wait(mdone, 0);
+        }
+    } else {  // epilogue warps 2-9
+        const int quad = warp & 3, half = (warp - 2) >> 2;
         const int row = quad * 32 + lane;
         int j = 0;
         for (int t = blockIdx.x; t < total; t += gridDim.x, j++) {
             const int buf = j & 1;
-            const bool ok = mbar_wait(acc_full(buf), (j >> 1) & 1, true, lim, fail);
+            int img, x0, y0, n0;
+            tile_of(t, img, x0, y0, n0);
+            const bool ok = mbar_wait(acc_full(buf), (j >> 1) & 1, lim, fail);
             if (!ok) {
-                if (row == 0) record_error(a.err, 4u);
+                if (row == 0 && half == 0) record_error(a.err, 4u);
                 break;
             }
             tc_fence_after();
-            int img, x0, y0, n0;
-            tile_of(t, img, x0, y0, n0);
-            if (HALO && a.pool)
-                fwd_epilogue_pool2(a, tmem + static_cast<uint32_t>(buf * 2 * a.n_tile), row, quad, img, x0, y0, n0);
-            else
-                for (int r = 0; r < hrows; r++)
-                    fwd_epilogue(a, tmem + static_cast<uint32_t>((buf * hrows + r) * a.n_tile), row, quad, img, x0,
-                                 y0 + r, n0, true);
+            const uint32_t acc = tmem + static_cast<uint32_t>(buf * kRows * a.n_tile);
+            if (HALO && R % 2 == 0 && a.pool) {  // row pairs; one pair: its column groups in turn
+#pragma unroll
+                for (int r = 0; r < R; r += 2)
+                    if (R < 4 || (r >> 1) == half)
+                        fwd_epilogue_pool2(a, acc + static_cast<uint32_t>(r * a.n_tile), row, quad, img, x0, y0 + r, n0,
+                                           R < 4 ? 16 * half : 0, R < 4 ? 32 : 16);
+            } else {  // rows in turn, or one row's column groups
+                for (int r = kRows > 1 ? half : 0; r < kRows; r += kRows > 1 ? 2 : 1)
+                    fwd_epilogue(a, acc + static_cast<uint32_t>(r * a.n_tile), row, quad, img, x0, y0 + r, n0,
+                                 kRows > 1 ? 0 : 16 * half, kRows > 1 ? 16 : 32);
+            }
             tc_fence_before();
             mbar_arrive(acc_empty(buf));
         }
@@ -683,7 +735,7 @@ __global__ void __launch_bounds__(128, 1)
         int k = 0;
         for (; k < nk; k++) {
             const int s = k % S;
-            if (k >= S && !mbar_wait(empty(s), ((k / S) - 1) & 1, false, a.wait_ns)) {
+            if (k >= S && !mbar_wait(empty(s), ((k / S) - 1) & 1, a.wait_ns)) {
                 record_error(a.err, 1u);
                 s_fail = 1;
                 break;
@@ -703,31 +755,37 @@ __global__ void __launch_bounds__(128, 1)
             for (int q = 0; q < nbb; q++) tma_load_4d(sb + q * 128 * RB, &gmap, full(s), n0 + q * KCB, x0, y0, img);
         }
         s_issued = k;
-    } else if (tid == 32) {
+    } else if (warp == 1) {  // the whole warp: descriptors stay uniform
+        const uint32_t elected = elect_one();
         const uint32_t idesc = idesc_bf16(128, a.n_tile, true, true);
-        int k = 0;
+        int k = 0, s = 0;
+        uint32_t phase = 0;
         for (; k < nk; k++) {
-            const int s = k % S;
-            if (!mbar_wait(full(s), (k / S) & 1, false, a.wait_ns)) {
-                record_error(a.err, 2u);
-                s_fail = 1;
+            if (!__all_sync(0xffffffffu, mbar_wait(full(s), phase, a.wait_ns))) {
+                if (elected) {
+                    record_error(a.err, 2u);
+                    s_fail = 1;
+                }
                 break;
             }
             tc_fence_after();
             const uint32_t sa = base + s * a.stage_bytes, sb = sa + a_bytes;
+            const uint64_t da0 = sdesc(sa, 128u * RA, 8u * RA, SWZA), db0 = sdesc(sb, 128u * RB, 8u * RB, SWZB);
 #pragma unroll
-            for (int j = 0; j < 8; j++) {  // 16 pixels per MMA
-                const uint64_t da = sdesc(sa + 16u * RA * j, 128u * RA, 8u * RA, SWZA);
-                const uint64_t db = sdesc(sb + 16u * RB * j, 128u * RB, 8u * RB, SWZB);
-                umma_bf16(tmem, da, db, idesc, (k | j) != 0 ? 1u : 0u);
+            for (int j = 0; j < 8; j++)  // 16 pixels per MMA
+                umma_bf16(tmem, da0 + static_cast<uint64_t>(RA * j), db0 + static_cast<uint64_t>(RB * j), idesc,
+                          (k | j) != 0 ? 1u : 0u, elected);
+            umma_commit(empty(s), elected);
+            if (++s == S) {
+                s = 0;
+                phase ^= 1u;
             }
-            umma_commit(empty(s));
         }
-        s_consumed = k;
-        umma_commit(done);
+        if (elected) s_consumed = k;
+        umma_commit(done, elected);
     }
     __syncwarp();
-    const bool ok = nk > 0 && mbar_wait(done, 0, true, a.wait_ns);
+    const bool ok = nk > 0 && mbar_wait(done, 0, a.wait_ns);
     if (!ok && nk > 0 && tid == 0) record_error(a.err, 4u);
     tc_fence_after();
 
@@ -738,8 +796,10 @@ __global__ void __launch_bounds__(128, 1)
     const uint32_t trow = tmem + (static_cast<uint32_t>(warp * 32) << 16);
     const size_t kdim = 9 * static_cast<size_t>(a.cin);
     for (int c = 0; c < a.n_tile; c += 16) {
+        uint32_t raw[16];
         float v[16];
-        tmem_ld16(trow + c, v);
+        tmem_ld16(trow + c, raw);
+        tmem_wait(raw, v);
         if (!valid && !bias_row) continue;
         float *dst = valid ? a.dw + g : a.db;
         const size_t stride = valid ? kdim : 1;
@@ -978,21 +1038,26 @@ int fwd_prepare(FwdOp *op, const Act &in, const void *w, int w_rows, int cout, c
     int ntiles = (cout_pad + 255) / 256;
     int n_tile = ((cout_pad / ntiles) + 15) / 16 * 16;
     ntiles = (cout_pad + n_tile - 1) / n_tile;
-    // two output rows per halo tile whenever both rows' double-buffered
-    // accumulators fit the 512 tensor-memory columns, even at one CTA per SM
-    // (training step 2.174 vs 2.243 ms against two rows only up to 256
-    // columns); PT_CONV_HALO_ROWS=1..4 overrides
-    int halo_rows = pow2_cols(4 * n_tile) <= 512 ? 2 : 1;
-    if (const char *e = getenv("PT_CONV_HALO_ROWS")) halo_rows = std::min(std::max(atoi(e), 1), 4);
-    while (halo_rows > 1 && pow2_cols(2 * halo_rows * n_tile) > 512) halo_rows--;
+    // Output rows per halo tile: four while both accumulators of every row fit the
+    // 512 tensor-memory columns and three rows' outputs one MMA (N <= 256), else
+    // two or one; fewer where the tiles would not give every SM two.
+    // PT_CONV_HALO_ROWS=1..4 overrides (as far as tensor memory allows).
+    const auto rows_fit = [&](int r) {
+        return pow2_cols(2 * r * n_tile) <= 512 && std::min(r, 3) * n_tile <= 256;
+    };
+    const auto tiles_at = [&](int r) {
+        return (long long)in.n * ((in.w + 127) / 128) * ((in.h + r - 1) / r) * ntiles;
+    };
+    int halo_rows = 4;
+    while (halo_rows > 1 && (!rows_fit(halo_rows) || tiles_at(halo_rows) < 2ll * sm_count())) halo_rows /= 2;
+    if (const char *e = getenv("PT_CONV_HALO_ROWS")) {
+        halo_rows = std::min(std::max(atoi(e), 1), 4);
+        while (halo_rows > 1 && !rows_fit(halo_rows)) halo_rows--;
+    }
     int st;
     if (halo) {
-        if (!getenv_flag("PT_CONV_HALO_PLANES")) {
-            if ((st = act_map_box(&op->act, in, 16, kHaloW, halo_rows + 2, CU_TENSOR_MAP_SWIZZLE_32B, 16)) != PT_OK)
-                return st;
-        } else if ((st = act_map_box(&op->act, in, 8, kHaloW, halo_rows + 2, CU_TENSOR_MAP_SWIZZLE_NONE, 8)) != PT_OK) {
+        if ((st = act_map_box(&op->act, in, 16, kHaloW, halo_rows + 2, CU_TENSOR_MAP_SWIZZLE_32B, 16)) != PT_OK)
             return st;
-        }
     } else if ((st = act_map(&op->act, in, kc, t)) != PT_OK) {
         return st;
     }
@@ -1013,27 +1078,28 @@ int fwd_prepare(FwdOp *op, const Act &in, const void *w, int w_rows, int cout, c
     a.n_tiles_n = ntiles;
     a.tmem_cols = pow2_cols(2 * (halo ? halo_rows : 1) * n_tile);  // double-buffered accumulators
     a.halo_rows = halo_rows;
-    a.halo_box_bytes = halo_box_bytes(halo_rows);
-    a.halo_plane_bytes = halo_plane_bytes(halo_rows);
-    a.halo_sw32 = halo && !getenv_flag("PT_CONV_HALO_PLANES");
-    a.halo_a_tx = a.halo_sw32 ? 2 * halo_box_bytes(halo_rows) : 2 * a.halo_box_bytes;
-    a.halo_a_bytes = a.halo_sw32 ? (a.halo_a_tx + 1023) / 1024 * 1024 : 2 * a.halo_plane_bytes;
-    const int wres_bytes = a.nchunks * 9 * halo_b_tap_bytes(n_tile);
-    a.wres_bytes = (halo && ntiles == 1 && wres_bytes <= kMaxResidentWeights && !getenv_flag("PT_CONV_NO_RESIDENT"))
-                       ? wres_bytes : 0;
-    a.stage_bytes = halo ? a.halo_a_bytes + (a.wres_bytes ? 0 : 9 * halo_b_tap_bytes(n_tile))
+    a.halo_a_bytes = (halo_box_bytes(halo_rows) + 1023) / 1024 * 1024;
+    // CTAs per SM (two at most: 640 threads; PT_CONV_FWD_CTAS=1 or 2 overrides) and
+    // the ring: resident weights where a ring of three stages fits beside them,
+    // at one CTA per SM if need be
+    int ctas = std::min(512 / a.tmem_cols, 2);
+    if (const char *e = getenv("PT_CONV_FWD_CTAS")) ctas = std::min(ctas, std::max(atoi(e), 1));
+    const int wres_bytes = a.nchunks * halo_b_bytes(n_tile);
+    const auto budget_of = [](int c) { return (225 * 1024) / c - 4096; };
+    a.wres_bytes = 0;
+    if (halo && ntiles == 1 && !getenv_flag("PT_CONV_NO_RESIDENT"))
+        for (int c = ctas; c >= 1 && !a.wres_bytes; c--)
+            if (wres_bytes + 3 * a.halo_a_bytes <= budget_of(c)) {
+                a.wres_bytes = wres_bytes;
+                ctas = c;
+            }
+    a.stage_bytes = halo ? a.halo_a_bytes + (a.wres_bytes ? 0 : halo_b_bytes(n_tile))
                          : (128 * 2 * kc + n_tile * 2 * kc + 1023) / 1024 * 1024;
-    // CTAs per SM the ring is sized for (PT_CONV_FWD_CTAS=1..4 overrides):
-    // training step at batch 16 x 256^2 2.308 / 2.251 / 2.298 ms for 2 / 3 / 4
-    int max_ctas = 3;
-    if (const char *e = getenv("PT_CONV_FWD_CTAS")) max_ctas = std::min(std::max(atoi(e), 1), 4);
-    const int target_ctas = std::min(512 / a.tmem_cols, max_ctas);
-    const int budget = (225 * 1024) / target_ctas - 2048 - a.wres_bytes;
-    a.stages = std::max(2, std::min(kMaxStages, budget / a.stage_bytes));
-    // every TMA destination (stage, A box or plane, weight tap region) on a
-    // 1 KiB boundary of the 1 KiB-aligned ring; the producer checks it again
-    if (a.stage_bytes % 1024 || a.wres_bytes % 1024 ||
-        (halo && (a.halo_a_bytes % 1024 || a.halo_plane_bytes % 1024 || halo_b_tap_bytes(n_tile) % 1024))) {
+    if (ctas > 1 && 2 * a.stage_bytes + a.wres_bytes > budget_of(ctas)) ctas = 1;
+    a.stages = std::max(2, std::min(kMaxStages, (budget_of(ctas) - a.wres_bytes) / a.stage_bytes));
+    // every stage, A box and chunk of weights on a 1 KiB boundary of the
+    // 1 KiB-aligned ring (the producer checks it again), a tap's weights on 512 B
+    if (a.stage_bytes % 1024 || a.wres_bytes % 1024 || (halo && (a.halo_a_bytes % 1024 || n_tile % 16))) {
         pt_set_error("conv forward: shared-memory layout off 1 KiB boundaries");
         return PT_ERR_INVALID;
     }
@@ -1068,10 +1134,10 @@ int fwd_prepare(FwdOp *op, const Act &in, const void *w, int w_rows, int cout, c
         a.up = static_cast<uint16_t *>(up);
         a.up_ctot = up_ctot;
     }
-    // the 2x2 average pooling of the output, in the epilogue of two-row halo
-    // tiles (both rows of a pixel pair are in one thread, the pair in
+    // the 2x2 average pooling of the output, in the epilogue of halo tiles of two
+    // or four rows (both rows of a pixel pair are in one thread, the pair in
     // neighbouring lanes); otherwise the caller pools
-    if (pool && halo && halo_rows == 2 && epi == EPI_BF16 && cout % 16 == 0 && in.w % 128 == 0 && in.h % 2 == 0 &&
+    if (pool && halo && halo_rows % 2 == 0 && epi == EPI_BF16 && cout % 16 == 0 && in.w % 2 == 0 && in.h % 2 == 0 &&
         ntiles == 1 && al32(pool, pool_ctot, pool_coff) && al32(out, out_ctot, out_coff) &&
         !getenv_flag("PT_CONV_NO_FUSED_POOL")) {  // (the pooled epilogue writes both outputs with 32-byte stores)
         a.pool = static_cast<uint16_t *>(pool);
@@ -1085,12 +1151,16 @@ int fwd_prepare(FwdOp *op, const Act &in, const void *w, int w_rows, int cout, c
     a.wait_ns = wait_limit_ns();
     a.stall = take_stall_request() ? 1 : 0;
     op->kc = kc;
-    op->halo = halo;
-    while (a.stages > 2 && smem_request(a.stages, a.stage_bytes, a.tmem_cols) + a.wres_bytes > 220 * 1024) a.stages--;
-    op->smem = smem_request(a.stages, a.stage_bytes, a.tmem_cols) + a.wres_bytes;
+    // no more CTAs on an SM than tensor memory holds accumulators for
+    const auto smem_of = [&] {
+        const int by_stages = a.stages * a.stage_bytes + a.wres_bytes + 1024;
+        return std::max(by_stages, (228 * 1024) / (ctas + 1) + 1024);
+    };
+    while (a.stages > 2 && smem_of() > 220 * 1024) a.stages--;
+    op->smem = smem_of();
+    op->rows = halo ? halo_rows : 0;
     const long long total = (long long)in.n * a.tiles_x * a.tiles_y * ntiles;
-    const int per_sm = std::max(1, std::min((228 * 1024) / (op->smem + 1024), 512 / a.tmem_cols));
-    op->grid = dim3(static_cast<unsigned>(std::min<long long>(total, (long long)per_sm * sm_count())), 1, 1);
+    op->grid = dim3(static_cast<unsigned>(std::min<long long>(total, (long long)ctas * sm_count())), 1, 1);
     if (op->smem > 220 * 1024) {
         pt_set_error("conv forward: shared memory request %d too large", op->smem);
         return PT_ERR_INVALID;
@@ -1098,20 +1168,26 @@ int fwd_prepare(FwdOp *op, const Act &in, const void *w, int w_rows, int cout, c
     return PT_OK;
 }
 
-template <int KC, bool HALO>
+template <int KC, int R>
 static int fwd_persistent_go(const FwdOp &op, cudaStream_t stream) {
-    int st = set_smem_attr(k_conv_fwd_persistent<KC, HALO>, op.smem);
+    int st = set_smem_attr(k_conv_fwd_persistent<KC, R>, op.smem);
     if (st != PT_OK) return st;
-    k_conv_fwd_persistent<KC, HALO><<<op.grid, 192, op.smem, stream>>>(op.act, op.wgt, op.args);
+    k_conv_fwd_persistent<KC, R><<<op.grid, kFwdThreads, op.smem, stream>>>(op.act, op.wgt, op.args);
     PT_CUDA_TRY(cudaGetLastError());
     return PT_OK;
 }
 
 int fwd_launch(const FwdOp &op, cudaStream_t stream) {
-    if (op.halo) return fwd_persistent_go<16, true>(op, stream);
-    if (op.kc == 64) return fwd_persistent_go<64, false>(op, stream);
-    if (op.kc == 32) return fwd_persistent_go<32, false>(op, stream);
-    return fwd_persistent_go<16, false>(op, stream);
+    switch (op.rows) {
+        case 1: return fwd_persistent_go<16, 1>(op, stream);
+        case 2: return fwd_persistent_go<16, 2>(op, stream);
+        case 3: return fwd_persistent_go<16, 3>(op, stream);
+        case 4: return fwd_persistent_go<16, 4>(op, stream);
+        default: break;
+    }
+    if (op.kc == 64) return fwd_persistent_go<64, 0>(op, stream);
+    if (op.kc == 32) return fwd_persistent_go<32, 0>(op, stream);
+    return fwd_persistent_go<16, 0>(op, stream);
 }
 
 int wgrad_prepare(WgradOp *op, const Act &x, const Act &gy, float *dw, float *db, int num_sms, unsigned *err) {

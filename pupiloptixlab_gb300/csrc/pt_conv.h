@@ -39,12 +39,12 @@ struct FwdArgs {
     int cin, nchunks;     // K = 9 * cin, in chunks of KC channels per tap
     int n_tile, cout;     // N per CTA; valid output channels
     int tmem_cols, stages, stage_bytes;
-    int halo_a_bytes;     // halo kernel: bytes of the A planes at the start of a stage
+    int halo_a_bytes;     // halo kernel: bytes of the A box at the start of a stage
     int wres_bytes;       // halo kernel: > 0 = all weights resident in shared memory (loaded once per CTA)
     int n_tiles_n;        // output-channel tiles (persistent kernel: tile = pixel tile x channel tile)
     int epi, relu;
     const float *bias;
-    void *out;
+    void *out;            // null (EPI_BF16 with `up`): only the up-sampled copy is written
     int out_ctot, out_coff;
     const uint16_t *mask;
     int mask_ctot, mask_coff;
@@ -52,15 +52,11 @@ struct FwdArgs {
     unsigned long long wait_ns;  // limit of every bounded wait (kWaitNs unless pt_conv_set_wait_limit changed it)
     int stall;                   // test of the timeout path: the MMA warp first waits on a barrier nothing arrives at
     int halo_rows;               // halo kernel: output rows per tile (1-4); the box holds halo_rows + 2 rows
-    int halo_box_bytes;          // halo kernel: bytes of one 8-channel plane as TMA writes it
-    int halo_plane_bytes;        // halo kernel: plane stride (1 KiB-aligned TMA destinations)
     int wide_io;                 // BF16 output / mask rows 32-byte aligned: 256-bit accesses in the epilogue
-    int halo_sw32;               // halo kernel: one 16-channel box per chunk, 32-byte swizzle (else two planes)
-    int halo_a_tx;               // halo kernel: bytes of A the TMA delivers per stage
     int bias16;                  // bias 16-byte aligned: the epilogue reads it in 16-byte loads
     uint16_t *up;                // EPI_BF16: also written, 2x nearest up-sampled, to channels [0, cout) of
     int up_ctot;                 // this (n, 2H, 2W, up_ctot) tensor (the decoder's concatenation)
-    uint16_t *pool;              // halo kernel, two-row tiles, EPI_BF16: the 2x2 average of the BF16 outputs
+    uint16_t *pool;              // halo kernel, tiles of two or four rows, EPI_BF16: the 2x2 average of the BF16 outputs
     int pool_ctot, pool_coff;    // also goes to this (n, H/2, W/2, pool_ctot) tensor at channel pool_coff
 };
 
@@ -84,7 +80,7 @@ struct FwdOp {
     FwdArgs args;
     dim3 grid;
     int smem = 0, kc = 0;
-    bool halo = false;  // halo loads (width >= 128)
+    int rows = 0;       // halo loads (width >= 128): output rows per tile; 0: per-tap loads
 };
 
 struct WgradOp {
@@ -108,7 +104,7 @@ bool take_stall_request();
 
 // Forward (or data-gradient) launch over `in`.  Images at least 128 pixels
 // wide use the halo kernel (one input load per 16-channel chunk for all nine
-// taps, two output rows per tile); the environment variable PT_CONV_NO_HALO=1
+// taps, up to four output rows per tile); the environment variable PT_CONV_NO_HALO=1
 // selects the per-tap kernel for every width, for comparison runs.  `w` holds
 // rows [w_rows][9][in.c] in bf16 (rows beyond w_rows read as zero); `cout`
 // output channels are written to channels [out_coff, out_coff + cout) of `out`
