@@ -509,55 +509,73 @@ __global__ void __launch_bounds__(kFwdThreads, 2)
     volatile int *fail = &s_fail;
 
     if (warp == 0) {
-        if (lane == 0) {  // producer
-            // the nine weight boxes of a chunk: [dx][2 - dy] blocks (tap = 3 dy + dx)
-            const auto load_weights = [&](uint32_t dst, uint32_t bar, int k, int n0) {
-                for (int tap = 0; tap < 9; tap++) {
-                    const int dy = tap / 3, dx = tap - 3 * dy;
-                    tma_load_2d(dst + static_cast<uint32_t>(dx * 3 + 2 - dy) * tap_b, &wgt, bar, tap * a.cin + k * 16, n0);
-                }
-            };
-            if (wres) {
-                mbar_expect_tx(wbar, static_cast<uint32_t>(a.nchunks * 9 * a.n_tile * ROWB));
-                for (int k = 0; k < a.nchunks; k++) load_weights(wbase + static_cast<uint32_t>(k) * chunk_b, wbar, k, 0);
-            }
-            int kg = 0;  // stages issued so far (ring position and phase)
-            int s = 0;
-            uint32_t phase = 0;
-            for (int t = blockIdx.x; t < total && !*fail; t += gridDim.x) {
-                int img, x0, y0, n0;
-                tile_of(t, img, x0, y0, n0);
-                for (int k = 0; k < nk; k++, kg++) {
-                    if (kg >= S && !mbar_wait(empty(s), phase ^ 1u, lim, fail)) {
+        // producer: lane 0 waits for nobody but the ring; the nine weight boxes of a
+        // chunk ([dx][2 - dy] blocks, tap = 3 dy + dx) are issued by nine lanes
+        const int wdy = lane / 3, wdx = lane - 3 * wdy;
+        const auto load_weights = [&](uint32_t dst, uint32_t bar, int k, int n0) {
+            if (lane < 9)
+                tma_load_2d(dst + static_cast<uint32_t>(wdx * 3 + 2 - wdy) * tap_b, &wgt, bar, lane * a.cin + k * 16, n0);
+        };
+        const auto wait = [&](uint32_t bar, uint32_t parity) {  // every lane, one answer
+            return __all_sync(0xffffffffu, mbar_wait(bar, parity, lim, fail)) != 0;
+        };
+        if (wres) {
+            if (lane == 0) mbar_expect_tx(wbar, static_cast<uint32_t>(a.nchunks * 9 * a.n_tile * ROWB));
+            __syncwarp();
+            for (int k = 0; k < a.nchunks; k++) load_weights(wbase + static_cast<uint32_t>(k) * chunk_b, wbar, k, 0);
+        }
+        int kg = 0;  // stages issued so far (ring position and phase)
+        int s = 0;
+        uint32_t phase = 0;
+        bool ok = true;
+        for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+            int img, x0, y0, n0;
+            tile_of(t, img, x0, y0, n0);
+            for (int k = 0; k < nk; k++, kg++) {
+                if (kg >= S && !(ok = wait(empty(s), phase ^ 1u))) {
+                    if (lane == 0) {
                         record_error(a.err, 1u);
                         *fail = 1;
-                        break;
                     }
-                    const uint32_t sa = base + s * a.stage_bytes, sb = sa + a_bytes;
-                    if ((sa | sb) & 1023u) {  // never with a layout fwd_prepare accepted: give up, bounded
+                    break;
+                }
+                const uint32_t sa = base + s * a.stage_bytes, sb = sa + a_bytes;
+                if ((sa | sb) & 1023u) {  // never with a layout fwd_prepare accepted: give up, bounded
+                    if (lane == 0) {
                         record_error(a.err, 8u);
                         *fail = 1;
-                        break;
                     }
+                    ok = false;
+                    break;
+                }
+                if (lane == 0) {
                     mbar_expect_tx(full(s), tx_bytes);
                     if (HALO) {
                         tma_load_4d(sa, &act, full(s), k * 16, x0 - 1, y0 - 1, img);
-                        if (!wres) load_weights(sb, full(s), k, n0);
                     } else {
                         const int tap = k / a.nchunks, ch = k - tap * a.nchunks;
                         const int dy = tap / 3, dx = tap - dy * 3;
                         tma_load_4d(sa, &act, full(s), ch * KC, x0 + dx - 1, y0 + dy - 1, img);
                         tma_load_2d(sb, &wgt, full(s), tap * a.cin + ch * KC, n0);
                     }
-                    if (++s == S) {
-                        s = 0;
-                        phase ^= 1u;
-                    }
+                }
+                if (HALO && !wres) {
+                    __syncwarp();
+                    load_weights(sb, full(s), k, n0);
+                }
+                if (++s == S) {
+                    s = 0;
+                    phase ^= 1u;
                 }
             }
-            // drain: every copy this thread issued has landed before the CTA
-            // leaves (the last issue on each ring slot, and the resident
-            // weights), also when another warp gave up; within the normal limit
+            if (*fail) ok = false;
+            ok = __all_sync(0xffffffffu, ok);
+        }
+        __syncwarp();
+        // drain: every copy this warp issued has landed before the CTA leaves (the
+        // last issue on each ring slot, and the resident weights), also when another
+        // warp gave up; within the normal limit
+        if (lane == 0) {
             for (int k = kg - S; k < kg; k++)
                 if (k >= 0) (void)mbar_wait(full(k % S), (k / S) & 1);
             if (wres) (void)mbar_wait(wbar, 0);
@@ -1027,6 +1045,14 @@ int fwd_prepare(FwdOp *op, const Act &in, const void *w, int w_rows, int cout, c
         pt_set_error("conv forward: mask tensor missing or of the wrong shape");
         return PT_ERR_INVALID;
     }
+    if (!out && !(up && epi == EPI_BF16)) {
+        pt_set_error("conv forward: no output");
+        return PT_ERR_INVALID;
+    }
+    if (!out && !(up && epi == EPI_BF16)) {
+        pt_set_error("conv forward: no output");
+        return PT_ERR_INVALID;
+    }
     if (epi != EPI_F32 && ((out_ctot % 8) || (out_coff % 8))) {
         pt_set_error("conv forward: bf16 output channel stride/offset must be multiples of 8");
         return PT_ERR_INVALID;
@@ -1048,8 +1074,15 @@ int fwd_prepare(FwdOp *op, const Act &in, const void *w, int w_rows, int cout, c
     const auto tiles_at = [&](int r) {
         return (long long)in.n * ((in.w + 127) / 128) * ((in.h + r - 1) / r) * ntiles;
     };
+    const auto box_bytes = [](int r) { return (halo_box_bytes(r) + 1023) / 1024 * 1024; };
+    const int wres_bytes = in.c / 16 * halo_b_bytes(n_tile);
+    const auto resident = [&](int r, int budget) { return ntiles == 1 && wres_bytes + 3 * box_bytes(r) <= budget; };
+    const auto budget_of = [](int ctas) { return (225 * 1024) / ctas - 4096; };
     int halo_rows = 4;
-    while (halo_rows > 1 && (!rows_fit(halo_rows) || tiles_at(halo_rows) < 2ll * sm_count())) halo_rows /= 2;
+    // (weights that do not stay cross L2 once per tile: then one tile for most SMs is enough)
+    while (halo_rows > 1 && (!rows_fit(halo_rows) ||
+                             tiles_at(halo_rows) < (resident(halo_rows, budget_of(1)) ? 2ll * sm_count() : 3ll * sm_count() / 4)))
+        halo_rows /= 2;
     if (const char *e = getenv("PT_CONV_HALO_ROWS")) {
         halo_rows = std::min(std::max(atoi(e), 1), 4);
         while (halo_rows > 1 && !rows_fit(halo_rows)) halo_rows--;
@@ -1078,18 +1111,16 @@ int fwd_prepare(FwdOp *op, const Act &in, const void *w, int w_rows, int cout, c
     a.n_tiles_n = ntiles;
     a.tmem_cols = pow2_cols(2 * (halo ? halo_rows : 1) * n_tile);  // double-buffered accumulators
     a.halo_rows = halo_rows;
-    a.halo_a_bytes = (halo_box_bytes(halo_rows) + 1023) / 1024 * 1024;
+    a.halo_a_bytes = box_bytes(halo_rows);
     // CTAs per SM (two at most: 640 threads; PT_CONV_FWD_CTAS=1 or 2 overrides) and
     // the ring: resident weights where a ring of three stages fits beside them,
     // at one CTA per SM if need be
     int ctas = std::min(512 / a.tmem_cols, 2);
     if (const char *e = getenv("PT_CONV_FWD_CTAS")) ctas = std::min(ctas, std::max(atoi(e), 1));
-    const int wres_bytes = a.nchunks * halo_b_bytes(n_tile);
-    const auto budget_of = [](int c) { return (225 * 1024) / c - 4096; };
     a.wres_bytes = 0;
-    if (halo && ntiles == 1 && !getenv_flag("PT_CONV_NO_RESIDENT"))
+    if (halo && !getenv_flag("PT_CONV_NO_RESIDENT"))
         for (int c = ctas; c >= 1 && !a.wres_bytes; c--)
-            if (wres_bytes + 3 * a.halo_a_bytes <= budget_of(c)) {
+            if (resident(halo_rows, budget_of(c))) {
                 a.wres_bytes = wres_bytes;
                 ctas = c;
             }

@@ -332,11 +332,13 @@ __global__ void k_expm1(const float *o, const uint16_t *x0, long long npix, floa
 
 __device__ __forceinline__ float lum(float r, float g, float b) { return 0.2126f * r + 0.7152f * g + 0.0722f * b; }
 
+// The log colour as the network's input stores it (k_pack_frame).
+__device__ __forceinline__ float log_colour(float c) { return bf2f(f2bf(log1pf(fmaxf(c, 0.f)))); }
 // linear colour of padded-frame pixel q: expm1(network output + input log colour)
-__device__ __forceinline__ float3 denoised(const float *o, const uint16_t *x0, long long q) {
-    return make_float3(fmaxf(expm1f(o[q * 3] + bf2f(x0[q * 16])), 0.f),
-                       fmaxf(expm1f(o[q * 3 + 1] + bf2f(x0[q * 16 + 1])), 0.f),
-                       fmaxf(expm1f(o[q * 3 + 2] + bf2f(x0[q * 16 + 2])), 0.f));
+__device__ __forceinline__ float3 denoised(const float *o, float4 c, long long q) {
+    return make_float3(fmaxf(expm1f(o[q * 3] + log_colour(c.x)), 0.f),
+                       fmaxf(expm1f(o[q * 3 + 1] + log_colour(c.y)), 0.f),
+                       fmaxf(expm1f(o[q * 3 + 2] + log_colour(c.z)), 0.f));
 }
 
 // Left-right mirror of every row of the 16-channel network input, in place
@@ -368,17 +370,26 @@ __global__ void k_mirror_average(float *acc, const float *o, int wp, long long n
 // One block per tile: mean luminance of the raw and the denoised colour and
 // the raw colour's standard error; write the tile's pixels, falling back to
 // the raw colour where the denoised mean moved by more than the threshold.
-__global__ void k_denoise_out(const float4 *color, const float *o, const uint16_t *xin, int w, int h, int wp, int tile,
+// Bound by memory: each thread keeps its first pixel (all of them in tiles of up
+// to 16 x 16) between the two steps, and the log colour is formed again from
+// the colour instead of read back in 32-byte sectors of the network's input.
+__global__ void k_denoise_out(const float4 *color, const float *o, int w, int h, int wp, int tile,
                               float rel, float sig, float4 *out, uint8_t *tile_flag, unsigned *fallback_count) {
     const int tiles_x = (w + tile - 1) / tile;
     const int tx = blockIdx.x % tiles_x, ty = blockIdx.x / tiles_x;
     const int tx0 = tx * tile, ty0 = ty * tile;
     const int tw = min(tile, w - tx0), th = min(tile, h - ty0);
+    float4 kept_c = make_float4(0.f, 0.f, 0.f, 0.f);
+    float3 kept_d = make_float3(0.f, 0.f, 0.f);
     float s_raw = 0.f, s_raw2 = 0.f, s_den = 0.f;
     for (int i = threadIdx.x; i < tw * th; i += blockDim.x) {
         const int x = tx0 + i % tw, y = ty0 + i / tw;
         const float4 c = color[(long long)y * w + x];
-        const float3 dc = denoised(o, xin, (long long)y * wp + x);
+        const float3 dc = denoised(o, c, (long long)y * wp + x);
+        if (i == (int)threadIdx.x) {
+            kept_c = c;
+            kept_d = dc;
+        }
         const float lr = lum(c.x, c.y, c.z);
         s_raw += lr;
         s_raw2 += lr * lr;
@@ -416,11 +427,11 @@ __global__ void k_denoise_out(const float4 *color, const float *o, const uint16_
     for (int i = threadIdx.x; i < tw * th; i += blockDim.x) {
         const int x = tx0 + i % tw, y = ty0 + i / tw;
         const long long q = (long long)y * w + x;
+        const float4 c = i == (int)threadIdx.x ? kept_c : color[q];
         if (fallback) {
-            const float4 c = color[q];
             out[q] = make_float4(c.x, c.y, c.z, 1.f);
         } else {
-            const float3 dc = denoised(o, xin, (long long)y * wp + x);
+            const float3 dc = i == (int)threadIdx.x ? kept_d : denoised(o, c, (long long)y * wp + x);
             out[q] = make_float4(dc.x, dc.y, dc.z, 1.f);
         }
     }
@@ -514,7 +525,14 @@ int plan_prepare(pt_denoiser *dn, Plan &P, int n, int h, int w, bool train) {
     if ((st = alloc_bf16(P.buf, px[lvl] * (c))) != PT_OK) return st;
     PT_A(x0, 0, 16) PT_A(a0, 0, 32) PT_A(cat0, 0, 80) PT_A(p0, 1, 32) PT_A(a1, 1, 48) PT_A(cat1, 1, 112)
     PT_A(p1, 2, 48) PT_A(a2, 2, 64) PT_A(cat2, 2, 192) PT_A(p2, 3, 64) PT_A(a3, 3, 128) PT_A(cat3, 3, 384)
-    PT_A(p3, 4, 128) PT_A(b4, 4, 256) PT_A(d3, 3, 128) PT_A(d2, 2, 64) PT_A(d1, 1, 48) PT_A(d0, 0, 32)
+    PT_A(p3, 4, 128) PT_A(d0, 0, 32)
+    const bool separate_up = getenv("PT_DENOISER_SEPARATE_UPSAMPLE") != nullptr;
+    P.fused_up = !separate_up;
+    // a decoder's own output is read by the backward pass, or to be up-sampled
+    const bool decoder_out = train || separate_up;
+    if (decoder_out) {
+        PT_A(b4, 4, 256) PT_A(d3, 3, 128) PT_A(d2, 2, 64) PT_A(d1, 1, 48)
+    }
     if ((st = P.out.ensure(px[0] * 3 * sizeof(float))) != PT_OK) return st;
     if (train) {
         PT_A(g_out, 0, 16) PT_A(g_d0, 0, 32) PT_A(g_cat0, 0, 80) PT_A(g_d1, 1, 48) PT_A(g_cat1, 1, 112)
@@ -542,8 +560,10 @@ int plan_prepare(pt_denoiser *dn, Plan &P, int n, int h, int w, bool train) {
         {A(P.a0, 0, 32, 0, 32), &P.cat0, 0, 80, 48, nullptr, 0, &P.p0},
         {A(P.p0, 1, 32, 0, 32), &P.a1, 1, 48, 0},
         {A(P.a1, 1, 48, 0, 48), &P.cat1, 1, 112, 64, nullptr, 0, &P.p1},
-        {A(P.p1, 2, 48, 0, 48), &P.a2, 2, 64, 0},         {A(P.a2, 2, 64, 0, 64), &P.cat2, 2, 192, 128},
-        {A(P.p2, 3, 64, 0, 64), &P.a3, 3, 128, 0},        {A(P.a3, 3, 128, 0, 128), &P.cat3, 3, 384, 256},
+        {A(P.p1, 2, 48, 0, 48), &P.a2, 2, 64, 0},
+        {A(P.a2, 2, 64, 0, 64), &P.cat2, 2, 192, 128, nullptr, 0, &P.p2},
+        {A(P.p2, 3, 64, 0, 64), &P.a3, 3, 128, 0},
+        {A(P.a3, 3, 128, 0, 128), &P.cat3, 3, 384, 256, nullptr, 0, &P.p3},
         {A(P.p3, 4, 128, 0, 128), &P.b4, 4, 256, 0, &P.cat3, 384},
         {A(P.cat3, 3, 384, 0, 384), &P.d3, 3, 128, 0, &P.cat2, 192},
         {A(P.cat2, 2, 192, 0, 192), &P.d2, 2, 64, 0, &P.cat1, 112},
@@ -551,14 +571,13 @@ int plan_prepare(pt_denoiser *dn, Plan &P, int n, int h, int w, bool train) {
         {A(P.cat0, 0, 80, 0, 80), &P.d0, 0, 32, 0},       {A(P.d0, 0, 32, 0, 32), &P.out, 0, 3, 0},
     };
     unsigned *err = dn->err.as<unsigned>();
-    const bool separate_up = getenv("PT_DENOISER_SEPARATE_UPSAMPLE") != nullptr;
-    P.fused_up = !separate_up;
     for (int l = 0; l < kLayers; l++) {
         const LayerSpec &L = kSpec[l];
         const bool last = l == OUT;
         if ((st = ptconv::fwd_prepare(&P.fwd[l], io[l].in, wbf_ptr(dn, l), L.cout, last ? kOutChannels : L.cout,
                                       bias_ptr(dn, l), last ? ptconv::EPI_F32 : ptconv::EPI_BF16, L.relu,
-                                      io[l].out->ptr, io[l].octot, io[l].ocoff, nullptr, err,
+                                      io[l].up && !decoder_out ? nullptr : io[l].out->ptr, io[l].octot, io[l].ocoff,
+                                      nullptr, err,
                                       io[l].up && !separate_up ? io[l].up->ptr : nullptr, io[l].up_ctot,
                                       io[l].pool ? io[l].pool->ptr : nullptr, L.cout, 0)) != PT_OK)
             return st;
@@ -630,10 +649,10 @@ int run_forward(pt_denoiser *dn, Plan &P, cudaStream_t s) {
     if (!ptconv::fwd_pooled(P.fwd[E1B])) pool(P.cat1, 112, 64, 48, 1, P.p1);
     PT_TRY(ptconv::fwd_launch(P.fwd[E2A], s));
     PT_TRY(ptconv::fwd_launch(P.fwd[E2B], s));
-    pool(P.cat2, 192, 128, 64, 2, P.p2);
+    if (!ptconv::fwd_pooled(P.fwd[E2B])) pool(P.cat2, 192, 128, 64, 2, P.p2);
     PT_TRY(ptconv::fwd_launch(P.fwd[E3A], s));
     PT_TRY(ptconv::fwd_launch(P.fwd[E3B], s));
-    pool(P.cat3, 384, 256, 128, 3, P.p3);
+    if (!ptconv::fwd_pooled(P.fwd[E3B])) pool(P.cat3, 384, 256, 128, 3, P.p3);
     auto up = [&](const DevBuf &lo, int c, int lvl, DevBuf &cat, int cat_ctot) {
         if (P.fused_up) return;
         const int hh = h >> lvl, ww = w >> lvl;
@@ -1160,11 +1179,10 @@ int pt_denoise(pt_denoiser *dn, const pt_denoise_io *io, void *stream) {
         k_mirror_x0<<<grid_for(npix / 2), 256, 0, s>>>(P.x0.as<uint16_t>(), wp, hp);
         PT_TRY(run_forward(dn, P, s));
         k_mirror_average<<<grid_for(npix), 256, 0, s>>>(P.out_acc.as<float>(), P.out.as<float>(), wp, npix);
-        k_mirror_x0<<<grid_for(npix / 2), 256, 0, s>>>(P.x0.as<uint16_t>(), wp, hp);
         o = P.out_acc.as<float>();
     }
     k_denoise_out<<<tiles, 256, 0, s>>>(reinterpret_cast<const float4 *>(io->color), o,
-                                        P.x0.as<uint16_t>(), w, h, wp, tile,
+                                        w, h, wp, tile,
                                         io->fallback_rel, io->fallback_sigma, reinterpret_cast<float4 *>(io->output),
                                         io->tile_fallback, dn->fallback.as<unsigned>());
     PT_CUDA_TRY(cudaGetLastError());
