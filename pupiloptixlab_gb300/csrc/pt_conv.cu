@@ -837,6 +837,222 @@ __global__ void __launch_bounds__(128, 1)
 }
 
 // ---------------------------------------------------------------------------
+// weight gradient from halo boxes (width >= 128, or a multiple of 16)
+// ---------------------------------------------------------------------------
+// The per-tap kernel above brings every 128-pixel tile of x nine times, in rows
+// as narrow as 32 bytes, and is bound by those copies (16 x 256^2: 80 -> 32
+// channels 222 us, here 121; 32 -> 32 85 us, here 47; 112 -> 48 at half the size 87
+// us, here 59; without the MMAs 87, 34 and 30 us, the copies).  Here a CTA takes one chunk of KCA input channels and all
+// nine taps: one TMA box per tile holds the chunk's (rows + 2) x (tile_w + 2)
+// pixels, and the A operand of a tap is that box read from the tap's pixel on
+// (MN-major: 8-pixel groups SBO = 8 RA bytes apart; any start row works, as in
+// the forward kernel).  M = 128 holds 128 / KCA channel blocks, LBO bytes apart:
+//   KCA = 64: two taps, LBO = their distance; five accumulators
+//             (taps 0 1 | 2 3 | 4 5 | 6 7 | 7 8, the second 7 unused)
+//   KCA = 32, 16: LBO = one pixel, so the blocks are dx = 0, 1, 2 and unused ones;
+//             three accumulators (dy)
+// A K slice is 16 pixels of one row.  Unused blocks read up to five pixels past
+// the box (inside the stage) and only reach unused accumulator rows.  The last
+// chunk may reach past cin: its channels arrive as zeros and are not written.
+// Warps 2 and 3 sum dy over the pixels meanwhile: the bias gradient (CTAs of
+// chunk 0).
+template <int KCA, int KCB, int TW>
+__global__ void __launch_bounds__(128, 1)
+    k_conv_wgrad_halo(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap gmap,
+                      const __grid_constant__ WgradArgs a) {
+    constexpr int RA = KCA * 2, RB = KCB * 2;
+    constexpr uint32_t SWZA = swz_mode<KCA>(), SWZB = swz_mode<KCB>();
+    constexpr int kSets = KCA == 64 ? 5 : 3;
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ __align__(8) uint64_t bars[2 * kMaxStages + 1];
+    __shared__ uint32_t tmem_slot;
+    __shared__ int s_fail;
+    __shared__ float s_db[128];
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    const int S = a.stages;
+    const int chunk = blockIdx.x;
+    s_db[tid] = 0.f;
+    const int n0 = blockIdx.y * a.n_tile;
+    const int nbb = a.n_tile / KCB;
+    const int t_begin = blockIdx.z * a.tiles_per_split;
+    const int nk = max(0, min(a.total_tiles, t_begin + a.tiles_per_split) - t_begin);
+    constexpr int kPitch = TW + 2;  // pixels per row of the box
+    const int tile_px = TW * a.tile_rows;
+    const uint32_t tx_bytes = static_cast<uint32_t>((a.tile_rows + 2) * kPitch * RA + nbb * tile_px * RB);
+    const int tiles_img = a.tiles_x * a.tiles_y;
+    const bool bias = a.db != nullptr && chunk == 0;
+    const uint32_t bar0 = smem_u32(bars);
+    auto full = [&](int s) { return bar0 + 8u * s; };
+    auto empty = [&](int s) { return bar0 + 8u * (kMaxStages + s); };
+    const uint32_t done = bar0 + 8u * (2 * kMaxStages);
+
+    if (warp == 0) tmem_alloc(smem_u32(&tmem_slot), a.tmem_cols);
+    if (tid == 32) {
+        for (int s = 0; s < S; s++) {
+            mbar_init(full(s), 1);
+            mbar_init(empty(s), bias ? 3 : 1);  // the MMAs, and the two summing warps
+        }
+        mbar_init(done, 1);
+        mbar_fence_init();
+        s_fail = 0;
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+    volatile int *fail = &s_fail;
+
+    if (warp == 0) {
+        if (lane == 0) {  // producer
+            int k = 0, s = 0;
+            uint32_t phase = 0;
+            int img = t_begin / tiles_img, ty = (t_begin - img * tiles_img) / a.tiles_x;
+            int tx = t_begin - img * tiles_img - ty * a.tiles_x;
+            for (; k < nk && !*fail; k++) {
+                if (k >= S && !mbar_wait(empty(s), phase ^ 1u, a.wait_ns, fail)) {
+                    record_error(a.err, 1u);
+                    *fail = 1;
+                    break;
+                }
+                const int x0 = tx * TW, y0 = ty * a.tile_rows;
+                const uint32_t sa = base + s * a.stage_bytes, sb = sa + a.a_bytes;
+                mbar_expect_tx(full(s), tx_bytes);
+                tma_load_4d(sa, &xmap, full(s), chunk * KCA, x0 - 1, y0 - 1, img);
+                for (int q = 0; q < nbb; q++) tma_load_4d(sb + q * 128 * RB, &gmap, full(s), n0 + q * KCB, x0, y0, img);
+                if (++s == S) {
+                    s = 0;
+                    phase ^= 1u;
+                }
+                if (++tx == a.tiles_x) {
+                    tx = 0;
+                    if (++ty == a.tiles_y) {
+                        ty = 0;
+                        img++;
+                    }
+                }
+            }
+            // every copy issued has landed before the CTA leaves, also on failure
+            for (int q = k - S; q < k; q++)
+                if (q >= 0) (void)mbar_wait(full(q % S), (q / S) & 1);
+        }
+    } else if (warp == 1) {  // MMA issuer (whole warp: descriptors stay uniform)
+        const uint32_t elected = elect_one();
+        const uint32_t idesc = idesc_bf16(128, a.n_tile, true, true);
+        const int slices = tile_px / 16;
+        // per accumulator set: the A descriptor relative to the stage and the slice's pixel
+        uint64_t dq[kSets];
+#pragma unroll
+        for (int q = 0; q < kSets; q++) {
+            const int t0 = KCA == 64 ? (q < 4 ? 2 * q : 7) : 3 * q, t1 = t0 + 1;  // taps of the first two blocks
+            const uint32_t off = static_cast<uint32_t>((t0 / 3) * kPitch + t0 % 3);
+            const uint32_t lbo = static_cast<uint32_t>((t1 / 3 - t0 / 3) * kPitch + t1 % 3 - t0 % 3);
+            dq[q] = sdesc(off * RA, (KCA == 64 ? lbo : 1u) * RA, 8u * RA, SWZA);
+        }
+        int s = 0;
+        uint32_t phase = 0;
+        for (int k = 0; k < nk; k++) {
+            if (!__all_sync(0xffffffffu, mbar_wait(full(s), phase, a.wait_ns, fail))) {
+                if (elected) {
+                    record_error(a.err, 2u);
+                    *fail = 1;
+                }
+                break;
+            }
+            tc_fence_after();
+            const uint32_t sa = base + s * a.stage_bytes, sb = sa + a.a_bytes;
+            const uint64_t db0 = sdesc(sb, 128u * RB, 8u * RB, SWZB);
+#pragma unroll
+            for (int j = 0; j < 8; j++) {  // 16 pixels of row j / (TW / 16)
+                if (j >= slices) continue;
+                const uint32_t at = (sa >> 4) + static_cast<uint32_t>(j / (TW / 16) * kPitch + j % (TW / 16) * 16) * (RA >> 4);
+#pragma unroll
+                for (int q = 0; q < kSets; q++)
+                    umma_bf16(tmem + static_cast<uint32_t>(q * a.n_tile), dq[q] + at,
+                              db0 + static_cast<uint64_t>(16 * j * (RB >> 4)), idesc, (k | j) != 0 ? 1u : 0u, elected);
+            }
+            umma_commit(empty(s), elected);
+            if (++s == S) {
+                s = 0;
+                phase ^= 1u;
+            }
+        }
+        umma_commit(done, elected);
+    } else if (bias) {  // warps 2, 3: 8 channels of the pixels lane_p, lane_p + step, ... each
+        const int units = a.n_tile / 8, t2 = tid - 64;
+        const int unit = t2 % units, lane_p = t2 / units, step = 64 / units;
+        const bool active = lane_p < step;
+        const int ch = 8 * unit;
+        const uint32_t col = static_cast<uint32_t>((ch / KCB) * 128 * RB + (ch % KCB) * 2);
+        const uint8_t *smem0 = smem_raw - smem_u32(smem_raw);  // + a shared address
+        float sum[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) sum[i] = 0.f;
+        int s = 0;
+        uint32_t phase = 0;
+        bool ok = true;
+        for (int k = 0; k < nk && ok; k++) {
+            ok = __all_sync(0xffffffffu, mbar_wait(full(s), phase, a.wait_ns, fail));
+            if (!ok) break;
+            const uint32_t sb = base + s * a.stage_bytes + a.a_bytes + col;
+#pragma unroll 4
+            for (int p = active ? lane_p : tile_px; p < tile_px; p += step) {
+                uint32_t addr = sb + static_cast<uint32_t>(p) * RB;
+                // the TMA's swizzle: 16-byte unit bits XOR the row bits above 128 bytes
+                addr ^= (addr >> 3) & (KCB == 64 ? 0x70u : KCB == 32 ? 0x30u : 0x10u);
+                const uint4 v = *reinterpret_cast<const uint4 *>(smem0 + addr);
+                const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    sum[2 * i] += __uint_as_float(w[i] << 16);
+                    sum[2 * i + 1] += __uint_as_float(w[i] & 0xffff0000u);
+                }
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(empty(s));
+            if (++s == S) {
+                s = 0;
+                phase ^= 1u;
+            }
+        }
+        if (ok && active)
+#pragma unroll
+            for (int i = 0; i < 8; i++) atomicAdd(&s_db[ch + i], sum[i]);
+    }
+    __syncwarp();
+    const bool ok = nk > 0 && mbar_wait(done, 0, a.wait_ns);
+    if (!ok && nk > 0 && tid == 0) record_error(a.err, 4u);
+    tc_fence_after();
+
+    // epilogue: accumulator row tid = (block, channel) of each set
+    const int blk = tid / KCA, ci = chunk * KCA + tid % KCA;
+    const uint32_t trow = tmem + (static_cast<uint32_t>(warp * 32) << 16);
+    const bool good = __all_sync(0xffffffffu, ok && !*fail);
+    for (int q = 0; q < kSets && good; q++) {
+        const int tap = KCA == 64 ? (q < 4 ? 2 * q + blk : 8) : 3 * q + blk;
+        const bool used = ci < a.cin && (KCA == 64 ? (q < 4 || blk == 1) : blk < 3);
+        float *dst = a.dw + static_cast<size_t>(tap) * a.cin + ci;
+        for (int c = 0; c < a.n_tile; c += 16) {
+            uint32_t raw[16];
+            float v[16];
+            tmem_ld16(trow + static_cast<uint32_t>(q * a.n_tile + c), raw);
+            tmem_wait(raw, v);
+            if (!used) continue;
+#pragma unroll
+            for (int i = 0; i < 16; i++) {
+                const int co = n0 + c + i;
+                if (co < a.cout) atomicAdd(dst + static_cast<size_t>(co) * 9 * a.cin, v[i]);
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (bias && !*fail && tid < a.n_tile && n0 + tid < a.cout) atomicAdd(a.db + n0 + tid, s_db[tid]);
+    if (warp == 0) tmem_dealloc(tmem, a.tmem_cols);
+}
+
+// ---------------------------------------------------------------------------
 // small kernels
 // ---------------------------------------------------------------------------
 __global__ void k_bias_grad(const uint16_t *g, int ctot, int coff, int c, long long npix, float *db) {
@@ -1049,10 +1265,6 @@ int fwd_prepare(FwdOp *op, const Act &in, const void *w, int w_rows, int cout, c
         pt_set_error("conv forward: no output");
         return PT_ERR_INVALID;
     }
-    if (!out && !(up && epi == EPI_BF16)) {
-        pt_set_error("conv forward: no output");
-        return PT_ERR_INVALID;
-    }
     if (epi != EPI_F32 && ((out_ctot % 8) || (out_coff % 8))) {
         pt_set_error("conv forward: bf16 output channel stride/offset must be multiples of 8");
         return PT_ERR_INVALID;
@@ -1221,11 +1433,86 @@ int fwd_launch(const FwdOp &op, cudaStream_t stream) {
     return fwd_persistent_go<16, 0>(op, stream);
 }
 
+// Halo kernel: chunk width by the MMAs a tile takes (accumulator sets x chunks;
+// 48, 64, 112 and wider inputs: 64 channels, 80: 32), equal ones wider.
+static int wgrad_prepare_halo(WgradOp *op, const Act &x, const Act &gy, float *dw, float *db, int num_sms,
+                              unsigned *err) {
+    int kca = 64, cost = 5 * ((x.c + 63) / 64);
+    for (int kc : {32, 16}) {
+        const int c = 3 * ((x.c + kc - 1) / kc);
+        if (c < cost) {
+            cost = c;
+            kca = kc;
+        }
+    }
+    const int sets = kca == 64 ? 5 : 3;
+    // output channels per CTA: a multiple of the dy chunk whose accumulators fit
+    // the 512 tensor-memory columns
+    const int kcb = pick_kc(gy.c);
+    int n_tile = gy.c;
+    while (sets * n_tile > 512 || n_tile > 128 || gy.c % n_tile || n_tile % kcb) n_tile -= 16;
+    Tiling t;
+    // 32 x 4 pixels (16 x 8 where 32 would leave part of every row): 204 pixels of
+    // x per tile instead of the 390 of a 128-pixel row segment
+    t.tile_w = x.w >= 128 || x.w % 32 == 0 ? 32 : 16;
+    t.tile_rows = std::min(128 / t.tile_w, x.h);
+    t.tiles_x = (x.w + t.tile_w - 1) / t.tile_w;
+    t.tiles_y = (x.h + t.tile_rows - 1) / t.tile_rows;
+    int st;
+    if ((st = act_map_box(&op->act, x, kca, t.tile_w + 2, t.tile_rows + 2, swizzle_for(kca), 16)) != PT_OK) return st;
+    if ((st = act_map(&op->grad, gy, kcb, t)) != PT_OK) return st;
+    WgradArgs &a = op->args;
+    memset(&a, 0, sizeof(a));
+    a.n_img = x.n;
+    a.H = x.h;
+    a.W = x.w;
+    a.tile_w = t.tile_w;
+    a.tile_rows = t.tile_rows;
+    a.tiles_x = t.tiles_x;
+    a.tiles_y = t.tiles_y;
+    a.cin = x.c;
+    a.nchunks_a = (x.c + kca - 1) / kca;
+    a.cout = gy.c;
+    a.n_tile = n_tile;
+    a.tmem_cols = pow2_cols(sets * n_tile);
+    a.a_bytes = ((t.tile_rows + 2) * (t.tile_w + 2) * 2 * kca + 1023) / 1024 * 1024;
+    a.stage_bytes = a.a_bytes + 256 * n_tile;
+    // about half an SM's shared memory, so that a data-gradient CTA of the other
+    // stream fits beside it; two stages at least
+    a.stages = std::min(4, std::max(2, (100 * 1024) / a.stage_bytes));
+    a.total_tiles = x.n * t.tiles_x * t.tiles_y;
+    a.db = db;
+    a.ones_row = -1;
+    a.dw = dw;
+    a.err = err;
+    a.wait_ns = wait_limit_ns();
+    op->bias_fused = db != nullptr;
+    op->smem = std::max(a.stages * a.stage_bytes + 1024, (228 * 1024) / (512 / a.tmem_cols + 1) + 1024);
+    const int base_ctas = a.nchunks_a * (gy.c / n_tile);
+    // Pixel ranges: one CTA per SM.  (Fewer, so that fewer CTAs add to the gradient,
+    // measured no faster: 64 -> 64 channels on 16 x 64^2 28 against 25 us.)
+    int splits = std::max(1, std::max(num_sms, 1) / base_ctas);
+    splits = std::min(splits, a.total_tiles);
+    a.tiles_per_split = (a.total_tiles + splits - 1) / splits;
+    splits = (a.total_tiles + a.tiles_per_split - 1) / a.tiles_per_split;
+    op->kca = kca;
+    op->kcb = kcb;
+    op->halo = true;
+    op->grid = dim3(static_cast<unsigned>(a.nchunks_a), static_cast<unsigned>(gy.c / n_tile),
+                    static_cast<unsigned>(splits));
+    if (op->smem > 220 * 1024) {
+        pt_set_error("conv weight gradient: shared memory request %d too large", op->smem);
+        return PT_ERR_INVALID;
+    }
+    return PT_OK;
+}
+
 int wgrad_prepare(WgradOp *op, const Act &x, const Act &gy, float *dw, float *db, int num_sms, unsigned *err) {
     if (x.n != gy.n || x.h != gy.h || x.w != gy.w || x.c % 16 || gy.c % 16 || x.c <= 0 || gy.c <= 0) {
         pt_set_error("conv weight gradient: shapes differ or channels not multiples of 16");
         return PT_ERR_INVALID;
     }
+    if (x.w >= 128 || x.w % 16 == 0) return wgrad_prepare_halo(op, x, gy, dw, db, num_sms, err);
     const int kca = pick_kc(x.c);
     const Tiling t = tiling_for(x.h, x.w);
     // output channels per CTA: a multiple of the dy chunk, at most 256
@@ -1276,6 +1563,7 @@ int wgrad_prepare(WgradOp *op, const Act &x, const Act &gy, float *dw, float *db
     a.wait_ns = wait_limit_ns();
     op->kca = kca;
     op->kcb = kcb;
+    op->halo = false;
     op->grid = dim3(static_cast<unsigned>(m_tiles), static_cast<unsigned>(ntiles), static_cast<unsigned>(splits));
     if (op->smem > 220 * 1024) {
         pt_set_error("conv weight gradient: shared memory request %d too large", op->smem);
@@ -1286,6 +1574,14 @@ int wgrad_prepare(WgradOp *op, const Act &x, const Act &gy, float *dw, float *db
 
 template <int KCA, int KCB>
 static int wgrad_go(const WgradOp &op, cudaStream_t stream) {
+    if (op.halo) {
+        const auto kernel = op.args.tile_w == 32 ? k_conv_wgrad_halo<KCA, KCB, 32> : k_conv_wgrad_halo<KCA, KCB, 16>;
+        const int e = set_smem_attr(kernel, op.smem);
+        if (e != PT_OK) return e;
+        kernel<<<op.grid, 128, op.smem, stream>>>(op.act, op.grad, op.args);
+        PT_CUDA_TRY(cudaGetLastError());
+        return PT_OK;
+    }
     int st = set_smem_attr(k_conv_wgrad<KCA, KCB>, op.smem);
     if (st != PT_OK) return st;
     k_conv_wgrad<KCA, KCB><<<op.grid, 128, op.smem, stream>>>(op.act, op.grad, op.args);

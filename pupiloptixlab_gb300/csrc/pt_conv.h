@@ -66,6 +66,7 @@ struct WgradArgs {
     int cin, nchunks_a;   // A rows: (tap, chunk) blocks of KCA channels, 9 * nchunks_a blocks
     int cout, n_tile;     // N per CTA (a multiple of KCB)
     int tmem_cols, stages, stage_bytes;
+    int a_bytes;          // halo kernel: bytes of the x box at the start of a stage
     int total_tiles, tiles_per_split;
     int zero_fill;        // pixel tiles smaller than 128: clear the stages once
     float *dw;            // [cout][9][cin] FP32, accumulated
@@ -88,6 +89,7 @@ struct WgradOp {
     WgradArgs args;
     dim3 grid;
     int smem = 0, kca = 0, kcb = 0;
+    bool halo = false;        // one x box per tile for all nine taps (width >= 128 or a multiple of 16)
     bool bias_fused = false;  // the kernel also accumulates db (else bias_grad_launch does)
 };
 
