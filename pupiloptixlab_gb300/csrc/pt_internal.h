@@ -70,9 +70,9 @@ struct EmitterSource {
 
 struct RenderWorkspace {
     size_t capacity = 0;  // path slots
-    DevBuf ray, hit, thr, rad, q0, q1, sh_o, sh_d, sh_c, mat_key, counters, sort_tmp;
+    DevBuf paths;       // path state, queues and binning scratch of `capacity` slots
+    DevBuf counters;
     DevBuf bin_blocks;  // material binning: each block's count, then start, per bin
-    size_t sort_capacity = 0;
     // CUDA-graph replay: an internal stream (the caller's may be the legacy
     // default stream, which cannot be captured), events that order it after
     // and before the caller's stream, and the instantiated graph.
@@ -83,6 +83,7 @@ struct RenderWorkspace {
     cudaStream_t side = nullptr;
     cudaEvent_t ev_shade = nullptr, ev_shadow = nullptr;
     cudaGraphExec_t exec = nullptr;
+    std::vector<unsigned char> exec_key;  // the launches that exec replays, by value
 };
 
 struct pt_scene {

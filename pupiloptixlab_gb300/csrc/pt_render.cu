@@ -27,6 +27,7 @@
 
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 namespace {
 using namespace ptd;
@@ -45,7 +46,9 @@ enum Counter : int {
     kNonFinite = 6,  // samples whose radiance was NaN or infinite
     kStatBase = 8,   // uint64 statistics start at counters + 8 (32-byte offset)
 };
-constexpr uint32_t kFirstSet = 24, kSetWords = 8;
+constexpr uint32_t kFixedSets = 24, kSetWords = 8;  // three sets taken in turn, then
+constexpr uint32_t kCallWord = 48;                  // the call's arguments (CallBlock), then
+constexpr uint32_t kFirstSet = 64;                  // a set per bounce
 enum SetCounter : int { kNIn = 0, kNShadow, kWorkExtend, kWorkShadow };
 enum Stat : int { kStatExtNodes = 0, kStatExtPrims, kStatShNodes, kStatShPrims, kStatExtRays, kStatShRays, kNumStats };
 
@@ -53,8 +56,6 @@ struct Wave {
     uint32_t npix;
     uint32_t frames;       // frames in this wave
     uint32_t frame0;       // first frame of the wave (relative to the call)
-    uint32_t seed0;        // random seed of the call's first frame
-    uint32_t cnt0;         // sample_cnt of the call's first frame
     uint32_t last_frame;   // spp - 1: only that frame writes the AOV / test buffers
     uint32_t max_depth;
     uint32_t rng_mode;
@@ -78,6 +79,7 @@ struct State {
     uint32_t *counters;
     uint32_t *cur, *next;  // counter sets of this bounce and the next
     unsigned long long *stats;
+    const struct CallBlock *call;
 };
 constexpr uint32_t kEntryDelta = 1u << 31;  // slots are below 2^31
 PT_DI uint32_t entry_slot(uint32_t e) { return e & ~kEntryDelta; }
@@ -87,6 +89,22 @@ struct Outputs {
     float *albedo, *normal, *test;
     uint32_t drop_nonfinite;  // PT_RENDER_DROP_NONFINITE
 };
+
+// What changes from one call to the next of the same render: read by the kernels
+// from device memory, so that the captured graph stays valid.
+struct CallBlock {
+    Outputs out;
+    uint32_t seed0;  // random seed of the call's first frame
+    uint32_t cnt0;   // sample_cnt of the call's first frame
+};
+static_assert(sizeof(CallBlock) <= 4 * (kFirstSet - kCallWord), "CallBlock does not fit its words");
+
+// Clears the counters (the first `words`) and sets the call's arguments.
+__global__ void k_begin(uint32_t *counters, uint32_t words, CallBlock call) {
+    for (uint32_t i = threadIdx.x; i < words; i += blockDim.x)
+        if (i < kCallWord || i >= kFirstSet) counters[i] = 0;
+    if (threadIdx.x == 0) *reinterpret_cast<CallBlock *>(counters + kCallWord) = call;
+}
 
 // Multi-scene launch (pt_render_batch): the wave's pixel range is the
 // concatenation of every scene's pixels; pix_off[k] is scene k's first.  The
@@ -201,13 +219,13 @@ __global__ void k_raygen(DevScene s, Batch bt, State st, Wave w) {
         const uint32_t r = slot / w.frames, fl = slot - r * w.frames;
         Sampler rng;
         float3 o, d;
+        const uint32_t seed = st.call->seed0 + w.frame0 + fl;
         if (BATCH) {
             const uint32_t k = batch_scene(bt, r);
             const DevScene &sk = bt.scenes[k];
-            raygen_one(sk, tile_pixel(r - bt.pix_off[k], sk.width_px, sk.height_px), w.seed0 + w.frame0 + fl, w.rng_mode,
-                       o, d, rng);
+            raygen_one(sk, tile_pixel(r - bt.pix_off[k], sk.width_px, sk.height_px), seed, w.rng_mode, o, d, rng);
         } else {
-            raygen_one(s, tile_pixel(r, s.width_px, s.height_px), w.seed0 + w.frame0 + fl, w.rng_mode, o, d, rng);
+            raygen_one(s, tile_pixel(r, s.width_px, s.height_px), seed, w.rng_mode, o, d, rng);
         }
         store_ray(st, slot, o, d, rng);
         if (w.bounces == 0) st.rad[slot] = make_float4(0.f, 0.f, 0.f, 0.f);  // else the first bounce starts it
@@ -424,7 +442,7 @@ PT_DI void shade_one(const DevScene &s, const Outputs &out, const State &st, con
         const float3 rad = xyz(st.rad[slot]) + c;
         st.rad[slot] = make_float4(rad.x, rad.y, rad.z, 0.f);
     };
-    Sampler rng = load_rng(o4.w, d4.w, w.rng_mode, w.seed0 + frame);
+    Sampler rng = load_rng(o4.w, d4.w, w.rng_mode, st.call->seed0 + frame);
     int prim = __float_as_int(h.y);
     bool alive = prim >= 0;
     HitGeo g;
@@ -539,7 +557,7 @@ PT_DI void shade_one(const DevScene &s, const Outputs &out, const State &st, con
 // frame of the 1M-triangle field, 0.209 / 0.226 / 0.246 ms on the Cornell box.
 // 32.7 ms with a path's ray, stream and flags in separate 4- to 16-byte arrays.
 template <bool BATCH>
-__global__ void __launch_bounds__(256, 4) k_shade(DevScene s, Batch bt, State st, Wave w, Outputs out) {
+__global__ void __launch_bounds__(256, 4) k_shade(DevScene s, Batch bt, State st, Wave w) {
     __shared__ uint32_t push_smem[72];
     const uint32_t n = st.cur[kNIn];
     const float env_pdf = 0.25f * kInvPi;  // ConstEnvEmitter::Eval (env.h:82-85)
@@ -556,7 +574,7 @@ __global__ void __launch_bounds__(256, 4) k_shade(DevScene s, Batch bt, State st
                 const uint32_t k = batch_scene(bt, r);
                 shade_one(bt.scenes[k], bt.outs[k], st, w, entry, fl, r - bt.pix_off[k], env_pdf, so);
             } else {
-                shade_one(s, out, st, w, entry, fl, r, env_pdf, so);
+                shade_one(s, st.call->out, st, w, entry, fl, r, env_pdf, so);
             }
         }
         uint32_t pos_ext, pos_sh;
@@ -758,17 +776,19 @@ __global__ void k_bin_scatter_batch(Batch bt, State st, const uint16_t *keys, ui
 // thread's frames are neighbours in memory; they are loaded eight at a time
 // (one 128-byte line per pixel) so that each line is fetched once.
 template <bool BATCH>
-__global__ void k_accumulate(State st, Wave w, Outputs out0, Batch bt, uint32_t width, uint32_t height) {
+__global__ void k_accumulate(State st, Wave w, Batch bt, uint32_t width, uint32_t height) {
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < w.npix; q += gridDim.x * blockDim.x) {
         uint32_t p;
-        Outputs out = out0;
+        Outputs out;
         if (BATCH) {
             const uint32_t k = batch_scene(bt, q);
             out = bt.outs[k];
             p = tile_pixel(q - bt.pix_off[k], bt.scenes[k].width_px, bt.scenes[k].height_px);
         } else {
+            out = st.call->out;
             p = tile_pixel(q, width, height);
         }
+        const uint32_t cnt0 = st.call->cnt0 + w.frame0;
         float4 acc = out.accum[p];
         float3 a = xyz(acc);
         const float4 *rad = st.rad + (size_t)q * w.frames;
@@ -784,7 +804,7 @@ __global__ void k_accumulate(State st, Wave w, Outputs out0, Batch bt, uint32_t 
                     atomicAdd(st.counters + kNonFinite, 1u);
                     if (out.drop_nonfinite) L = f3s(0.f);
                 }
-                const uint32_t cnt = w.cnt0 + w.frame0 + f0 + k;
+                const uint32_t cnt = cnt0 + f0 + k;
                 if (w.accumulate && cnt > 0) {
                     const float t = 1.f / (cnt + 1.f);
                     L = lerp(a, L, t);
@@ -857,6 +877,10 @@ int set_smem(F kernel, size_t bytes) {
     if (bytes > 48 * 1024) PT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
     return PT_OK;
 }
+
+// A path slot of the workspace: ray, hit, throughput, radiance, shadow ray (3),
+// two queues, the binned queue and its keys.
+constexpr size_t kSlotBytes = 32 + 6 * 16 + 3 * 4 + 2;
 
 // Events for per-kernel timing (PT_RENDER_KERNEL_TIMING).
 struct Timer {
@@ -933,29 +957,41 @@ struct Launcher {
                          frames_per_wave, npix);
             return PT_ERR_INVALID;
         }
-        if (ws.capacity < cap) {
-            int e;
-            if ((e = ws.ray.ensure(32 * cap)) || (e = ws.hit.ensure(16 * cap)) ||
-                (e = ws.thr.ensure(16 * cap)) || (e = ws.rad.ensure(16 * cap)) ||
-                (e = ws.q0.ensure(4 * cap)) || (e = ws.q1.ensure(4 * cap)) ||
-                (e = ws.sh_o.ensure(16 * cap)) || (e = ws.sh_d.ensure(16 * cap)) || (e = ws.sh_c.ensure(16 * cap)))
-                return e;
-            ws.capacity = cap;
-        }
         const size_t set_bytes = 4 * (size_t)kSetWords * (bounces + 1);
         const size_t counter_bytes = 4 * kFirstSet + set_bytes;
-        int e = ws.counters.ensure(std::max<size_t>(counter_bytes, 256));
+        int e = ws.counters.ensure(counter_bytes);
         if (e != PT_OK) return e;
+        if (ws.capacity < cap) {  // one allocation, carved below: ten of them took most of a small scene's first call
+            if ((e = ws.paths.ensure(kSlotBytes * ((cap + 15) / 16 * 16))) != PT_OK) {
+                ws.capacity = 0;
+                return e;
+            }
+            ws.capacity = (cap + 15) / 16 * 16;
+        }
+        char *at = ws.paths.as<char>();
+        const auto carve = [&](auto *&ptr, size_t bytes_per_slot) {
+            ptr = reinterpret_cast<std::remove_reference_t<decltype(ptr)>>(at);
+            at += bytes_per_slot * ws.capacity;
+        };
         State stt;
-        stt.ray = ws.ray.as<float4>();
-        stt.hit = ws.hit.as<float4>();
-        stt.thr = ws.thr.as<float4>();
-        stt.rad = ws.rad.as<float4>();
-        stt.sh_o = ws.sh_o.as<float4>();
-        stt.sh_d = ws.sh_d.as<float4>();
-        stt.sh_c = ws.sh_c.as<float4>();
+        uint32_t *q0, *q1, *q_sorted;
+        uint16_t *bin_keys;
+        carve(stt.ray, 32);
+        carve(stt.hit, 16);
+        carve(stt.thr, 16);
+        carve(stt.rad, 16);
+        carve(stt.sh_o, 16);
+        carve(stt.sh_d, 16);
+        carve(stt.sh_c, 16);
+        carve(q0, 4);
+        carve(q1, 4);
+        carve(q_sorted, 4);
+        carve(bin_keys, 2);
         stt.counters = ws.counters.as<uint32_t>();
-        stt.stats = reinterpret_cast<unsigned long long *>(ws.counters.as<uint32_t>() + kStatBase);
+        stt.stats = reinterpret_cast<unsigned long long *>(stt.counters + kStatBase);
+        stt.call = reinterpret_cast<const CallBlock *>(stt.counters + kCallWord);
+        stt.q_in = stt.q_out = nullptr;
+        stt.cur = stt.next = nullptr;
 
         const int tb = p->block_size ? (int)p->block_size : (t.tuned_block ? (int)t.tuned_block : 128);
         const size_t smem = (size_t)d.smem_nodes * 32 * K + (size_t)kShortStack * stack_entry_bytes(false) * tb;
@@ -974,10 +1010,6 @@ struct Launcher {
         const uint32_t grid_shade = (uint32_t)std::max(1, occ_s) * t.num_sms;
 
         const bool sort = (p->flags & PT_RENDER_NO_MATERIAL_SORT) == 0 && !t.one_bsdf;
-        if (sort && ws.sort_capacity < cap) {
-            if ((e = ws.mat_key.ensure(2 * cap)) != PT_OK || (e = ws.sort_tmp.ensure(4 * cap)) != PT_OK) return e;
-            ws.sort_capacity = cap;
-        }
         int occ_b = 0;
         PT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_b, k_bin_scatter, 256, 0));
         const uint32_t grid_bin = (uint32_t)std::max(1, occ_b) * t.num_sms;
@@ -985,8 +1017,12 @@ struct Launcher {
 
         // The whole render is captured into a CUDA graph on the scene's own
         // stream (ordered after and before the caller's stream by events) and
-        // replayed; later calls update the instantiated graph in place.  The
-        // graph has a second branch: a bounce's shadow rays run beside the next
+        // replayed.  What a call may change freely (seed, sample count, buffers) is
+        // in the call block, so a call whose launches are the last one's, argument
+        // for argument, replays the instantiated graph as it is; any other is captured
+        // again and updates it in place.  A 256 x 256 preview call took 192 us with a
+        // capture per call, 170 replayed (151 of them on the device).
+        // The graph has a second branch: a bounce's shadow rays run beside the next
         // bounce's extension rays and binning (they meet before shading, which
         // adds to the same radiance), so that the last long rays of one kernel
         // do not leave the chip idle: 1M-triangle field at 1080p, 1 spp 4.27 ->
@@ -1002,29 +1038,52 @@ struct Launcher {
             PT_CUDA_TRY(cudaEventCreateWithFlags(&ws.ev_shadow, cudaEventDisableTiming));
         }
         cudaStream_t ls = graph ? ws.stream : st;
+        std::vector<unsigned char> key;  // every value the launches below depend on
         if (graph) {
+            const auto add = [&](const auto &v) {
+                const auto *b = reinterpret_cast<const unsigned char *>(&v);
+                key.insert(key.end(), b, b + sizeof(v));
+            };
+            const void *kernels[] = {reinterpret_cast<const void *>(k_ext), reinterpret_cast<const void *>(k_sh)};
+            const size_t launch[] = {smem, smem_sh, (size_t)tb, grid_trace, grid_shadow, grid_shade, grid_bin};
+            const uint32_t call[] = {npix, max_depth, bounces, p->spp, frames_per_wave, p->rng, p->accumulate, sort};
+            add(d);
+            add(bt);
+            add(stt);
+            add(kernels);
+            add(launch);
+            add(call);
+            add(ws.capacity);
+            add(ws.bin_blocks.ptr);
             PT_CUDA_TRY(cudaEventRecord(ws.ev_in, st));
             PT_CUDA_TRY(cudaStreamWaitEvent(ws.stream, ws.ev_in, 0));
-            PT_CUDA_TRY(cudaStreamBeginCapture(ws.stream, cudaStreamCaptureModeThreadLocal));
         }
+        const bool replay = graph && ws.exec && key == ws.exec_key;
+        k_begin<<<1, 256, 0, ls>>>(stt.counters, (uint32_t)(counter_bytes / 4), CallBlock{out, p->seed, p->sample_cnt});
+        PT_CUDA_TRY(cudaGetLastError());
+        if (graph && !replay) PT_CUDA_TRY(cudaStreamBeginCapture(ws.stream, cudaStreamCaptureModeThreadLocal));
         Timer tm;
-        uint32_t launches = 0;
+        uint32_t launches = 1;
         uint32_t waves = 0;
-        pt_nvtx::Range nv_render(graph ? "pt_render: capture" : "pt_render: launches");
+        pt_nvtx::Range nv_render(replay ? "pt_render: replay" : graph ? "pt_render: capture" : "pt_render: launches");
         if (!graph) PT_CUDA_TRY(cudaEventRecord(t.ev0, st));
-        cudaError_t enq = cudaMemsetAsync(ws.counters.ptr, 0, counter_bytes, ls);
+        cudaError_t enq = cudaSuccess;
         const auto order = [&](cudaStream_t from, cudaStream_t to, cudaEvent_t ev) {  // `to` continues after `from`
             if (from == to || enq != cudaSuccess) return;
             enq = cudaEventRecord(ev, from);
             if (enq == cudaSuccess) enq = cudaStreamWaitEvent(to, ev, 0);
         };
         for (uint32_t f0 = 0; f0 < p->spp && enq == cudaSuccess; f0 += frames_per_wave) {
+            if (replay) {  // counted as captured
+                const uint32_t full = bounces ? bounces - 1 : 0;
+                launches += 2 + 2 * bounces + full * (sort ? 4 : 1);
+                waves++;
+                continue;
+            }
             Wave w;
             w.npix = npix;
             w.frames = std::min(frames_per_wave, p->spp - f0);
             w.frame0 = f0;
-            w.seed0 = p->seed;
-            w.cnt0 = p->sample_cnt;
             w.last_frame = p->spp - 1;
             w.max_depth = max_depth;
             w.rng_mode = p->rng;
@@ -1033,8 +1092,8 @@ struct Launcher {
             w.bounces = bounces;
             const size_t slots = (size_t)w.frames * npix;
             uint32_t *sets = stt.counters + kFirstSet;
-            stt.q_in = ws.q0.as<uint32_t>();
-            stt.q_out = ws.q1.as<uint32_t>();
+            stt.q_in = q0;
+            stt.q_out = q1;
             stt.cur = sets;
             stt.next = sets;
             pt_nvtx::Range nv_wave("wave");
@@ -1045,7 +1104,7 @@ struct Launcher {
             }
             launches++;
             cudaStream_t ss = graph ? ws.side : ls;  // the shadow rays' branch
-            uint32_t *q_sorted = ws.sort_tmp.as<uint32_t>(), *bin_blocks = ws.bin_blocks.as<uint32_t>();
+            uint32_t *bin_blocks = ws.bin_blocks.as<uint32_t>();
             for (uint32_t b = 0; b < bounces && enq == cudaSuccess; b++) {
                 w.bounce = b;
                 stt.cur = sets + (size_t)kSetWords * b;
@@ -1062,12 +1121,11 @@ struct Launcher {
                 State shade_st = stt;
                 if (sort && !last_bounce) {  // the last bounce evaluates no BSDF
                     if (BATCH) {
-                        uint16_t *keys = ws.mat_key.as<uint16_t>();
-                        k_bin_count_batch<<<grid_bin, 256, bt.nbins * 4, ls>>>(bt, w.frames, stt, keys);
+                        k_bin_count_batch<<<grid_bin, 256, bt.nbins * 4, ls>>>(bt, w.frames, stt, bin_keys);
                         k_bin_scan_batch<<<1, 1024, 0, ls>>>(bt);
-                        k_bin_scatter_batch<<<grid_bin, 256, 2 * bt.nbins * 4, ls>>>(bt, stt, keys, q_sorted);
+                        k_bin_scatter_batch<<<grid_bin, 256, 2 * bt.nbins * 4, ls>>>(bt, stt, bin_keys, q_sorted);
                     } else {
-                        uint8_t *keys = ws.mat_key.as<uint8_t>();
+                        uint8_t *keys = reinterpret_cast<uint8_t *>(bin_keys);
                         k_bin_count<<<grid_bin, 256, 0, ls>>>(d, stt, keys, bin_blocks);
                         k_bin_scan<<<1, 32 * kNumBins, 0, ls>>>(bin_blocks, grid_bin);
                         k_bin_scatter<<<grid_bin, 256, 0, ls>>>(stt, keys, bin_blocks, q_sorted);
@@ -1080,7 +1138,7 @@ struct Launcher {
                 if (timing) tm.mark(2, ls);
                 {
                     pt_nvtx::Range r("shade (MIS, NEE, BSDF sample)");
-                    k_shade<BATCH><<<grid_shade, 256, 0, ls>>>(d, bt, shade_st, w, out);
+                    k_shade<BATCH><<<grid_shade, 256, 0, ls>>>(d, bt, shade_st, w);
                 }
                 launches++;
                 if (timing) tm.mark(2, ls);
@@ -1098,13 +1156,14 @@ struct Launcher {
             }
             {
                 pt_nvtx::Range r("accumulate");
-                k_accumulate<BATCH><<<nblocks(npix, 256), 256, 0, ls>>>(stt, w, out, bt, d.width_px, d.height_px);
+                k_accumulate<BATCH><<<nblocks(npix, 256), 256, 0, ls>>>(stt, w, bt, d.width_px, d.height_px);
             }
             launches++;
             waves++;
             if (enq == cudaSuccess) enq = cudaGetLastError();
         }
-        if (graph) {
+        if (graph && !replay) {
+            ws.exec_key.clear();  // until the graph below is the executable one
             cudaGraph_t g = nullptr;
             cudaError_t ec = cudaStreamEndCapture(ws.stream, &g);
             if (enq != cudaSuccess || ec != cudaSuccess) {
@@ -1132,24 +1191,25 @@ struct Launcher {
                 }
             }
             cudaGraphDestroy(g);
+            ws.exec_key.swap(key);
+        } else if (enq != cudaSuccess) {
+            pt_set_error("kernel launch failed: %s", cudaGetErrorString(enq));
+            return PT_ERR_CUDA;
+        }
+        if (graph) {
             pt_nvtx::Range r("pt_render: graph launch");
             PT_CUDA_TRY(cudaEventRecord(t.ev0, ws.stream));
             PT_CUDA_TRY(cudaGraphLaunch(ws.exec, ws.stream));
             PT_CUDA_TRY(cudaEventRecord(t.ev1, ws.stream));
             PT_CUDA_TRY(cudaEventRecord(ws.ev_out, ws.stream));
             PT_CUDA_TRY(cudaStreamWaitEvent(st, ws.ev_out, 0));
-        } else {
-            if (enq != cudaSuccess) {
-                pt_set_error("kernel launch failed: %s", cudaGetErrorString(enq));
-                return PT_ERR_CUDA;
-            }
-        }
-        PT_CUDA_TRY(cudaGetLastError());
-        if (!graph) {
-            // direct launches: time the enqueued work with events around it on the caller's stream
+        } else {  // direct launches: time the enqueued work with events around it on the caller's stream
+            PT_CUDA_TRY(cudaGetLastError());
             PT_CUDA_TRY(cudaEventRecord(t.ev1, st));
         }
-        PT_CUDA_TRY(cudaEventSynchronize(t.ev1));
+        uint32_t hc[8 + 2 * kNumStats] = {};
+        PT_CUDA_TRY(cudaMemcpyAsync(hc, ws.counters.ptr, sizeof(hc), cudaMemcpyDeviceToHost, ls));
+        PT_CUDA_TRY(cudaStreamSynchronize(ls));
         pt_render_stats &rs = *t.rs;
         rs = pt_render_stats{};
         PT_CUDA_TRY(cudaEventElapsedTime(&rs.render_ms, t.ev0, t.ev1));
@@ -1160,8 +1220,6 @@ struct Launcher {
             else if (tm.kind[i] == 1) { rs.shadow_ms += ms; rs.shadow_launches++; }
             else { rs.shade_ms += ms; rs.shade_launches++; }
         }
-        uint32_t hc[8 + 2 * kNumStats] = {};
-        PT_CUDA_TRY(cudaMemcpy(hc, ws.counters.ptr, sizeof(hc), cudaMemcpyDeviceToHost));
         const unsigned long long *hs = reinterpret_cast<const unsigned long long *>(hc + kStatBase);
         rs.samples = (uint64_t)npix * p->spp;
         rs.nodes_visited = hs[kStatExtNodes];
@@ -1200,7 +1258,7 @@ struct Launcher {
         uint32_t *c = s->ws.counters.as<uint32_t>();
         PT_CUDA_TRY(cudaMemsetAsync(c, 0, 256, st));
         if (n) kern<<<(uint32_t)std::max(1, occ) * s->num_sms, tb, smem, st>>>(
-            d, reinterpret_cast<const float4 *>(rays), reinterpret_cast<float4 *>(hits), n, c + kFirstSet + kWorkExtend, c + kOverflow);
+            d, reinterpret_cast<const float4 *>(rays), reinterpret_cast<float4 *>(hits), n, c + kFixedSets + kWorkExtend, c + kOverflow);
         PT_CUDA_TRY(cudaGetLastError());
         uint32_t ovf = 0;
         PT_CUDA_TRY(cudaMemcpyAsync(&ovf, c + kOverflow, 4, cudaMemcpyDeviceToHost, st));
@@ -1245,8 +1303,7 @@ void pt_batch_release(BatchWorkspace *b) {
     DevBuf *bufs[] = {&b->nodes, &b->cnodes, &b->prims, &b->scenes, &b->outs, &b->pix_off, &b->roots, &b->bins};
     for (DevBuf *d : bufs) d->release();
     RenderWorkspace &w = b->ws;
-    DevBuf *wb[] = {&w.ray, &w.hit, &w.thr, &w.rad, &w.q0,
-                    &w.q1, &w.sh_o, &w.sh_d, &w.sh_c, &w.mat_key, &w.counters, &w.sort_tmp, &w.bin_blocks};
+    DevBuf *wb[] = {&w.paths, &w.counters, &w.bin_blocks};
     for (DevBuf *d : wb) d->release();
     if (w.exec) cudaGraphExecDestroy(w.exec);
     if (w.ev_in) cudaEventDestroy(w.ev_in);
@@ -1340,7 +1397,7 @@ int render_batch(pt_context *ctx, pt_scene *const *scenes, const pt_render_param
     dt.num_nodes = static_cast<uint32_t>(total_nodes);
     dt.smem_nodes = 0;
     dt.pad_mag = pad_mag;
-    Batch bt;
+    Batch bt{};
     bt.scenes = b.scenes.as<DevScene>();
     bt.outs = b.outs.as<Outputs>();
     bt.pix_off = b.pix_off.as<uint32_t>();
@@ -1570,6 +1627,7 @@ int render_noalloc(pt_scene *s, const pt_render_params *p, const pt_frame_buffer
     };
     stt.counters = reinterpret_cast<uint32_t *>(scratch);
     stt.stats = reinterpret_cast<unsigned long long *>(stt.counters + kStatBase);
+    stt.call = reinterpret_cast<const CallBlock *>(stt.counters + kCallWord);
     stt.ray = reinterpret_cast<float4 *>(take(32));
     stt.hit = reinterpret_cast<float4 *>(take(16));
     stt.thr = reinterpret_cast<float4 *>(take(16));
@@ -1605,14 +1663,12 @@ int render_noalloc(pt_scene *s, const pt_render_params *p, const pt_frame_buffer
     const uint32_t grid_shade = (uint32_t)std::max(1, occ_s) * s->num_sms;
 
     // the array keeps the previous call's contents: clear the counters and statistics
-    PT_CUDA_TRY(cudaMemsetAsync(scratch, 0, kNoAllocCounterBytes, st));
+    k_begin<<<1, 256, 0, st>>>(stt.counters, kNoAllocCounterBytes / 4, CallBlock{out, p->seed, p->sample_cnt});
     for (uint32_t f0 = 0; f0 < p->spp; f0 += frames_per_wave) {
         Wave w;
         w.npix = npix;
         w.frames = std::min(frames_per_wave, p->spp - f0);
         w.frame0 = f0;
-        w.seed0 = p->seed;
-        w.cnt0 = p->sample_cnt;
         w.last_frame = p->spp - 1;
         w.max_depth = max_depth;
         w.rng_mode = p->rng;
@@ -1621,20 +1677,20 @@ int render_noalloc(pt_scene *s, const pt_render_params *p, const pt_frame_buffer
         w.bounces = max_depth;
         stt.q_in = q0;
         stt.q_out = q1;
-        stt.cur = stt.counters + kFirstSet;
+        stt.cur = stt.counters + kFixedSets;
         if (f0) PT_CUDA_TRY(cudaMemsetAsync(stt.cur, 0, 3 * kSetWords * 4, st));
         k_raygen<false><<<nblocks((size_t)w.frames * npix, 256), 256, 0, st>>>(d, Batch{}, stt, w);
         for (uint32_t b = 0; b < max_depth; b++) {
             w.bounce = b;
-            stt.cur = stt.counters + kFirstSet + kSetWords * (b % 3);
-            stt.next = stt.counters + kFirstSet + kSetWords * ((b + 1) % 3);
+            stt.cur = stt.counters + kFixedSets + kSetWords * (b % 3);
+            stt.next = stt.counters + kFixedSets + kSetWords * ((b + 1) % 3);
             if (b > 0) k_advance<<<1, 32, 0, st>>>(stt.next);  // sets 0 and 1 start clear
             k_ext<<<grid_trace, tb, smem, st>>>(d, stt, Batch{}, w.frames);
-            k_shade<false><<<grid_shade, 256, 0, st>>>(d, Batch{}, stt, w, out);
+            k_shade<false><<<grid_shade, 256, 0, st>>>(d, Batch{}, stt, w);
             if (b + 1 < max_depth) k_sh<<<grid_shadow, tb, smem_sh, st>>>(d, stt, Batch{}, w.frames);  // the last bounce casts none
             std::swap(stt.q_in, stt.q_out);
         }
-        k_accumulate<false><<<nblocks(npix, 256), 256, 0, st>>>(stt, w, out, Batch{}, d.width_px, d.height_px);
+        k_accumulate<false><<<nblocks(npix, 256), 256, 0, st>>>(stt, w, Batch{}, d.width_px, d.height_px);
     }
     PT_CUDA_TRY(cudaGetLastError());
     // the overflow and non-finite counters are adjacent: one small read-back

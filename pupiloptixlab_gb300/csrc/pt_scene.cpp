@@ -824,9 +824,8 @@ void DevBuf::release() {
 
 pt_scene::~pt_scene() {
     DevBuf *all[] = {&prims_world, &prims_bvh, &nodes, &cnodes, &tri_vidx, &vpos, &vnrm, &vuv, &prim_inst, &inst, &mats, &curve_seg, &curve_cp,
-                     &emitters, &emitter_cdf, &emitter_tex, &mesh_obj_pos, &bvh_scratch, &bvh_order, &sah_scratch, &xform_table, &all_obj_pos, &ws.ray, &ws.hit, &ws.thr,
-                     &ws.rad, &ws.q0, &ws.q1, &ws.sh_o, &ws.sh_d, &ws.sh_c, &ws.mat_key,
-                     &ws.counters, &ws.sort_tmp, &ws.bin_blocks};
+                     &emitters, &emitter_cdf, &emitter_tex, &mesh_obj_pos, &bvh_scratch, &bvh_order, &sah_scratch, &xform_table, &all_obj_pos,
+                     &ws.paths, &ws.counters, &ws.bin_blocks};
     for (DevBuf *b : all) b->release();
     env_row_cdf.release();
     env_col_cdf.release();
