@@ -736,14 +736,14 @@ __device__ __forceinline__ void padded(float4 lo, float4 hi, float scene_mag, fl
 }
 
 template <int K>
-__device__ __forceinline__ void write_slot(float *node, int c, float3 lo, float3 hi, int child, int count) {
-    node[c] = lo.x;
-    node[K + c] = hi.x;
-    node[2 * K + c] = lo.y;
-    node[3 * K + c] = hi.y;
-    node[4 * K + c] = lo.z;
-    node[5 * K + c] = hi.z;
-    node[6 * K + c] = __int_as_float(count > 0 ? ptd::make_leaf(child, count) : child);
+__device__ __forceinline__ void write_slot(float *node, uint32_t swz, int c, float3 lo, float3 hi, int child, int count) {
+    node[c ^ swz] = lo.x;
+    node[(K + c) ^ swz] = hi.x;
+    node[(2 * K + c) ^ swz] = lo.y;
+    node[(3 * K + c) ^ swz] = hi.y;
+    node[(4 * K + c) ^ swz] = lo.z;
+    node[(5 * K + c) ^ swz] = hi.z;
+    node[(6 * K + c) ^ swz] = __int_as_float(count > 0 ? ptd::make_leaf(child, count) : child);
 }
 __device__ __forceinline__ int item_count(int item) { return ptd::is_leaf(item) ? ptd::leaf_count(item) : 0; }
 // The primitives of leaf x (at most 15), depth first, from position `first` on.
@@ -887,10 +887,13 @@ __global__ void __launch_bounds__(128) k_collapse(const Tree t, BuildCounts *bc,
             f[7 * K + c] = 0.f;
         }
         float4 *node = reinterpret_cast<float4 *>(nodes) + (size_t)(start + k) * 2 * K;
+        const uint32_t x4 = ptd::node_swizzle<K>(start + k) / 4;
 #pragma unroll
-        for (int i = 0; i < K; i++)
-            ptd::st8(node + 2 * i, make_float4(f[8 * i], f[8 * i + 1], f[8 * i + 2], f[8 * i + 3]),
-                     make_float4(f[8 * i + 4], f[8 * i + 5], f[8 * i + 6], f[8 * i + 7]));
+        for (int i = 0; i < K; i++) {
+            const float4 a = make_float4(f[8 * i], f[8 * i + 1], f[8 * i + 2], f[8 * i + 3]);
+            const float4 b = make_float4(f[8 * i + 4], f[8 * i + 5], f[8 * i + 6], f[8 * i + 7]);
+            ptd::st8(node + ((2 * i) ^ (x4 & ~1u)), x4 & 1 ? b : a, x4 & 1 ? a : b);
+        }
         if (level == 0) {
             const double ex = rhi.x - rlo.x, ey = rhi.y - rlo.y, ez = rhi.z - rlo.z;
             bc->root_area = ex * ey + ey * ez + ez * ex;
@@ -923,11 +926,12 @@ __global__ void k_sah(const float *nodes, uint32_t num_nodes, double *acc) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     double v = 0.0;
     if (i < num_nodes) {
-        const float *nd = nodes + (size_t)i * 8 * K;
+        const float *rec = nodes + (size_t)i * 8 * K;
+        const auto nd = [&](int w) { return rec[w ^ ptd::node_swizzle<K>(i)]; };
         for (int c = 0; c < K; c++) {
-            const int item = __float_as_int(nd[6 * K + c]);
+            const int item = __float_as_int(nd(6 * K + c));
             if (item == ptd::kNoItem) continue;
-            float ex = nd[K + c] - nd[c], ey = nd[3 * K + c] - nd[2 * K + c], ez = nd[5 * K + c] - nd[4 * K + c];
+            float ex = nd(K + c) - nd(c), ey = nd(3 * K + c) - nd(2 * K + c), ez = nd(5 * K + c) - nd(4 * K + c);
             float a = ex * ey + ey * ez + ez * ex;
             const int cnt = item_count(item);
             v += (double)a * (cnt > 0 ? (double)kCostPrim * cnt : (double)kCostNode);
@@ -944,8 +948,9 @@ __global__ void k_refit_level(float *nodes, uint32_t first, uint32_t last, const
     uint32_t i = first + blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= last) return;
     float *nd = nodes + (size_t)i * 8 * K;
+    const uint32_t swz = ptd::node_swizzle<K>(i);
     for (int c = 0; c < K; c++) {
-        const int item = __float_as_int(nd[6 * K + c]);
+        const int item = __float_as_int(nd[(6 * K + c) ^ swz]);
         if (item == ptd::kNoItem) continue;
         const int cnt = item_count(item), ch = cnt > 0 ? ptd::leaf_first(item) : item;
         float4 lo = make_float4(FLT_MAX, FLT_MAX, FLT_MAX, 0.f), hi = make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, 0.f);
@@ -957,16 +962,17 @@ __global__ void k_refit_level(float *nodes, uint32_t first, uint32_t last, const
                 hi = make_float4(fmaxf(hi.x, b.x), fmaxf(hi.y, b.y), fmaxf(hi.z, b.z), 0.f);
             }
         } else {
-            const float *cn = nodes + (size_t)ch * 8 * K;
+            const float *rec = nodes + (size_t)ch * 8 * K;
+            const auto cn = [&](int w) { return rec[w ^ ptd::node_swizzle<K>(ch)]; };
             for (int g = 0; g < K; g++) {
-                if (__float_as_int(cn[6 * K + g]) == ptd::kNoItem) continue;
-                lo = make_float4(fminf(lo.x, cn[g]), fminf(lo.y, cn[2 * K + g]), fminf(lo.z, cn[4 * K + g]), 0.f);
-                hi = make_float4(fmaxf(hi.x, cn[K + g]), fmaxf(hi.y, cn[3 * K + g]), fmaxf(hi.z, cn[5 * K + g]), 0.f);
+                if (__float_as_int(cn(6 * K + g)) == ptd::kNoItem) continue;
+                lo = make_float4(fminf(lo.x, cn(g)), fminf(lo.y, cn(2 * K + g)), fminf(lo.z, cn(4 * K + g)), 0.f);
+                hi = make_float4(fmaxf(hi.x, cn(K + g)), fmaxf(hi.y, cn(3 * K + g)), fmaxf(hi.z, cn(5 * K + g)), 0.f);
             }
         }
         float3 plo, phi;
         padded(lo, hi, scene_mag, plo, phi);
-        write_slot<K>(nd, c, plo, phi, ch, cnt);
+        write_slot<K>(nd, swz, c, plo, phi, ch, cnt);
     }
 }
 

@@ -240,11 +240,6 @@ __global__ void k_advance(uint32_t *next) {
     if (threadIdx.x < kSetWords) next[threadIdx.x] = 0;
 }
 
-template <int K>
-PT_DI size_t smem_node_bytes(const DevScene &s) {
-    return (size_t)s.smem_nodes * 32 * K;
-}
-
 // Ray sources / result sinks of the persistent traversal.
 struct ExtendSrc {  // closest hit of the active queue
     State st;
@@ -318,8 +313,9 @@ struct UserSrc {  // pt_trace_rays
 };
 
 // Stages the top smem_nodes nodes in shared memory; returns the stack base.
-template <int K>
+template <int K, int FORM>
 PT_DI void *stage_smem(const DevScene &s, float4 *smem) {
+    if ((FORM & kStaged) == 0) return smem;
     for (uint32_t i = threadIdx.x; i < s.smem_nodes * 2 * K; i += blockDim.x) smem[i] = __ldg(s.nodes + i);
     __syncthreads();
     return smem + s.smem_nodes * 2 * K;
@@ -328,21 +324,21 @@ PT_DI void *stage_smem(const DevScene &s, float4 *smem) {
 // ANY = false: closest hit of the extension rays; ANY = true: shadow rays.
 // Widths 2 and 4 are capped at 72 registers (7 blocks of 128 threads per SM),
 // width 8 (compressed nodes) at 96.
-template <int K, bool ANY, bool COUNT, bool BATCH = false, bool CURVES = false>
+template <int K, bool ANY, bool COUNT, bool BATCH = false, int FORM = 0>
 __global__ void __maxnreg__(K == 8 ? 96 : 72) k_trace_queue(DevScene s, State st, Batch bt, uint32_t frames) {
     extern __shared__ float4 smem[];
-    void *sstack = stage_smem<K>(s, smem);
+    void *sstack = stage_smem<K, FORM>(s, smem);
     if (ANY) {
         if (BATCH) {
             BatchShadowSrc src;
             src.st = st;
             src.bt = bt;
             src.frames = frames;
-            trace_persistent<K, true, COUNT, decltype(src), CURVES>(s, smem, sstack, src, st.cur + kWorkShadow, st.counters + kOverflow,
+            trace_persistent<K, true, COUNT, decltype(src), FORM>(s, smem, sstack, src, st.cur + kWorkShadow, st.counters + kOverflow,
                                              st.stats + kStatShNodes, st.stats + kStatShPrims, st.stats + kStatShRays);
         } else {
             ShadowSrc src{st};
-            trace_persistent<K, true, COUNT, decltype(src), CURVES>(s, smem, sstack, src, st.cur + kWorkShadow, st.counters + kOverflow,
+            trace_persistent<K, true, COUNT, decltype(src), FORM>(s, smem, sstack, src, st.cur + kWorkShadow, st.counters + kOverflow,
                                              st.stats + kStatShNodes, st.stats + kStatShPrims, st.stats + kStatShRays);
         }
     } else {
@@ -351,14 +347,28 @@ __global__ void __maxnreg__(K == 8 ? 96 : 72) k_trace_queue(DevScene s, State st
             src.st = st;
             src.bt = bt;
             src.frames = frames;
-            trace_persistent<K, false, COUNT, decltype(src), CURVES>(s, smem, sstack, src, st.cur + kWorkExtend, st.counters + kOverflow,
+            trace_persistent<K, false, COUNT, decltype(src), FORM>(s, smem, sstack, src, st.cur + kWorkExtend, st.counters + kOverflow,
                                               st.stats + kStatExtNodes, st.stats + kStatExtPrims, st.stats + kStatExtRays);
         } else {
             ExtendSrc src{st};
-            trace_persistent<K, false, COUNT, decltype(src), CURVES>(s, smem, sstack, src, st.cur + kWorkExtend, st.counters + kOverflow,
+            trace_persistent<K, false, COUNT, decltype(src), FORM>(s, smem, sstack, src, st.cur + kWorkExtend, st.counters + kOverflow,
                                               st.stats + kStatExtNodes, st.stats + kStatExtPrims, st.stats + kStatExtRays);
         }
     }
+}
+
+template <int K>
+int trace_form(const DevScene &s, bool curves) {
+    return (curves ? kCurves : 0) | (K != 8 && s.smem_nodes ? kStaged : 0);
+}
+template <int K, bool ANY, bool COUNT, bool BATCH>
+auto queue_kernel(int form) {
+    if constexpr (K != 8 && !BATCH) {  // the others stage no nodes
+        if (form & kStaged)
+            return form & kCurves ? k_trace_queue<K, ANY, COUNT, BATCH, kCurves | kStaged>
+                                  : k_trace_queue<K, ANY, COUNT, BATCH, kStaged>;
+    }
+    return form & kCurves ? k_trace_queue<K, ANY, COUNT, BATCH, kCurves> : k_trace_queue<K, ANY, COUNT, BATCH>;
 }
 
 struct HitGeo {
@@ -818,12 +828,20 @@ __global__ void k_accumulate(State st, Wave w, Batch bt, uint32_t width, uint32_
 }
 
 // pt_trace_rays: rays (ox,oy,oz,tmin, dx,dy,dz,tmax) -> hits.
-template <int K, bool ANY, bool CURVES>
-__global__ void k_trace_rays(DevScene s, const float4 *rays, float4 *hits, uint32_t n, uint32_t *work, uint32_t *ovf_flag) {
+template <int K, bool ANY, int FORM>
+__global__ void __maxnreg__(K == 8 ? 96 : 72) k_trace_rays(DevScene s, const float4 *rays, float4 *hits, uint32_t n, uint32_t *work, uint32_t *ovf_flag) {
     extern __shared__ float4 smem[];
-    void *sstack = stage_smem<K>(s, smem);
+    void *sstack = stage_smem<K, FORM>(s, smem);
     UserSrc<ANY> src{rays, hits, n};
-    trace_persistent<K, ANY, false, UserSrc<ANY>, CURVES>(s, smem, sstack, src, work, ovf_flag, nullptr, nullptr, nullptr);
+    trace_persistent<K, ANY, false, UserSrc<ANY>, FORM>(s, smem, sstack, src, work, ovf_flag, nullptr, nullptr, nullptr);
+}
+template <int K, bool ANY>
+auto rays_kernel(int form) {
+    if constexpr (K != 8) {
+        if (form & kStaged)
+            return form & kCurves ? k_trace_rays<K, ANY, kCurves | kStaged> : k_trace_rays<K, ANY, kStaged>;
+    }
+    return form & kCurves ? k_trace_rays<K, ANY, kCurves> : k_trace_rays<K, ANY, 0>;
 }
 
 __global__ void k_bsdf_eval(const float *bsdf, const float *wo, const float *wi, float *f, float *pdf, uint32_t n) {
@@ -996,10 +1014,9 @@ struct Launcher {
         const int tb = p->block_size ? (int)p->block_size : (t.tuned_block ? (int)t.tuned_block : 128);
         const size_t smem = (size_t)d.smem_nodes * 32 * K + (size_t)kShortStack * stack_entry_bytes(false) * tb;
         const size_t smem_sh = (size_t)d.smem_nodes * 32 * K + (size_t)kShortStack * stack_entry_bytes(true) * tb;
-        auto k_ext = t.curves ? (count ? k_trace_queue<K, false, true, BATCH, true> : k_trace_queue<K, false, false, BATCH, true>)
-                              : (count ? k_trace_queue<K, false, true, BATCH> : k_trace_queue<K, false, false, BATCH>);
-        auto k_sh = t.curves ? (count ? k_trace_queue<K, true, true, BATCH, true> : k_trace_queue<K, true, false, BATCH, true>)
-                             : (count ? k_trace_queue<K, true, true, BATCH> : k_trace_queue<K, true, false, BATCH>);
+        const int form = trace_form<K>(d, t.curves);
+        const auto k_ext = count ? queue_kernel<K, false, true, BATCH>(form) : queue_kernel<K, false, false, BATCH>(form);
+        const auto k_sh = count ? queue_kernel<K, true, true, BATCH>(form) : queue_kernel<K, true, false, BATCH>(form);
         if ((e = set_smem(k_ext, smem)) != PT_OK || (e = set_smem(k_sh, smem_sh)) != PT_OK) return e;
         int occ_t = 0, occ_s = 0, occ_h = 0;
         PT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_t, k_ext, tb, smem));
@@ -1250,8 +1267,8 @@ struct Launcher {
         const int tb = 128;
         const size_t smem = (size_t)d.smem_nodes * 32 * K + (size_t)kShortStack * stack_entry_bytes(anyhit != 0) * tb;
         const bool curves = s->num_curve_pieces > 0;
-        auto kern = curves ? (anyhit ? k_trace_rays<K, true, true> : k_trace_rays<K, false, true>)
-                           : (anyhit ? k_trace_rays<K, true, false> : k_trace_rays<K, false, false>);
+        const int form = trace_form<K>(d, curves);
+        const auto kern = anyhit ? rays_kernel<K, true>(form) : rays_kernel<K, false>(form);
         if ((e = set_smem(kern, smem)) != PT_OK) return e;
         int occ = 0;
         PT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, tb, smem));
@@ -1271,19 +1288,20 @@ struct Launcher {
     }
 };
 
-// Merged-BVH child rebasing: inner children move by the scene's first node,
-// leaves by its first primitive slot.
+// A scene's nodes into the merged BVH, a word per thread: inner children move by
+// the scene's first node, leaves by its first primitive slot, and the swizzle
+// follows the new index.
 template <int K>
-__global__ void k_rebase_nodes(float4 *nodes, uint32_t num_nodes, int node_off, int prim_off) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < num_nodes; i += gridDim.x * blockDim.x) {
-        float *f = reinterpret_cast<float *>(nodes + (size_t)i * 2 * K);
-#pragma unroll
-        for (int c = 0; c < K; c++) {
-            const int item = __float_as_int(f[6 * K + c]);
-            if (item == ptd::kNoItem) continue;
-            f[6 * K + c] = __int_as_float(is_leaf(item) ? make_leaf(leaf_first(item) + prim_off, leaf_count(item))
-                                                        : item + node_off);
-        }
+__global__ void k_merge_nodes(const float *src, uint32_t num_nodes, float *dst, uint32_t node_off, int prim_off) {
+    const size_t n = (size_t)num_nodes * 8 * K;
+    for (size_t j = blockIdx.x * (size_t)blockDim.x + threadIdx.x; j < n; j += (size_t)gridDim.x * blockDim.x) {
+        const uint32_t i = (uint32_t)(j / (8 * K)), w = (uint32_t)(j % (8 * K)) ^ node_swizzle<K>(i);
+        float v = src[j];
+        const int item = __float_as_int(v);
+        if (w >= 6 * K && w < 7 * K && item != ptd::kNoItem)
+            v = __int_as_float(is_leaf(item) ? make_leaf(leaf_first(item) + prim_off, leaf_count(item))
+                                             : item + (int)node_off);
+        dst[(size_t)(node_off + i) * 8 * K + (w ^ node_swizzle<K>(node_off + i))] = v;
     }
 }
 
@@ -1367,12 +1385,11 @@ int render_batch(pt_context *ctx, pt_scene *const *scenes, const pt_render_param
     uint64_t node_off = 0, prim_off = 0;
     for (uint32_t k = 0; k < n; k++) {
         const pt_scene *s = scenes[k];
-        float4 *dn = b.nodes.as<float4>() + node_off * 2 * K;
-        PT_CUDA_TRY(cudaMemcpyAsync(dn, s->dev.nodes, (size_t)s->dev.num_nodes * 32 * K, cudaMemcpyDeviceToDevice, st));
         PT_CUDA_TRY(cudaMemcpyAsync(b.prims.as<float4>() + prim_off * 3, s->dev.prims, (size_t)s->num_prims * 48,
                                     cudaMemcpyDeviceToDevice, st));
-        k_rebase_nodes<K><<<nblocks(s->dev.num_nodes, 256), 256, 0, st>>>(dn, s->dev.num_nodes, (int)node_off,
-                                                                          (int)prim_off);
+        k_merge_nodes<K><<<nblocks((size_t)s->dev.num_nodes * 8 * K, 256), 256, 0, st>>>(
+            reinterpret_cast<const float *>(s->dev.nodes), s->dev.num_nodes, b.nodes.as<float>(), (uint32_t)node_off,
+            (int)prim_off);
         PT_CUDA_TRY(cudaGetLastError());
         node_off += s->dev.num_nodes;
         prim_off += s->num_prims;
@@ -1650,8 +1667,8 @@ int render_noalloc(pt_scene *s, const pt_render_params *p, const pt_frame_buffer
     const size_t smem = (size_t)d.smem_nodes * 32 * K + (size_t)kShortStack * stack_entry_bytes(false) * tb;
     const size_t smem_sh = (size_t)d.smem_nodes * 32 * K + (size_t)kShortStack * stack_entry_bytes(true) * tb;
     const bool curves = s->num_curve_pieces > 0;
-    auto k_ext = curves ? k_trace_queue<K, false, false, false, true> : k_trace_queue<K, false, false>;
-    auto k_sh = curves ? k_trace_queue<K, true, false, false, true> : k_trace_queue<K, true, false>;
+    const int form = trace_form<K>(d, curves);
+    const auto k_ext = queue_kernel<K, false, false, false>(form), k_sh = queue_kernel<K, true, false, false>(form);
     int e;
     if ((e = set_smem(k_ext, smem)) != PT_OK || (e = set_smem(k_sh, smem_sh)) != PT_OK) return e;
     int occ_t = 0, occ_s = 0, occ_h = 0;

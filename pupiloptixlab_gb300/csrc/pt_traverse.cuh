@@ -240,15 +240,26 @@ PT_DI float3 safe_inv(float3 d) {
               d.z != 0.f ? __frcp_rn(d.z) : copysignf(1e30f, d.z));
 }
 
+// Word w of node i is stored at word w ^ node_swizzle<K>(i) of its record.  The
+// lanes of a warp read the same words of different nodes at a time; unswizzled
+// these lie in the same banks of L1, one lane per cycle.  112-byte gathers of a
+// 128-byte node by 16 lanes of a warp: 1.82 ms unswizzled, 0.97 swizzled while the
+// nodes are in L1; 2.21 and 1.82 when they come from L2.  The 1M-triangle field at
+// 1080p, 64 spp: closest / any hit 86.8 / 25.2 ms, so 80.0 / 22.1.  Width 4 moves
+// 16-byte pieces, width 2 32-byte halves; 8-wide nodes are read as 96-byte copies,
+// which fall on different banks by themselves.
+template <int K>
+PT_HDI constexpr uint32_t node_swizzle(uint32_t i) {
+    return K == 4 ? (i & 7) << 2 : K == 2 ? (i & 2) << 2 : 0;
+}
+
+// A node as a ray sees it.  Widths 2 and 8: low and high planes, then items.
+// Width 4: near and far planes by the ray's octant.
 template <int K>
 struct WideNode {
     float f[8 * K];
-    PT_DI float lox(int c) const { return f[c]; }
-    PT_DI float hix(int c) const { return f[K + c]; }
-    PT_DI float loy(int c) const { return f[2 * K + c]; }
-    PT_DI float hiy(int c) const { return f[3 * K + c]; }
-    PT_DI float loz(int c) const { return f[4 * K + c]; }
-    PT_DI float hiz(int c) const { return f[5 * K + c]; }
+    PT_DI float p0(int axis, int c) const { return f[2 * axis * K + c]; }
+    PT_DI float p1(int axis, int c) const { return f[(2 * axis + 1) * K + c]; }
     PT_DI int item(int c) const { return __float_as_int(f[6 * K + c]); }
 };
 
@@ -301,34 +312,38 @@ PT_DI void st_stream(T *p, T v) {
     __stcs(p, v);
 }
 
-// The 7*K floats in use: width 4 three 256-bit loads and one of 128 bits.
-template <int K>
-PT_DI void load_node(const float4 *__restrict__ p, WideNode<K> &n) {
-#pragma unroll
-    for (int i = 0; i < 7 * K / 8; i++) ld_bvh8(p + 2 * i, n.f + 8 * i);
-    if (7 * K % 8) {
-        const float4 v = ld_bvh(p + 7 * K / 8 * 2);
-        float *f = n.f + 7 * K / 8 * 8;
-        f[0] = v.x;
-        f[1] = v.y;
-        f[2] = v.z;
-        f[3] = v.w;
-        if (7 * K % 8 > 4) {  // width 2: floats 12, 13
-            const float4 u = ld_bvh(p + 7 * K / 8 * 2 + 1);
-            f[4] = u.x;
-            f[5] = u.y;
-        }
-    }
-}
-template <int K>
-PT_DI void load_node_smem(const float4 *p, WideNode<K> &n) {
-#pragma unroll
-    for (int i = 0; i < 2 * K; i++) {
-        float4 v = p[i];
+// The 7*K floats in use, from global (GLOBAL) or shared memory.  Width 4 loads 16
+// bytes at a time and picks each axis's near and far planes by address, which
+// takes 24 minima and maxima out of the slab test: 1.5 to 3 % of the small frames'
+// time against 32-byte loads and min / max (which ask less of L1: equal at 64 spp).
+template <int K, bool GLOBAL>
+PT_DI void load_node(const float4 *__restrict__ nodes, int item, int oct, WideNode<K> &n) {
+    const uint32_t swz = 4 * node_swizzle<K>(item);  // in bytes; the array in global memory is aligned to a record
+    const float4 *rec = nodes + (size_t)item * 2 * K;
+    const uintptr_t p = reinterpret_cast<uintptr_t>(rec) | swz;
+    const auto load4 = [&](int i, uint32_t at) {
+        const float4 v = GLOBAL ? ld_bvh(reinterpret_cast<const float4 *>(p ^ at)) : rec[(at ^ swz) / 16];
         n.f[4 * i + 0] = v.x;
         n.f[4 * i + 1] = v.y;
         n.f[4 * i + 2] = v.z;
         n.f[4 * i + 3] = v.w;
+    };
+    if constexpr (K == 4) {
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            const uint32_t side = (oct << (4 - a)) & 16;
+            load4(2 * a, (32 * a) | side);
+            load4(2 * a + 1, ((32 * a) | side) ^ 16);
+        }
+        load4(6, 96);
+    } else if constexpr (GLOBAL) {
+        static_assert(K == 2, "8-wide nodes are read compressed");
+        ld_bvh8(reinterpret_cast<const float4 *>(p), n.f);
+        load4(2, 32);
+        load4(3, 48);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 2 * K; i++) load4(i, 16 * i);
     }
 }
 
@@ -503,10 +518,12 @@ constexpr int kNodeWaitMax = 8;
 // Src provides: count(), load(i, o, d, tmin, tmax, tag), root(tag) (the node
 // the ray starts at), store(i, tag, result).  A load that leaves tmin and tmax
 // alone (extension rays: always 0.001 and 1e16) keeps them out of registers.
-// CURVES = false compiles the leaf test without the curve-piece branch (a
-// record with non-zero kind bits is then treated as a sphere), so that scenes
-// without curves run the smaller kernel.
-template <int K, bool ANY, bool COUNT, class Src, bool CURVES = false>
+// FORM: without kCurves the leaf test has no curve-piece branch (a record with
+// non-zero kind bits is then treated as a sphere), so that scenes without curves
+// run the smaller kernel; without kStaged every node comes from global memory (the
+// test for a staged one costs 1 to 5 %: 1M rays 772 -> 737 us).
+enum TraceForm : int { kCurves = 1, kStaged = 2 };
+template <int K, bool ANY, bool COUNT, class Src, int FORM = 0>
 PT_DI void trace_persistent(const DevScene &s, const float4 *snodes, void *sstack_base, Src &src, uint32_t *work,
                             uint32_t *ovf_flag, unsigned long long *stat_nodes, unsigned long long *stat_prims,
                             unsigned long long *stat_rays) {
@@ -522,7 +539,7 @@ PT_DI void trace_persistent(const DevScene &s, const float4 *snodes, void *sstac
     uint32_t idx = 0, tag = 0;
     float3 o = f3s(0.f), d = f3s(0.f), inv = f3s(0.f), oi = f3s(0.f);
     bool fma_slab = false;
-    int oct = 0;  // direction octant (compressed 8-wide nodes)
+    int oct = 0;  // direction octant: signs of inv
     RayWT w{0, 1, 2, 0.f, 0.f, 1.f};
     float tmin = 0.001f, tmax = 1e16f;  // the extension rays' range (main.cu:80-85)
     TraceResult best{0.f, -1, 0.f, 0.f};
@@ -550,7 +567,8 @@ PT_DI void trace_persistent(const DevScene &s, const float4 *snodes, void *sstac
                     // the FMA slab form is conservative for origins inside the
                     // magnitude the boxes were padded for
                     fma_slab = fmaxf(fmaxf(fabsf(o.x), fabsf(o.y)), fabsf(o.z)) <= s.pad_mag;
-                    oct = (d.x < 0.f ? 1 : 0) | (d.y < 0.f ? 2 : 0) | (d.z < 0.f ? 4 : 0);
+                    oct = (__float_as_uint(inv.x) >> 31) | (__float_as_uint(inv.y) >> 31) << 1 |
+                          (__float_as_uint(inv.z) >> 31) << 2;
                     best.t = tmax;
                     best.prim = -1;
                     best.u = best.v = 0.f;
@@ -597,8 +615,8 @@ PT_DI void trace_persistent(const DevScene &s, const float4 *snodes, void *sstac
                 item = next != kNoItem ? next : pop_valid();
             } else {
                 WideNode<K> nd;
-                if (item < static_cast<int>(s.smem_nodes)) load_node_smem<K>(snodes + (size_t)item * 2 * K, nd);
-                else load_node<K>(s.nodes + (size_t)item * 2 * K, nd);
+                if ((FORM & kStaged) != 0 && item < static_cast<int>(s.smem_nodes)) load_node<K, false>(snodes, item, oct, nd);
+                else load_node<K, true>(s.nodes, item, oct, nd);
                 if (COUNT) nodes++;
                 int ci[K];
                 float ct[K];
@@ -609,22 +627,24 @@ PT_DI void trace_persistent(const DevScene &s, const float4 *snodes, void *sstac
                     ct[c] = __int_as_float(0x7f800000);
                     float tx0, tx1, ty0, ty1, tz0, tz1;
                     if (fma_slab) {  // t = lo * inv - o * inv: one rounding, conservative within pad_mag
-                        tx0 = __fmaf_rn(nd.lox(c), inv.x, -oi.x);
-                        tx1 = __fmaf_rn(nd.hix(c), inv.x, -oi.x);
-                        ty0 = __fmaf_rn(nd.loy(c), inv.y, -oi.y);
-                        ty1 = __fmaf_rn(nd.hiy(c), inv.y, -oi.y);
-                        tz0 = __fmaf_rn(nd.loz(c), inv.z, -oi.z);
-                        tz1 = __fmaf_rn(nd.hiz(c), inv.z, -oi.z);
+                        tx0 = __fmaf_rn(nd.p0(0, c), inv.x, -oi.x);
+                        tx1 = __fmaf_rn(nd.p1(0, c), inv.x, -oi.x);
+                        ty0 = __fmaf_rn(nd.p0(1, c), inv.y, -oi.y);
+                        ty1 = __fmaf_rn(nd.p1(1, c), inv.y, -oi.y);
+                        tz0 = __fmaf_rn(nd.p0(2, c), inv.z, -oi.z);
+                        tz1 = __fmaf_rn(nd.p1(2, c), inv.z, -oi.z);
                     } else {
-                        tx0 = (nd.lox(c) - o.x) * inv.x;
-                        tx1 = (nd.hix(c) - o.x) * inv.x;
-                        ty0 = (nd.loy(c) - o.y) * inv.y;
-                        ty1 = (nd.hiy(c) - o.y) * inv.y;
-                        tz0 = (nd.loz(c) - o.z) * inv.z;
-                        tz1 = (nd.hiz(c) - o.z) * inv.z;
+                        tx0 = (nd.p0(0, c) - o.x) * inv.x;
+                        tx1 = (nd.p1(0, c) - o.x) * inv.x;
+                        ty0 = (nd.p0(1, c) - o.y) * inv.y;
+                        ty1 = (nd.p1(1, c) - o.y) * inv.y;
+                        tz0 = (nd.p0(2, c) - o.z) * inv.z;
+                        tz1 = (nd.p1(2, c) - o.z) * inv.z;
                     }
-                    float tn = fmaxf(fmaxf(fminf(tx0, tx1), fminf(ty0, ty1)), fmaxf(fminf(tz0, tz1), tmin));
-                    float tf = fminf(fminf(fmaxf(tx0, tx1), fmaxf(ty0, ty1)), fmaxf(tz0, tz1));
+                    const auto lower = [](float a, float b) { return K == 4 ? a : fminf(a, b); };
+                    const auto upper = [](float a, float b) { return K == 4 ? b : fmaxf(a, b); };
+                    float tn = fmaxf(fmaxf(lower(tx0, tx1), lower(ty0, ty1)), fmaxf(lower(tz0, tz1), tmin));
+                    float tf = fminf(fminf(upper(tx0, tx1), upper(ty0, ty1)), upper(tz0, tz1));
                     tf = fminf(tf * kSlabScale, tlimit);
                     if (!(tn <= tf)) continue;
                     ci[c] = nd.item(c);  // an empty slot's stays kNoItem whatever its box says
@@ -689,7 +709,7 @@ PT_DI void trace_persistent(const DevScene &s, const float4 *snodes, void *sstac
                     if (pid >= 0) {
                         float4 cc = ld_bvh(pr + 2);
                         hit = intersect_triangle(o, w, xyz(a), xyz(b), xyz(cc), tmin, tlim, t, u, v);
-                    } else if (!CURVES || __float_as_int(b.w) == 0) {
+                    } else if ((FORM & kCurves) == 0 || __float_as_int(b.w) == 0) {
                         pid &= 0x7fffffff;
                         hit = intersect_sphere(o, d, xyz(a), b.x, tmin, tlim, t);
                     } else {
