@@ -49,7 +49,7 @@ enum Counter : int {
 constexpr uint32_t kFixedSets = 24, kSetWords = 8;  // three sets taken in turn, then
 constexpr uint32_t kCallWord = 48;                  // the call's arguments (CallBlock), then
 constexpr uint32_t kFirstSet = 64;                  // a set per bounce
-enum SetCounter : int { kNIn = 0, kNShadow, kWorkExtend, kWorkShadow };
+enum SetCounter : int { kNIn = 0, kNShadow, kWorkExtend, kWorkShadow, kBinBlocks };
 enum Stat : int { kStatExtNodes = 0, kStatExtPrims, kStatShNodes, kStatShPrims, kStatExtRays, kStatShRays, kNumStats };
 
 struct Wave {
@@ -158,35 +158,33 @@ PT_DI Sampler load_rng(float lo, float hi, uint32_t mode, uint32_t frame_seed) {
     return s;
 }
 
-// Block-aggregated append to two queues: warp ballots give the lane offsets,
-// thread 0 does one atomicAdd per queue for the whole block.  sh: 66 words of
-// shared memory.  Every thread of the block must call it.
-PT_DI void block_push2(bool p0, bool p1, uint32_t *c0, uint32_t *c1, uint32_t &pos0, uint32_t &pos1, uint32_t *sh) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    uint32_t b0 = __ballot_sync(0xffffffffu, p0), b1 = __ballot_sync(0xffffffffu, p1);
-    uint32_t *wc0 = sh, *wc1 = sh + 32, *base = sh + 64;
-    if (lane == 0) {
-        wc0[warp] = __popc(b0);
-        wc1[warp] = __popc(b1);
+// Block-aggregated append to two queues by a block of 256: warp ballots give the
+// lane offsets, each thread sums the warps' counts, two threads do one atomicAdd
+// each for the whole block.  Every thread of the block must call it, in turn with
+// either of two buffers, which saves a barrier (shading a 1-spp 1080p frame of the
+// 1M-triangle field 0.497 -> 0.483 ms, the Cornell box at 16 spp 0.234 -> 0.228).
+struct PushSmem {
+    uint32_t warp[8];  // counts of the two queues, 16 bits each
+    uint32_t base[2];
+};
+PT_DI void block_push2(bool p0, bool p1, uint32_t *c0, uint32_t *c1, uint32_t &pos0, uint32_t &pos1, PushSmem &sh) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t b0 = __ballot_sync(0xffffffffu, p0), b1 = __ballot_sync(0xffffffffu, p1);
+    if (lane == 0) sh.warp[warp] = __popc(b0) | __popc(b1) << 16;
+    __syncthreads();
+    uint32_t before = 0, all = 0;
+#pragma unroll
+    for (int w = 0; w < 8; w++) {
+        const uint32_t c = sh.warp[w];
+        if (w < warp) before += c;
+        all += c;
     }
+    if (threadIdx.x == 0) sh.base[0] = (all & 0xffffu) ? atomicAdd(c0, all & 0xffffu) : 0;
+    if (threadIdx.x == 32) sh.base[1] = (all >> 16) ? atomicAdd(c1, all >> 16) : 0;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t s0 = 0, s1 = 0;
-        for (int w = 0; w < nw; w++) {
-            uint32_t a = wc0[w], b = wc1[w];
-            wc0[w] = s0;
-            wc1[w] = s1;
-            s0 += a;
-            s1 += b;
-        }
-        base[0] = s0 ? atomicAdd(c0, s0) : 0;
-        base[1] = s1 ? atomicAdd(c1, s1) : 0;
-    }
-    __syncthreads();
-    uint32_t lt = (1u << lane) - 1u;
-    pos0 = base[0] + wc0[warp] + __popc(b0 & lt);
-    pos1 = base[1] + wc1[warp] + __popc(b1 & lt);
-    __syncthreads();
+    const uint32_t lt = (1u << lane) - 1u;
+    pos0 = sh.base[0] + (before & 0xffffu) + __popc(b0 & lt);
+    pos1 = sh.base[1] + (before >> 16) + __popc(b1 & lt);
 }
 
 // Camera ray, example/path_tracer/main.cu:58-78.
@@ -568,7 +566,8 @@ PT_DI void shade_one(const DevScene &s, const Outputs &out, const State &st, con
 // 32.7 ms with a path's ray, stream and flags in separate 4- to 16-byte arrays.
 template <bool BATCH>
 __global__ void __launch_bounds__(256, 4) k_shade(DevScene s, Batch bt, State st, Wave w) {
-    __shared__ uint32_t push_smem[72];
+    __shared__ PushSmem push_smem[2];
+    int turn = 0;
     const uint32_t n = st.cur[kNIn];
     const float env_pdf = 0.25f * kInvPi;  // ConstEnvEmitter::Eval (env.h:82-85)
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
@@ -588,7 +587,7 @@ __global__ void __launch_bounds__(256, 4) k_shade(DevScene s, Batch bt, State st
             }
         }
         uint32_t pos_ext, pos_sh;
-        block_push2(so.push_ext, so.push_sh, st.next + kNIn, st.cur + kNShadow, pos_ext, pos_sh, push_smem);
+        block_push2(so.push_ext, so.push_sh, st.next + kNIn, st.cur + kNShadow, pos_ext, pos_sh, push_smem[turn ^= 1]);
         if (so.push_ext) st.q_out[pos_ext] = slot | (so.delta ? kEntryDelta : 0u);
         if (so.push_sh) {  // shadow ray from the hit point, tmin 1e-4, tmax distance - 1e-4 (main.cu:122-126)
             st.sh_o[pos_sh] = make_float4(so.hit_pos.x, so.hit_pos.y, so.hit_pos.z, 0.0001f);
@@ -611,9 +610,13 @@ PT_DI uint32_t material_bin(const DevScene &s, int prim) {
 // Material binning is a stable counting sort over the bins: block b takes
 // the contiguous stretch [b * chunk, (b + 1) * chunk) of the queue, so that
 // each bin keeps the queue's order (neighbouring path slots, i.e. the
-// samples of a pixel and its neighbours, stay neighbours inside a bin).  k_bin_count writes
-// every block's per-bin counts, k_bin_scan turns them into each block's first
-// position in every bin, k_bin_scatter places the entries.
+// samples of a pixel and its neighbours, stay neighbours inside a bin).  k_bin_count
+// writes every block's per-bin counts, bin by bin, and its last block to finish
+// turns them into each block's first position in every bin; k_bin_scatter places
+// the entries.  (The prefix as a kernel of one warp per bin took 12 to 15 us a
+// bounce of a 1080p frame, here about 3.)  Binning a block's chunk on its own needs
+// no prefix, but then every BSDF's code runs on every SM at once: shading 48.9 ms
+// against 22.7 in 64 spp of the 1M-triangle field.
 __device__ __forceinline__ void bin_stretch(uint32_t n, uint32_t &lo, uint32_t &hi) {
     const uint32_t per = (n + gridDim.x - 1) / gridDim.x;
     const uint32_t chunk = (per + blockDim.x - 1) / blockDim.x * blockDim.x;
@@ -621,8 +624,9 @@ __device__ __forceinline__ void bin_stretch(uint32_t n, uint32_t &lo, uint32_t &
     hi = min(n, lo + chunk);
 }
 
-__global__ void k_bin_count(DevScene s, State st, uint8_t *keys, uint32_t *block_bins) {
-    __shared__ uint32_t h[kNumBins];
+__global__ void __launch_bounds__(256) k_bin_count(DevScene s, State st, uint8_t *keys, uint32_t *block_bins) {
+    __shared__ uint32_t h[kNumBins], warp_sum[8];
+    __shared__ bool last;
     if (threadIdx.x < kNumBins) h[threadIdx.x] = 0;
     __syncthreads();
     uint32_t lo, hi;
@@ -635,34 +639,43 @@ __global__ void k_bin_count(DevScene s, State st, uint8_t *keys, uint32_t *block
         atomicAdd(&h[key], 1u);
     }
     __syncthreads();
-    if (threadIdx.x < kNumBins) block_bins[blockIdx.x * kNumBins + threadIdx.x] = h[threadIdx.x];
-}
-
-// One warp per bin (blockDim = 32 * kNumBins): the bin's total over the
-// blocks, the bins' starts, then each block's start in the bin (in place).
-__global__ void k_bin_scan(uint32_t *block_bins, uint32_t nblocks) {
-    __shared__ uint32_t total[kNumBins];
-    const unsigned FULL = 0xffffffffu;
-    const uint32_t bin = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint32_t t = 0;
-    for (uint32_t b = lane; b < nblocks; b += 32) t += block_bins[b * kNumBins + bin];
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(FULL, t, o);
-    if (lane == 0) total[bin] = t;
+    if (threadIdx.x < kNumBins) {
+        block_bins[threadIdx.x * gridDim.x + blockIdx.x] = h[threadIdx.x];
+        __threadfence();
+    }
     __syncthreads();
-    uint32_t carry = 0;
-    for (uint32_t k = 0; k < bin; k++) carry += total[k];
-    for (uint32_t b0 = 0; b0 < nblocks; b0 += 32) {
-        const uint32_t b = b0 + lane;
-        const uint32_t v = b < nblocks ? block_bins[b * kNumBins + bin] : 0u;
-        uint32_t x = v;
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(FULL, x, o);
-            if (lane >= (uint32_t)o) x += y;
-        }
-        if (b < nblocks) block_bins[b * kNumBins + bin] = carry + x - v;
-        carry += __shfl_sync(FULL, x, 31);
+    if (threadIdx.x == 0) last = atomicAdd(st.cur + kBinBlocks, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    // exclusive prefix over bins, then blocks: a run of words per thread
+    __threadfence();
+    const uint32_t total = kNumBins * gridDim.x, per = (total + 1023) / 1024 * 4;
+    const uint32_t from = min(total, threadIdx.x * per), to = min(total, from + per);
+    uint4 *words = reinterpret_cast<uint4 *>(block_bins);
+    uint32_t sum = 0;
+#pragma unroll 4
+    for (uint32_t k = from / 4; k < to / 4; k++) {
+        const uint4 v = __ldcg(words + k);
+        sum += v.x + v.y + v.z + v.w;
+    }
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t x = sum;
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= (uint32_t)o) x += y;
+    }
+    if (lane == 31) warp_sum[warp] = x;
+    __syncthreads();
+    x -= sum;
+    for (uint32_t k = 0; k < warp; k++) x += warp_sum[k];
+#pragma unroll 4
+    for (uint32_t k = from / 4; k < to / 4; k++) {
+        const uint4 v = __ldcg(words + k);
+        words[k] = make_uint4(x, x + v.x, x + v.x + v.y, x + v.x + v.y + v.z);
+        x += v.x + v.y + v.z + v.w;
     }
 }
+static_assert(kNumBins % 4 == 0, "k_bin_count reads the counts four at a time");
 
 // Per stretch of blockDim entries: each warp's count per key, a prefix over
 // the warps per key, then every entry at its block's running position in
@@ -673,7 +686,7 @@ __global__ void k_bin_scatter(State st, const uint8_t *keys, const uint32_t *blo
     __shared__ uint32_t run[kNumBins];
     const unsigned FULL = 0xffffffffu;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x < kNumBins) run[threadIdx.x] = block_bins[blockIdx.x * kNumBins + threadIdx.x];
+    if (threadIdx.x < kNumBins) run[threadIdx.x] = block_bins[threadIdx.x * gridDim.x + blockIdx.x];
     if (threadIdx.x < kWarps * kNumBins) wc[threadIdx.x / kNumBins][threadIdx.x % kNumBins] = 0;
     __syncthreads();
     uint32_t lo, hi;
@@ -1093,7 +1106,7 @@ struct Launcher {
         for (uint32_t f0 = 0; f0 < p->spp && enq == cudaSuccess; f0 += frames_per_wave) {
             if (replay) {  // counted as captured
                 const uint32_t full = bounces ? bounces - 1 : 0;
-                launches += 2 + 2 * bounces + full * (sort ? 4 : 1);
+                launches += 2 + 2 * bounces + full * (!sort ? 1 : BATCH ? 4 : 3);
                 waves++;
                 continue;
             }
@@ -1144,11 +1157,10 @@ struct Launcher {
                     } else {
                         uint8_t *keys = reinterpret_cast<uint8_t *>(bin_keys);
                         k_bin_count<<<grid_bin, 256, 0, ls>>>(d, stt, keys, bin_blocks);
-                        k_bin_scan<<<1, 32 * kNumBins, 0, ls>>>(bin_blocks, grid_bin);
                         k_bin_scatter<<<grid_bin, 256, 0, ls>>>(stt, keys, bin_blocks, q_sorted);
                     }
                     shade_st.q_in = q_sorted;
-                    launches += 3;
+                    launches += BATCH ? 3 : 2;
                 }
                 // the previous bounce's shadow rays add to the radiance and read the shadow queue
                 if (b > 0) order(ss, ls, ws.ev_shadow);
