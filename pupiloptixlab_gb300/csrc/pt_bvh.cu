@@ -57,9 +57,8 @@ __device__ __forceinline__ float ord2f(uint32_t u) {
 }
 
 __device__ __forceinline__ void prim_box(const float4 *prims, uint32_t p, float3 &lo, float3 &hi) {
-    float4 a = prims[3 * (size_t)p], b = prims[3 * (size_t)p + 1];
+    const float4 a = prims[3 * (size_t)p], b = prims[3 * (size_t)p + 1], c = prims[3 * (size_t)p + 2];
     if (__float_as_int(a.w) >= 0) {
-        float4 c = prims[3 * (size_t)p + 2];
         lo = f3(fminf(a.x, fminf(b.x, c.x)), fminf(a.y, fminf(b.y, c.y)), fminf(a.z, fminf(b.z, c.z)));
         hi = f3(fmaxf(a.x, fmaxf(b.x, c.x)), fmaxf(a.y, fmaxf(b.y, c.y)), fmaxf(a.z, fmaxf(b.z, c.z)));
     } else if (__float_as_int(b.w) == 0) {  // sphere
@@ -67,7 +66,6 @@ __device__ __forceinline__ void prim_box(const float4 *prims, uint32_t p, float3
         lo = f3(a.x - r, a.y - r, a.z - r);
         hi = f3(a.x + r, a.y + r, a.z + r);
     } else {  // round-cone curve piece: the boxes of its two end spheres
-        float4 c = prims[3 * (size_t)p + 2];
         float r0 = b.x, r1 = b.y;
         lo = f3(fminf(a.x - r0, c.x - r1), fminf(a.y - r0, c.y - r1), fminf(a.z - r0, c.z - r1));
         hi = f3(fmaxf(a.x + r0, c.x + r1), fmaxf(a.y + r0, c.y + r1), fmaxf(a.z + r0, c.z + r1));
@@ -735,16 +733,6 @@ __device__ __forceinline__ void padded(float4 lo, float4 hi, float scene_mag, fl
     phi = f3(hi.x + pad, hi.y + pad, hi.z + pad);
 }
 
-template <int K>
-__device__ __forceinline__ void write_slot(float *node, uint32_t swz, int c, float3 lo, float3 hi, int child, int count) {
-    node[c ^ swz] = lo.x;
-    node[(K + c) ^ swz] = hi.x;
-    node[(2 * K + c) ^ swz] = lo.y;
-    node[(3 * K + c) ^ swz] = hi.y;
-    node[(4 * K + c) ^ swz] = lo.z;
-    node[(5 * K + c) ^ swz] = hi.z;
-    node[(6 * K + c) ^ swz] = __int_as_float(count > 0 ? ptd::make_leaf(child, count) : child);
-}
 __device__ __forceinline__ int item_count(int item) { return ptd::is_leaf(item) ? ptd::leaf_count(item) : 0; }
 // The primitives of leaf x (at most 15), depth first, from position `first` on.
 __device__ __forceinline__ void leaf_positions(const Tree &t, int x, int first, const uint32_t *order,
@@ -920,60 +908,113 @@ __global__ void k_gather_prims(const float4 *src, const uint32_t *order, uint32_
     dst[3 * (size_t)k + j] = src[3 * (size_t)order[k] + j];
 }
 
-// SAH cost of the wide tree: sum over slots of area * (node or primitive cost).
+// Refit of the nodes [first, last), K lanes a node, one a slot: leaf slots from
+// the primitives, inner slots from the union of the child node's slots (deeper
+// levels are refit first).  Returns the slots' SAH cost; plo, phi: this lane's box.
 template <int K>
-__global__ void k_sah(const float *nodes, uint32_t num_nodes, double *acc) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    double v = 0.0;
-    if (i < num_nodes) {
-        const float *rec = nodes + (size_t)i * 8 * K;
-        const auto nd = [&](int w) { return rec[w ^ ptd::node_swizzle<K>(i)]; };
-        for (int c = 0; c < K; c++) {
-            const int item = __float_as_int(nd(6 * K + c));
-            if (item == ptd::kNoItem) continue;
-            float ex = nd(K + c) - nd(c), ey = nd(3 * K + c) - nd(2 * K + c), ez = nd(5 * K + c) - nd(4 * K + c);
-            float a = ex * ey + ey * ez + ez * ex;
-            const int cnt = item_count(item);
-            v += (double)a * (cnt > 0 ? (double)kCostPrim * cnt : (double)kCostNode);
+__device__ __forceinline__ double refit_node(float *nodes, uint32_t i, uint32_t c, const float4 *prims_bvh,
+                                             float scene_mag, float3 &plo, float3 &phi) {
+    float *node = nodes + (size_t)i * 8 * K;
+    const uint32_t swz = ptd::node_swizzle<K>(i);
+    const int item = __float_as_int(node[(6 * K + c) ^ swz]);
+    plo = f3(FLT_MAX, FLT_MAX, FLT_MAX);
+    phi = f3(-FLT_MAX, -FLT_MAX, -FLT_MAX);
+    if (item == ptd::kNoItem) return 0.0;
+    const int cnt = item_count(item);
+    float4 lo = make_float4(FLT_MAX, FLT_MAX, FLT_MAX, 0.f), hi = make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, 0.f);
+    if (cnt > 0) {
+        const int at = ptd::leaf_first(item);
+        for (int j = 0; j < cnt; j += 2) {  // two at a time (the last alone: twice)
+            float3 a, b, a2, b2;
+            prim_box(prims_bvh, (uint32_t)(at + j), a, b);
+            prim_box(prims_bvh, (uint32_t)(at + min(j + 1, cnt - 1)), a2, b2);
+            lo = make_float4(fminf(lo.x, fminf(a.x, a2.x)), fminf(lo.y, fminf(a.y, a2.y)),
+                             fminf(lo.z, fminf(a.z, a2.z)), 0.f);
+            hi = make_float4(fmaxf(hi.x, fmaxf(b.x, b2.x)), fmaxf(hi.y, fmaxf(b.y, b2.y)),
+                             fmaxf(hi.z, fmaxf(b.z, b2.z)), 0.f);
+        }
+    } else {
+        const float4 *rec = reinterpret_cast<const float4 *>(nodes) + (size_t)item * 2 * K;
+        float f[8 * K];
+#pragma unroll
+        for (int q = 0; q < (7 * K + 3) / 4; q++) {
+            const float4 v = rec[q ^ (ptd::node_swizzle<K>(item) / 4)];
+            f[4 * q] = v.x;
+            f[4 * q + 1] = v.y;
+            f[4 * q + 2] = v.z;
+            f[4 * q + 3] = v.w;
+        }
+#pragma unroll
+        for (int g = 0; g < K; g++) {
+            if (__float_as_int(f[6 * K + g]) == ptd::kNoItem) continue;
+            lo = make_float4(fminf(lo.x, f[g]), fminf(lo.y, f[2 * K + g]), fminf(lo.z, f[4 * K + g]), 0.f);
+            hi = make_float4(fmaxf(hi.x, f[K + g]), fmaxf(hi.y, f[3 * K + g]), fmaxf(hi.z, f[5 * K + g]), 0.f);
         }
     }
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(acc, v);
+    padded(lo, hi, scene_mag, plo, phi);
+    node[c ^ swz] = plo.x;
+    node[(K + c) ^ swz] = phi.x;
+    node[(2 * K + c) ^ swz] = plo.y;
+    node[(3 * K + c) ^ swz] = phi.y;
+    node[(4 * K + c) ^ swz] = plo.z;
+    node[(5 * K + c) ^ swz] = phi.z;
+    const float ex = phi.x - plo.x, ey = phi.y - plo.y, ez = phi.z - plo.z;
+    const float area = ex * ey + ey * ez + ez * ex;
+    return (double)area * (cnt > 0 ? (double)kCostPrim * cnt : (double)kCostNode);
+}
+// The SAH sum's partial sums, 32 bytes apart: with one of them, a warp's atomic add
+// at a time, the sum alone took 2 ns a warp, 100 us for the widest level.
+constexpr uint32_t kSahSums = 64, kSahStride = 4;
+constexpr size_t kSahDoubles = 1 + kSahSums * kSahStride;  // the root's area, then the sums
+__device__ __forceinline__ void add_sah(double sah, double *acc) {
+    for (int o = 16; o > 0; o >>= 1) sah += __shfl_xor_sync(0xffffffffu, sah, o);
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) / 32;
+    if ((threadIdx.x & 31) == 0 && sah != 0.0) atomicAdd(acc + 1 + warp % kSahSums * kSahStride, sah);
 }
 
-// Refit of one level: leaf slots from the primitives, inner slots from the
-// union of the child node's slots (deeper levels are refit first).
+// One level, also summing the SAH cost.  Bound by the latency of its
+// gathers: 4.1M triangles (1.15M nodes), all levels with the SAH sum 0.17 ms, 0.53
+// with a thread a node, every level its own launch and the SAH in a pass of its
+// own.  One launch in which the last child's lanes go on with the parent (a counter
+// and two fences a node) took 0.26.
 template <int K>
-__global__ void k_refit_level(float *nodes, uint32_t first, uint32_t last, const float4 *prims_bvh, float scene_mag) {
-    uint32_t i = first + blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= last) return;
-    float *nd = nodes + (size_t)i * 8 * K;
-    const uint32_t swz = ptd::node_swizzle<K>(i);
-    for (int c = 0; c < K; c++) {
-        const int item = __float_as_int(nd[(6 * K + c) ^ swz]);
-        if (item == ptd::kNoItem) continue;
-        const int cnt = item_count(item), ch = cnt > 0 ? ptd::leaf_first(item) : item;
-        float4 lo = make_float4(FLT_MAX, FLT_MAX, FLT_MAX, 0.f), hi = make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, 0.f);
-        if (cnt > 0) {
-            for (int j = 0; j < cnt; j++) {
-                float3 a, b;
-                prim_box(prims_bvh, (uint32_t)(ch + j), a, b);
-                lo = make_float4(fminf(lo.x, a.x), fminf(lo.y, a.y), fminf(lo.z, a.z), 0.f);
-                hi = make_float4(fmaxf(hi.x, b.x), fmaxf(hi.y, b.y), fmaxf(hi.z, b.z), 0.f);
-            }
-        } else {
-            const float *rec = nodes + (size_t)ch * 8 * K;
-            const auto cn = [&](int w) { return rec[w ^ ptd::node_swizzle<K>(ch)]; };
-            for (int g = 0; g < K; g++) {
-                if (__float_as_int(cn(6 * K + g)) == ptd::kNoItem) continue;
-                lo = make_float4(fminf(lo.x, cn(g)), fminf(lo.y, cn(2 * K + g)), fminf(lo.z, cn(4 * K + g)), 0.f);
-                hi = make_float4(fmaxf(hi.x, cn(K + g)), fmaxf(hi.y, cn(3 * K + g)), fmaxf(hi.z, cn(5 * K + g)), 0.f);
-            }
-        }
-        float3 plo, phi;
-        padded(lo, hi, scene_mag, plo, phi);
-        write_slot<K>(nd, swz, c, plo, phi, ch, cnt);
+__global__ void __launch_bounds__(128) k_refit_level(float *nodes, uint32_t first, uint32_t last,
+                                                     const float4 *prims_bvh, float scene_mag, double *acc) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, i = first + t / K;
+    float3 plo, phi;
+    add_sah(i < last ? refit_node<K>(nodes, i, t % K, prims_bvh, scene_mag, plo, phi) : 0.0, acc);
+}
+
+// The levels from `top` up to the root (short ones, at most kTopLevels of them) in
+// one block, and the root's area into acc[0].
+constexpr int kTopLevels = 32;
+constexpr uint32_t kTopNodes = 256;  // of a level refit by one block
+struct TopLevels {
+    uint32_t start[kTopLevels + 1];  // first node of each level from the root down, then the end
+};
+template <int K>
+__global__ void __launch_bounds__(1024) k_refit_top(float *nodes, TopLevels lv, int levels, const float4 *prims_bvh,
+                                                    float scene_mag, double *acc) {
+    double sah = 0.0;
+    float3 plo = f3(0.f, 0.f, 0.f), phi = plo;
+    for (int l = levels - 1; l >= 0; l--) {
+        for (uint32_t t = threadIdx.x; t / K < lv.start[l + 1] - lv.start[l]; t += blockDim.x)
+            sah += refit_node<K>(nodes, lv.start[l] + t / K, t % K, prims_bvh, scene_mag, plo, phi);
+        __syncthreads();  // the level above reads these nodes
     }
+    if (threadIdx.x < K) {  // each holds its slot of the root
+        const unsigned slots = (1u << K) - 1u;
+        for (int o = 1; o < K; o <<= 1) {
+            plo = f3(fminf(plo.x, __shfl_xor_sync(slots, plo.x, o)), fminf(plo.y, __shfl_xor_sync(slots, plo.y, o)),
+                     fminf(plo.z, __shfl_xor_sync(slots, plo.z, o)));
+            phi = f3(fmaxf(phi.x, __shfl_xor_sync(slots, phi.x, o)), fmaxf(phi.y, __shfl_xor_sync(slots, phi.y, o)),
+                     fmaxf(phi.z, __shfl_xor_sync(slots, phi.z, o)));
+        }
+        const double ex = phi.x - plo.x, ey = phi.y - plo.y, ez = phi.z - plo.z;
+        if (threadIdx.x == 0) acc[0] = plo.x <= phi.x ? ex * ey + ey * ez + ez * ex : 0.0;
+    }
+    __syncthreads();
+    add_sah(sah, acc);
 }
 
 // World-space re-transform of one mesh instance's vertices (same arithmetic
@@ -987,17 +1028,16 @@ __global__ void k_transform_vertices(const float *obj, uint32_t nv, float4 m0, f
     float wz = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(m2.x, x), __fmul_rn(m2.y, y)), __fmul_rn(m2.z, z)), m2.w);
     vpos[v] = make_float4(wx, wy, wz, 0.f);
 }
+// A vertex of a triangle per thread, so that a record is written in one piece (4.1M triangles
+// 68 us; a triangle per thread 100).
 __global__ void k_rebuild_tri_records(const uint32_t *tri_vidx, const float4 *vpos, uint32_t first, uint32_t count,
                                       float4 *prims) {
-    uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t t = j / 3, v = j - 3 * t;
     if (t >= count) return;
-    uint32_t p = first + t;
-    float4 a = vpos[tri_vidx[3 * p]], b = vpos[tri_vidx[3 * p + 1]], c = vpos[tri_vidx[3 * p + 2]];
-    float4 *r = prims + 3 * (size_t)p;
-    float w = r[0].w;  // keep the id
-    r[0] = make_float4(a.x, a.y, a.z, w);
-    r[1] = make_float4(b.x, b.y, b.z, 0.f);
-    r[2] = make_float4(c.x, c.y, c.z, 0.f);
+    const size_t at = 3 * (size_t)first + j;
+    const float4 a = vpos[tri_vidx[at]];
+    prims[at] = make_float4(a.x, a.y, a.z, v == 0 ? __int_as_float((int)(first + t)) : 0.f);  // its id
 }
 
 // All mesh instances at once: world vertex v belongs to the instance whose
@@ -1023,22 +1063,6 @@ __global__ void k_transform_all(const float *obj, const XformRec *recs, uint32_t
     float wy = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(r.m1.x, x), __fmul_rn(r.m1.y, y)), __fmul_rn(r.m1.z, z)), r.m1.w);
     float wz = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(r.m2.x, x), __fmul_rn(r.m2.y, y)), __fmul_rn(r.m2.z, z)), r.m2.w);
     vpos[v] = make_float4(wx, wy, wz, 0.f);
-}
-
-// Root box area for the SAH normalisation: union of the root node's slots.
-template <int K>
-__global__ void k_root_area(const float *nodes, double *out) {
-    if (threadIdx.x || blockIdx.x) return;
-    float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-    for (int c = 0; c < K; c++) {
-        if (__float_as_int(nodes[6 * K + c]) == ptd::kNoItem) continue;
-        for (int a = 0; a < 3; a++) {
-            lo[a] = fminf(lo[a], nodes[2 * a * K + c]);
-            hi[a] = fmaxf(hi[a], nodes[(2 * a + 1) * K + c]);
-        }
-    }
-    double ex = hi[0] - lo[0], ey = hi[1] - lo[1], ez = hi[2] - lo[2];
-    *out = lo[0] <= hi[0] ? ex * ey + ey * ez + ez * ex : 0.0;
 }
 
 inline uint32_t blocks(size_t n, int b) { return (uint32_t)((n + b - 1) / b); }
@@ -1250,35 +1274,23 @@ int build_wide(pt_scene *s, const Scratch &sc, uint32_t n, int root, uint32_t ma
 }
 
 template <int K>
-void refit_levels(pt_scene *s, cudaStream_t st) {
+void refit_tree(pt_scene *s, cudaStream_t st) {
     float *nodes = s->nodes.as<float>();
-    for (int L = (int)s->level_start.size() - 2; L >= 0; L--) {
-        uint32_t a = s->level_start[L], b = s->level_start[L + 1];
-        if (b > a) k_refit_level<K><<<blocks(b - a, 128), 128, 0, st>>>(nodes, a, b, s->prims_bvh.as<float4>(), s->scene_mag);
+    const float4 *prims = s->prims_bvh.as<float4>();
+    double *acc = s->sah_scratch.as<double>();
+    const std::vector<uint32_t> &ls = s->level_start;
+    const int levels = (int)ls.size() - 1;
+    TopLevels tl = {};
+    int top = 0;  // levels of the last launch
+    while (top < std::min(levels, kTopLevels) && ls[top + 1] - ls[top] <= kTopNodes) {
+        tl.start[top] = ls[top];
+        tl.start[top + 1] = ls[top + 1];
+        top++;
     }
-}
-
-template <int K>
-void sah_launch(pt_scene *s, double *acc, cudaStream_t st) {
-    uint32_t nn = s->level_start.back();
-    k_sah<K><<<blocks(nn, 256), 256, 0, st>>>(s->nodes.as<float>(), nn, acc);
-    k_root_area<K><<<1, 1, 0, st>>>(s->nodes.as<float>(), acc + 1);
-}
-
-// SAH cost of the current wide tree (node cost 1.2, primitive cost 1),
-// normalised by the root box area.
-int compute_sah(pt_scene *s, double *scratch2, cudaStream_t st, float &out) {
-    PT_CUDA_TRY(cudaMemsetAsync(scratch2, 0, 2 * sizeof(double), st));
-    switch (s->bvh_opts.width) {
-        case 2: sah_launch<2>(s, scratch2, st); break;
-        case 4: sah_launch<4>(s, scratch2, st); break;
-        default: sah_launch<8>(s, scratch2, st); break;
-    }
-    double h[2] = {0.0, 0.0};
-    PT_CUDA_TRY(cudaMemcpyAsync(h, scratch2, sizeof(h), cudaMemcpyDeviceToHost, st));
-    PT_CUDA_TRY(cudaStreamSynchronize(st));
-    out = h[1] > 0 ? (float)((kCostNode * h[1] + h[0]) / h[1]) : 0.f;
-    return PT_OK;
+    for (int l = levels - 1; l >= top; l--)
+        k_refit_level<K><<<blocks((size_t)(ls[l + 1] - ls[l]) * K, 128), 128, 0, st>>>(nodes, ls[l], ls[l + 1], prims,
+                                                                                      s->scene_mag, acc);
+    k_refit_top<K><<<1, 1024, 0, st>>>(nodes, tl, top, prims, s->scene_mag, acc);
 }
 
 // PLOC over the sorted order in sc.vals[0] (n >= 2); the root is node n - 2.
@@ -1456,28 +1468,34 @@ int pt_compress_wide8(const float *nodes, uint32_t n, float4 *out, cudaStream_t 
 int pt_bvh_refit_impl(pt_scene *s, cudaStream_t st) {
     pt_nvtx::Range nv("pt_bvh_refit");
     const uint32_t n = s->num_prims;
+    int e = s->sah_scratch.ensure(kSahDoubles * sizeof(double));
+    if (e != PT_OK) return e;
     PT_CUDA_TRY(cudaEventRecord(s->ev0, st));
+    PT_CUDA_TRY(cudaMemsetAsync(s->sah_scratch.ptr, 0, kSahDoubles * sizeof(double), st));
     if (n > 0)
         k_gather_prims<<<blocks(3 * (size_t)n, 256), 256, 0, st>>>(s->prims_world.as<float4>(), s->bvh_order.as<uint32_t>(), n,
                                                         s->prims_bvh.as<float4>());
     switch (s->bvh_opts.width) {
-        case 2: refit_levels<2>(s, st); break;
-        case 4: refit_levels<4>(s, st); break;
-        default: refit_levels<8>(s, st); break;
+        case 2: refit_tree<2>(s, st); break;
+        case 4: refit_tree<4>(s, st); break;
+        default: refit_tree<8>(s, st); break;
     }
     PT_CUDA_TRY(cudaGetLastError());
     if (s->bvh_opts.width == 8) {
-        const int e = pt_compress_wide8(s->nodes.as<float>(), s->bvh_stats.num_nodes, s->cnodes.as<float4>(), st);
+        e = pt_compress_wide8(s->nodes.as<float>(), s->bvh_stats.num_nodes, s->cnodes.as<float4>(), st);
         if (e != PT_OK) return e;
     }
     PT_CUDA_TRY(cudaEventRecord(s->ev1, st));
-    PT_CUDA_TRY(cudaEventSynchronize(s->ev1));
+    double h[kSahDoubles] = {};
+    PT_CUDA_TRY(cudaMemcpyAsync(h, s->sah_scratch.ptr, sizeof(h), cudaMemcpyDeviceToHost, st));
+    PT_CUDA_TRY(cudaStreamSynchronize(st));
     float ms = 0.f;
     PT_CUDA_TRY(cudaEventElapsedTime(&ms, s->ev0, s->ev1));
     s->bvh_stats.build_ms = ms;
-    int e = s->sah_scratch.ensure(64);
-    if (e != PT_OK) return e;
-    return compute_sah(s, s->sah_scratch.as<double>(), st, s->bvh_stats.sah_cost);
+    double sah = 0.0;  // node cost 1.2, primitive cost 1, relative to the root's area
+    for (uint32_t k = 0; k < kSahSums; k++) sah += h[1 + k * kSahStride];
+    s->bvh_stats.sah_cost = h[0] > 0 ? (float)((kCostNode * h[0] + sah) / h[0]) : 0.f;
+    return PT_OK;
 }
 
 int pt_update_all_world_vertices(pt_scene *s, const float *d_obj_pos, cudaStream_t st) {
@@ -1506,7 +1524,7 @@ int pt_update_all_world_vertices(pt_scene *s, const float *d_obj_pos, cudaStream
     if (total) k_transform_all<<<blocks(total, 256), 256, 0, st>>>(d_obj_pos, s->xform_table.as<XformRec>(), nrec, total,
                                                                    s->vpos.as<float4>());
     if (s->num_tris)
-        k_rebuild_tri_records<<<blocks(s->num_tris, 256), 256, 0, st>>>(s->tri_vidx.as<uint32_t>(), s->vpos.as<float4>(), 0,
+        k_rebuild_tri_records<<<blocks(3 * (size_t)s->num_tris, 256), 256, 0, st>>>(s->tri_vidx.as<uint32_t>(), s->vpos.as<float4>(), 0,
                                                                         s->num_tris, s->prims_world.as<float4>());
     PT_CUDA_TRY(cudaGetLastError());
     PT_CUDA_TRY(cudaStreamSynchronize(st));
@@ -1527,7 +1545,7 @@ int pt_update_world_vertices(pt_scene *s, uint32_t mesh, const float *d_obj_pos,
         for (const MeshInstanceRef &q : s->mesh_instances)
             if (q.prim_offset > first && q.prim_offset < next) next = q.prim_offset;
         count = next - first;
-        if (count) k_rebuild_tri_records<<<blocks(count, 256), 256, 0, st>>>(s->tri_vidx.as<uint32_t>(), s->vpos.as<float4>(),
+        if (count) k_rebuild_tri_records<<<blocks(3 * (size_t)count, 256), 256, 0, st>>>(s->tri_vidx.as<uint32_t>(), s->vpos.as<float4>(),
                                                                              first, count, s->prims_world.as<float4>());
     }
     PT_CUDA_TRY(cudaGetLastError());

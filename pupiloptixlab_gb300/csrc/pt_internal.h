@@ -115,7 +115,7 @@ struct pt_scene {
     // BVH build scratch and results
     DevBuf bvh_scratch;
     DevBuf bvh_order;  // primitive id of each leaf slot (sorted Morton order)
-    DevBuf sah_scratch;     // two doubles for the SAH reduction
+    DevBuf sah_scratch;     // partial sums of the SAH reduction
     DevBuf xform_table;     // per mesh instance: world vertex range + matrix (all-vertex updates)
     DevBuf all_obj_pos;     // host positions staged for pt_scene_update_all_vertices
     uint64_t total_mesh_vertices = 0;
