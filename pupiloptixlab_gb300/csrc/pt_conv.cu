@@ -5,9 +5,9 @@
 // Tiling.  Accumulator tiles have 128 rows:
 //   forward / data gradient: 128 pixels (one 128-wide row segment, or
 //     128 / W whole rows of a narrow image) x n_tile output channels.  Persistent
-//     CTAs of 6 warps walk the tiles: warp 0 streams operands into a ring of
+//     CTAs of 10 warps walk the tiles: warp 0 streams operands into a ring of
 //     `stages` buffers, warp 1 issues the MMAs into one of two accumulators,
-//     warps 2-5 run the epilogue of the other (k_conv_fwd_persistent);
+//     warps 2-9 run the epilogue of the other (k_conv_fwd_persistent);
 //   weight gradient: 128 (tap, input channel) rows x n_tile output channels,
 //     accumulated over a range of pixel tiles and added to the FP32 result,
 //     one CTA of 4 warps per (row tile, channel tile, pixel range): thread 0
@@ -26,7 +26,7 @@
 // The zero padding of the convolution comes from TMA's out-of-bounds fill:
 // the box for tap (dy, dx) starts at (x0 + dx - 1, y0 + dy - 1).
 //
-// Every wait is bounded (%globaltimer, 2 s): on expiry the kernel records a
+// Every wait is bounded (at least 2 s by the SM clock): on expiry the kernel records a
 // code in *err, stops issuing work, lets issued copies and MMAs drain (again
 // with a bound), frees its tensor memory and returns.
 #include <cuda.h>
