@@ -564,7 +564,7 @@ PT_DI void shade_one(const DevScene &s, const Outputs &out, const State &st, con
 }
 
 // Bound by the latency of its gathers (path state, vertices, tables): 4 blocks
-// of 256 threads per SM (64 registers, 332 bytes of spills) hide more of it
+// of 256 threads per SM (64 registers, 300 bytes of spills) hide more of it
 // than 3 (80 registers) or 2 (no spills): 22.8 / 23.4 / 26.2 ms a 64-spp 1080p
 // frame of the 1M-triangle field, 0.209 / 0.226 / 0.246 ms on the Cornell box.
 // 32.7 ms with a path's ray, stream and flags in separate 4- to 16-byte arrays.

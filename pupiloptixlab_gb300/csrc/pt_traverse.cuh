@@ -15,7 +15,8 @@
 //   node  = 8*K floats: lo_x[K] hi_x[K] lo_y[K] hi_y[K] lo_z[K] hi_z[K]
 //           item[K], K unused.  item: a traversal item (below): an inner node's
 //           index, a leaf's first slot and count, or kNoItem (empty slot, a
-//           point box far away).  Loaded in 256-bit loads.
+//           point box far away).  Stored swizzled by the node's index
+//           (node_swizzle), loaded 16 or 32 bytes at a time (load_node).
 //   prim  = 3 float4 per slot: triangle (v0, id) (v1, 0) (v2, 0);
 //           sphere (centre, id | 1<<31) (radius, 0, 0, 0) (0);
 //           curve piece (c0, id | 1<<31) (r0, r1, u0, kind bits) (c1, u1):
