@@ -402,8 +402,10 @@ __device__ __forceinline__ NodeBox form_node(const Tree &t, int id, int l, int r
         }
     }
     const float c_wide = kCostNode * area + best;
-    const float c_leaf = u.count() <= t.max_leaf ? area * u.weight() : FLT_MAX;
-    const bool mk_leaf = c_leaf <= c_wide;
+    // the limit is a condition, not a cost: an area may overflow to infinity (the
+    // split then stays j = 1, and the node is wide)
+    const float c_leaf = area * u.weight();
+    const bool mk_leaf = u.count() <= t.max_leaf && c_leaf <= c_wide;
     sx[0] = mk_leaf ? c_leaf : c_wide;
     uint32_t sel = (uint32_t)jw | (mk_leaf ? kSelLeaf : 0);
 #pragma unroll

@@ -57,3 +57,33 @@ def test_every_primitive_is_found(cuda_ctx, n, kind, flags):
         # box's extent, 1e-6 of the box's) a side and level, 12 levels, against boxes of 0.05 and more:
         # 4 * 2.6e-6 * 12 / 0.05 = 2.5e-3 of an area
         assert g.refit().sah_cost == pytest.approx(st.sah_cost, rel=5e-3)
+
+
+@pytest.mark.parametrize("flags", [0, abi.BVH_FAST_BUILD], ids=["ploc", "radix"])
+@pytest.mark.parametrize("n", [40, 3000])
+def test_box_area_overflows(cuda_ctx, n, flags):
+    """A triangle whose box has no finite area (2.4e19 on two axes) among n small
+    ones: its ancestors' costs are infinite and every primitive is still found.
+    The triangle is a strip that passes 1.5e18 from the origin, so that the
+    intersection test itself stays finite; rays run along y, across it."""
+    sc, p = triangles(n, "scattered")
+    strip = np.array([[-1.2, 0, -1.0], [1.2, 0, 1.4], [1.2, 0, 1.3]]) * 1e19 + np.array([0.0, -3.0, 0.0])
+    sc.add_instance(abi.SHAPE_MESH, sc.add_mesh(scenes.Mesh(strip, np.array([[0, 1, 2]]))), sc.add_material(scenes.diffuse(0.5)))
+    r = np.random.default_rng(5)
+    pick = np.arange(1000) % n
+    o = np.concatenate([p[pick].mean(axis=1), np.tile([0.0, -1.0, 1.75e18], (3, 1))])
+    d = np.concatenate([r.normal(size=(1000, 3)) * [0.2, 0, 0.2] + [0, 1, 0], np.tile([1e-3, -1.0, 1e-3], (3, 1))])
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    o[:1000] -= 4.0 * d[:1000]
+    rays = np.zeros((len(o), 8), np.float32)
+    rays[:, 0:3], rays[:, 3], rays[:, 4:7], rays[:, 7] = o, 0.001, d, 1e16
+    ref = oracle.OracleScene(sc, bvh=False).trace(rays, brute_force=True)
+    hit = ref.view(np.int32)[:, 1] >= 0
+    assert hit[1000:].all() and hit[:1000].mean() > 0.9
+    dev = torch.from_numpy(rays).cuda()
+    g = GpuScene(cuda_ctx, sc, build=False)
+    for width in (2, 4, 8):
+        assert g.build_bvh(width=width, flags=flags).num_prims == n + 1
+        assert np.array_equal(g.trace(dev).cpu().numpy().view(np.uint32), ref.view(np.uint32)), (n, width)
+        g.refit()
+        assert np.array_equal(g.trace(dev).cpu().numpy().view(np.uint32), ref.view(np.uint32)), (n, width, "refit")
