@@ -571,7 +571,8 @@ int pt_conv3x3_backward_weights(const void *x, uint32_t n, uint32_t h, uint32_t 
                                 uint32_t cout, float *dweight, float *dbias, void *stream);
 /* Bounded waits of the convolution kernels (no counterpart in the reference,
  * whose closed OptiX denoiser has none): every mbarrier wait gives up after
- * wait_ns of GPU time (0 restores the default, 2 s); the kernel then records
+ * wait_ns of GPU time (0 restores the default, 2 s; counted in SM
+ * cycles, so longer where the clock is below its maximum); the kernel then records
  * an error, lets the copies and MMAs it issued finish, frees its tensor memory
  * and returns, and the call reports PT_ERR_TIMEOUT.  stall_next = 1 makes the
  * next forward convolution that is prepared first wait on a barrier that

@@ -26,7 +26,7 @@
 // The zero padding of the convolution comes from TMA's out-of-bounds fill:
 // the box for tap (dy, dx) starts at (x0 + dx - 1, y0 + dy - 1).
 //
-// Every wait is bounded (at least 2 s by the SM clock): on expiry the kernel records a
+// Every wait is bounded (at least 2 s, counted in SM cycles): on expiry the kernel records a
 // code in *err, stops issuing work, lets issued copies and MMAs drain (again
 // with a bound), frees its tensor memory and returns.
 #include <cuda.h>
@@ -80,15 +80,16 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 // Bounded wait for the phase with the given parity to complete: false after
-// limit_ns (in SM cycles at two per nanosecond, so at least that long), or as
-// soon as *abort is set (another warp of the CTA gave up), so that a failing CTA
-// leaves within one limit.  try_wait itself suspends the thread until the phase
+// limit_ns (counted in SM cycles, 2.25 per nanosecond: the clock's maximum is
+// 2.07 GHz, so at least that long; at two per nanosecond 400 ms ran out after 387),
+// or as soon as *abort is set (another warp of the CTA gave up), so that a failing
+// CTA leaves within one limit.  try_wait itself suspends the thread until the phase
 // completes or a short hardware limit passes.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint64_t limit_ns = kWaitNs,
                                           const volatile int *abort = nullptr) {
     if (mbar_try(bar, parity)) return true;
     const long long t0 = clock64();
-    const long long limit = static_cast<long long>(limit_ns * 2);
+    const long long limit = static_cast<long long>(limit_ns * 2 + limit_ns / 4);
     for (;;) {
 #pragma unroll 1
         for (int i = 0; i < 8; i++)

@@ -183,3 +183,26 @@ def test_bounded_wait_runs_out_and_the_next_convolution_is_right(cuda_ctx, shape
     ref = _ref_conv(x.cpu(), wt.cpu(), None)
     assert float((y - ref).abs().max()) <= 2e-3 * float(ref.abs().max())
     assert _rel_l2(y, ref) <= 1e-4
+
+
+def test_bounded_wait_lasts_its_limit(cuda_ctx):
+    """A wait that runs out lasted at least the limit it was given, whatever the
+    SM clock (the kernel counts cycles)."""
+    from pupiloptixlab_gb300 import abi
+    from pupiloptixlab_gb300 import denoiser as dnm
+    limit_ms = 400
+    g = torch.Generator().manual_seed(8)
+    x, wt = _bf16((1, 8, 16, 16), g).cuda(), _bf16((16, 9, 16), g, 0.1).cuda()
+    dnm.conv3x3_forward(x, wt, None, 16)
+    t0, t1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+    lib = cuda_ctx.lib
+    assert lib.pt_conv_set_wait_limit(limit_ms * 1_000_000, 1) == 0
+    try:
+        t0.record()
+        with pytest.raises(abi.PtError):
+            dnm.conv3x3_forward(x, wt, None, 16)
+        t1.record()
+    finally:
+        assert lib.pt_conv_set_wait_limit(0, 0) == 0
+    t1.synchronize()
+    assert limit_ms <= t0.elapsed_time(t1) < 1500
