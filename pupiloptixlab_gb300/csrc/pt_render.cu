@@ -1093,14 +1093,18 @@ struct Launcher {
             PT_CUDA_TRY(cudaStreamWaitEvent(ws.stream, ws.ev_in, 0));
         }
         const bool replay = graph && ws.exec && key == ws.exec_key;
-        k_begin<<<1, 256, 0, ls>>>(stt.counters, (uint32_t)(counter_bytes / 4), CallBlock{out, p->seed, p->sample_cnt});
-        PT_CUDA_TRY(cudaGetLastError());
+        const auto begin = [&]() -> int {  // the first launch inside render_ms
+            PT_CUDA_TRY(cudaEventRecord(t.ev0, ls));
+            k_begin<<<1, 256, 0, ls>>>(stt.counters, (uint32_t)(counter_bytes / 4), CallBlock{out, p->seed, p->sample_cnt});
+            PT_CUDA_TRY(cudaGetLastError());
+            return PT_OK;
+        };
+        if (!graph && (e = begin()) != PT_OK) return e;
         if (graph && !replay) PT_CUDA_TRY(cudaStreamBeginCapture(ws.stream, cudaStreamCaptureModeThreadLocal));
         Timer tm;
         uint32_t launches = 1;
         uint32_t waves = 0;
         pt_nvtx::Range nv_render(replay ? "pt_render: replay" : graph ? "pt_render: capture" : "pt_render: launches");
-        if (!graph) PT_CUDA_TRY(cudaEventRecord(t.ev0, st));
         cudaError_t enq = cudaSuccess;
         const auto order = [&](cudaStream_t from, cudaStream_t to, cudaEvent_t ev) {  // `to` continues after `from`
             if (from == to || enq != cudaSuccess) return;
@@ -1231,7 +1235,7 @@ struct Launcher {
         }
         if (graph) {
             pt_nvtx::Range r("pt_render: graph launch");
-            PT_CUDA_TRY(cudaEventRecord(t.ev0, ws.stream));
+            if ((e = begin()) != PT_OK) return e;
             PT_CUDA_TRY(cudaGraphLaunch(ws.exec, ws.stream));
             PT_CUDA_TRY(cudaEventRecord(t.ev1, ws.stream));
             PT_CUDA_TRY(cudaEventRecord(ws.ev_out, ws.stream));

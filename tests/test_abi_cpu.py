@@ -106,3 +106,15 @@ def test_entry_points_validate_without_a_device(ptlib):
         st = ptlib.pt_context_create(C.byref(abi.DeviceOpts(0, 0)), C.byref(h))
         assert st == 6 and not h.value  # PT_ERR_UNSUPPORTED, no context
         assert "no CUDA device" in abi.last_error(ptlib)
+
+
+def test_render_ms_covers_the_first_launch():
+    """pt_render_stats.render_ms is the device time of the whole call: the events
+    around it are recorded before the launch that clears the counters and sets
+    the call's arguments, on every route, and after the last one."""
+    text = (ROOT / "pupiloptixlab_gb300" / "csrc" / "pt_render.cu").read_text()
+    body = text[text.index("run_waves(const RunTarget"):text.index("cudaEventElapsedTime(&rs.render_ms")]
+    launches = body.count("k_begin<<<")
+    assert launches >= 1
+    assert len(re.findall(r"cudaEventRecord\(t\.ev0[^\n]*\n\s*k_begin<<<", body)) == launches
+    assert body.count("t.ev0") == launches  # and recorded nowhere later
