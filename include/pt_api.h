@@ -546,6 +546,10 @@ int pt_denoiser_set_lr(pt_denoiser *dn, float lr);
 /* Network output for a batch: out = width*height*n*3 FP32 linear RGB (device). */
 int pt_denoiser_forward(pt_denoiser *dn, const void *input_f16, uint32_t n, uint32_t height, uint32_t width,
                         float *out, void *stream);
+/* How the last forward or denoised frame was pooled: bit l of *levels is set where
+ * the convolution that ends encoder level l averaged its own output (images wide
+ * and large enough; the other levels are pooled by a kernel of their own). */
+int pt_denoiser_fused_pools(const pt_denoiser *dn, uint32_t *levels);
 /* Denoise one rendered frame (any size; padded internally to multiples of 16),
  * with the per-tile fallback to the raw colour. */
 int pt_denoise(pt_denoiser *dn, const pt_denoise_io *io, void *stream);

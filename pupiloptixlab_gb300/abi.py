@@ -194,6 +194,7 @@ PROTOTYPES = [
     ("pt_denoiser_set_lr", C.c_int, [C.c_void_p, C.c_float]),
     ("pt_denoiser_forward", C.c_int, [C.c_void_p, C.c_void_p, C.c_uint32, C.c_uint32, C.c_uint32, C.c_void_p,
                                       C.c_void_p]),
+    ("pt_denoiser_fused_pools", C.c_int, [C.c_void_p, C.POINTER(C.c_uint32)]),
     ("pt_denoise", C.c_int, [C.c_void_p, C.POINTER(DenoiseIO), C.c_void_p]),
     ("pt_denoise_get_stats", C.c_int, [C.c_void_p, C.POINTER(DenoiseStats)]),
     ("pt_denoise_pack", C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_uint32, C.c_uint32, C.c_void_p,

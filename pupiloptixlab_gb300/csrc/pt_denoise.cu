@@ -1153,6 +1153,18 @@ int pt_denoiser_forward(pt_denoiser *dn, const void *input_f16, uint32_t n, uint
     return leave(dn, caller);
 }
 
+int pt_denoiser_fused_pools(const pt_denoiser *dn, uint32_t *levels) {
+    if (!dn || !levels) {
+        pt_set_error("pt_denoiser_fused_pools: NULL argument");
+        return PT_ERR_INVALID;
+    }
+    const int ends[] = {E0B, E1B, E2B, E3B};
+    *levels = 0;
+    for (int l = 0; dn->infer_plan.n && l < 4; l++)  // (no frame yet: none)
+        if (ptconv::fwd_pooled(dn->infer_plan.fwd[ends[l]])) *levels |= 1u << l;
+    return PT_OK;
+}
+
 int pt_denoise(pt_denoiser *dn, const pt_denoise_io *io, void *stream) {
     pt_nvtx::Range nv("pt_denoise");
     (void)cudaGetLastError();

@@ -175,6 +175,12 @@ class Denoiser:
                   "pt_denoiser_forward", self.lib)
         return out
 
+    def fused_pools(self) -> int:
+        """Encoder levels (bit l) whose pooling the last forward or denoise call left to the convolution."""
+        v = C.c_uint32()
+        abi.check(self.lib.pt_denoiser_fused_pools(self.handle, C.byref(v)), "pt_denoiser_fused_pools", self.lib)
+        return v.value
+
     def denoise(self, buffers: dict, width: int, height: int, tile: int = 16, fallback_rel: float = 0.25,
                 fallback_sigma: float = 4.0, want_tiles: bool = False, ensemble: bool = False):
         """Denoise a rendered frame; returns (output (h*w, 4) f32, stats, tile flags or None).

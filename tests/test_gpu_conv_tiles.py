@@ -51,3 +51,34 @@ def test_weight_gradient_tiles(cuda_ctx, shape):
     ref = wr.grad.permute(0, 2, 3, 1).reshape(cout, 9, cin)
     assert float((dw - ref).abs().max()) <= 2e-3 * float(ref.abs().max())
     assert _rel(dw, ref) <= 1e-4 and _rel(db, br.grad) <= 1e-4
+
+
+@pytest.mark.parametrize("rows", ["2", "3", "4"])
+@pytest.mark.parametrize("shape", [(2, 7, 130, 16, 32), (1, 9, 256, 32, 64), (1, 6, 140, 48, 48)])
+def test_bf16_rows_agree(cuda_ctx, monkeypatch, rows, shape):
+    """BF16 outputs with ReLU and masked data gradients of halo tiles with several
+    rows: bit for bit those of one-row tiles."""
+    from pupiloptixlab_gb300 import denoiser as dnm
+    n, h, w, cin, cout = shape
+    g = torch.Generator().manual_seed(h + w)
+    x, wt, b = _bf16((n, h, w, cin), g).cuda(), _bf16((cout, 9, cin), g, 0.1).cuda(), torch.randn(cout, generator=g).cuda()
+    dy, mask = _bf16((n, h, w, cout), g).cuda(), _bf16((n, h, w, cin), g).cuda()
+    outs = []
+    for r in ("1", rows):
+        monkeypatch.setenv("PT_CONV_HALO_ROWS", r)
+        outs.append((dnm.conv3x3_forward(x, wt, b, cout, relu=True), dnm.conv3x3_backward_data(dy, wt, cin, mask)))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+
+
+def test_many_halo_tiles_a_cta(cuda_ctx, monkeypatch):
+    """More than three tiles a CTA at any number of rows (both accumulators, the ring across tiles)."""
+    from pupiloptixlab_gb300 import denoiser as dnm
+    n, h, w, cin, cout = 1, 1021, 600, 16, 32
+    g = torch.Generator().manual_seed(17)
+    x, wt, b = _bf16((n, h, w, cin), g), _bf16((cout, 9, cin), g, 0.1), torch.randn(cout, generator=g)
+    ref = F.conv2d(x.float().permute(0, 3, 1, 2), wt.float().reshape(cout, 3, 3, cin).permute(0, 3, 1, 2), b, padding=1)
+    ref = ref.permute(0, 2, 3, 1)
+    for rows in ("1", "2", "4"):
+        monkeypatch.setenv("PT_CONV_HALO_ROWS", rows)
+        y = dnm.conv3x3_forward(x.cuda(), wt.cuda(), b.cuda(), cout, out_f32=True).cpu()
+        assert float((y - ref).abs().max()) <= 2e-3 * float(ref.abs().max()) and _rel(y, ref) <= 1e-4, rows

@@ -84,6 +84,36 @@ def test_wide_frame_with_fused_pooling_and_upsampling(cuda_ctx, dn, monkeypatch)
     assert _rel(fused.numpy(), ref) <= 2e-2
 
 
+def test_pooling_in_the_epilogue_of_two_and_four_row_tiles(cuda_ctx, dn, monkeypatch):
+    """Encoder levels pooled by the convolution, with tiles of two and of four
+    rows and with the rows that the size gives, against pooling and up-sampling
+    by kernels of their own (one-row tiles): bit for bit the same, and close to the
+    CPU restatement."""
+    from oracle import denoiser_ref
+    from pupiloptixlab_gb300.denoiser import Denoiser
+    inp, _ = _batch(1, 384, 640, 6)  # levels 640, 320, 160 and 80 wide: the first three can be pooled there
+
+    def run(**env):
+        with monkeypatch.context() as m:
+            for k, v in env.items():
+                m.setenv(k, v)
+            d = Denoiser(cuda_ctx, seed=3)
+            d.set_params(dn.get_params())
+            out, levels = d.forward(inp.cuda()).cpu(), d.fused_pools()
+            d.close()
+        return out, levels
+
+    separate, levels = run(PT_CONV_HALO_ROWS="1", PT_CONV_NO_FUSED_POOL="1", PT_DENOISER_SEPARATE_UPSAMPLE="1")
+    assert levels == 0
+    for rows in ("2", "4"):
+        out, levels = run(PT_CONV_HALO_ROWS=rows)
+        assert levels == 0b111 and torch.equal(out, separate), rows
+    out, levels = run()
+    assert levels & 1 and torch.equal(out, separate)
+    ref = denoiser_ref.denoise(dn.get_params(), inp.float().numpy())
+    assert _rel(out.numpy(), ref) <= 2e-2
+
+
 def test_gradients_match_cpu(dn):
     from oracle import denoiser_ref
     inp, tgt = _batch(2, 32, 32, 2)
