@@ -87,3 +87,25 @@ def test_box_area_overflows(cuda_ctx, n, flags):
         assert np.array_equal(g.trace(dev).cpu().numpy().view(np.uint32), ref.view(np.uint32)), (n, width)
         g.refit()
         assert np.array_equal(g.trace(dev).cpu().numpy().view(np.uint32), ref.view(np.uint32)), (n, width, "refit")
+
+
+@pytest.mark.parametrize("width", [2, 4, 8])
+def test_many_clusters(cuda_ctx, width):
+    """Enough primitives that clustering searches for four positions a thread
+    (300,000 clusters, tiles of 1,120), with a part of a last tile."""
+    n = 301_001
+    sc, p = triangles(n, "scattered", seed=4)
+    r = np.random.default_rng(6)
+    pick = np.concatenate([r.integers(0, n, 1500), [0, n - 1]])
+    d = r.normal(size=(len(pick), 3))
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    rays = np.zeros((len(pick), 8), np.float32)
+    rays[:, 0:3], rays[:, 3], rays[:, 4:7], rays[:, 7] = p[pick].mean(axis=1) - 1e-2 * d, 0.001, d, 1e16
+    ref = oracle.OracleScene(sc).trace(rays)
+    g = GpuScene(cuda_ctx, sc, build=False)
+    st = g.build_bvh(width=width)
+    assert st.num_prims == n and st.builder == abi.BVH_BUILDER_PLOC
+    dev = torch.from_numpy(rays).cuda()
+    assert np.array_equal(g.trace(dev).cpu().numpy().view(np.uint32), ref.view(np.uint32))
+    g.refit()
+    assert np.array_equal(g.trace(dev).cpu().numpy().view(np.uint32), ref.view(np.uint32))
