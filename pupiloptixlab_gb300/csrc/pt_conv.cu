@@ -1335,7 +1335,6 @@ int fwd_prepare(FwdOp *op, const Act &in, const void *w, int w_rows, int cout, c
     a.cout = cout;
     a.n_tiles_n = ntiles;
     a.tmem_cols = pow2_cols(2 * (halo ? halo_rows : 1) * n_tile);  // double-buffered accumulators
-    a.halo_rows = halo_rows;
     a.halo_a_bytes = box_bytes(halo_rows);
     // CTAs per SM (two at most: 640 threads; PT_CONV_FWD_CTAS=1 or 2 overrides) and
     // the ring: resident weights where a ring of three stages fits beside them,

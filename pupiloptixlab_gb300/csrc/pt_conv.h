@@ -51,7 +51,6 @@ struct FwdArgs {
     unsigned *err;
     unsigned long long wait_ns;  // limit of every bounded wait (kWaitNs unless pt_conv_set_wait_limit changed it)
     int stall;                   // test of the timeout path: the MMA warp first waits on a barrier nothing arrives at
-    int halo_rows;               // halo kernel: output rows per tile (1-4); the box holds halo_rows + 2 rows
     int wide_io;                 // BF16 output / mask rows 32-byte aligned: 256-bit accesses in the epilogue
     int bias16;                  // bias 16-byte aligned: the epilogue reads it in 16-byte loads
     uint16_t *up;                // EPI_BF16: also written, 2x nearest up-sampled, to channels [0, cout) of

@@ -189,7 +189,6 @@ struct DevScene {
     const float4 *prims;    // 3 float4 per primitive slot in leaf order
     uint32_t width;         // 2, 4 or 8
     uint32_t num_nodes;
-    uint32_t root_is_leaf_count;  // >0: single leaf root with this many prims
     uint32_t smem_nodes;
     float pad_mag;          // scene magnitude the box padding was computed for
     // shading data (indexed by primitive id / vertex id)
