@@ -48,7 +48,11 @@
 namespace ptconv {
 
 constexpr int kMaxStages = 8;
-constexpr uint64_t kWaitNs = 2000000000ull;
+// A wait's limit counts ticks of two SM cycles, 9/8 per nanosecond: the clock's
+// maximum is 2.07 GHz, so it lasts at least its nanoseconds (at one tick per
+// nanosecond 400 ms ran out after 387).
+constexpr uint64_t wait_ticks(uint64_t ns) { return ns + ns / 8; }
+constexpr uint64_t kWaitTicks = wait_ticks(2000000000ull);
 
 // ---------------------------------------------------------------------------
 // device primitives (inline PTX)
@@ -80,16 +84,14 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 // Bounded wait for the phase with the given parity to complete: false after
-// limit_ns (counted in SM cycles, 2.25 per nanosecond: the clock's maximum is
-// 2.07 GHz, so at least that long; at two per nanosecond 400 ms ran out after 387),
-// or as soon as *abort is set (another warp of the CTA gave up), so that a failing
-// CTA leaves within one limit.  try_wait itself suspends the thread until the phase
-// completes or a short hardware limit passes.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint64_t limit_ns = kWaitNs,
+// `ticks`, or as soon as *abort is set (another warp of the CTA gave up), so that a
+// failing CTA leaves within one limit.  try_wait itself suspends the thread until
+// the phase completes or a short hardware limit passes.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint64_t ticks = kWaitTicks,
                                           const volatile int *abort = nullptr) {
     if (mbar_try(bar, parity)) return true;
     const long long t0 = clock64();
-    const long long limit = static_cast<long long>(limit_ns * 2 + limit_ns / 4);
+    const long long limit = static_cast<long long>(ticks * 2);
     for (;;) {
 #pragma unroll 1
         for (int i = 0; i < 8; i++)
@@ -476,7 +478,7 @@ __global__ void __launch_bounds__(kFwdThreads, 2)
     const uint32_t wbar = bar0 + 8u * (2 * kMaxStages + 4);  // resident weights landed
     const uint32_t sbar = bar0 + 8u * (2 * kMaxStages + 5);  // never arrived at: the stall test waits on it
     const uint32_t mdone = bar0 + 8u * (2 * kMaxStages + 6);  // MMAs of a failing CTA completed
-    const uint64_t lim = a.wait_ns;
+    const uint64_t lim = a.wait_ticks;
     auto tile_of = [&](int t, int &img, int &x0, int &y0, int &n0) {
         const int pt = t / n_n;
         n0 = (t - pt * n_n) * a.n_tile;
@@ -754,7 +756,7 @@ __global__ void __launch_bounds__(128, 1)
         int k = 0;
         for (; k < nk; k++) {
             const int s = k % S;
-            if (k >= S && !mbar_wait(empty(s), ((k / S) - 1) & 1, a.wait_ns)) {
+            if (k >= S && !mbar_wait(empty(s), ((k / S) - 1) & 1, a.wait_ticks)) {
                 record_error(a.err, 1u);
                 s_fail = 1;
                 break;
@@ -780,7 +782,7 @@ __global__ void __launch_bounds__(128, 1)
         int k = 0, s = 0;
         uint32_t phase = 0;
         for (; k < nk; k++) {
-            if (!__all_sync(0xffffffffu, mbar_wait(full(s), phase, a.wait_ns))) {
+            if (!__all_sync(0xffffffffu, mbar_wait(full(s), phase, a.wait_ticks))) {
                 if (elected) {
                     record_error(a.err, 2u);
                     s_fail = 1;
@@ -804,7 +806,7 @@ __global__ void __launch_bounds__(128, 1)
         umma_commit(done, elected);
     }
     __syncwarp();
-    const bool ok = nk > 0 && mbar_wait(done, 0, a.wait_ns);
+    const bool ok = nk > 0 && mbar_wait(done, 0, a.wait_ticks);
     if (!ok && nk > 0 && tid == 0) record_error(a.err, 4u);
     tc_fence_after();
 
@@ -912,7 +914,7 @@ __global__ void __launch_bounds__(128, 1)
             int img = t_begin / tiles_img, ty = (t_begin - img * tiles_img) / a.tiles_x;
             int tx = t_begin - img * tiles_img - ty * a.tiles_x;
             for (; k < nk && !*fail; k++) {
-                if (k >= S && !mbar_wait(empty(s), phase ^ 1u, a.wait_ns, fail)) {
+                if (k >= S && !mbar_wait(empty(s), phase ^ 1u, a.wait_ticks, fail)) {
                     record_error(a.err, 1u);
                     *fail = 1;
                     break;
@@ -954,7 +956,7 @@ __global__ void __launch_bounds__(128, 1)
         int s = 0;
         uint32_t phase = 0;
         for (int k = 0; k < nk; k++) {
-            if (!__all_sync(0xffffffffu, mbar_wait(full(s), phase, a.wait_ns, fail))) {
+            if (!__all_sync(0xffffffffu, mbar_wait(full(s), phase, a.wait_ticks, fail))) {
                 if (elected) {
                     record_error(a.err, 2u);
                     *fail = 1;
@@ -994,7 +996,7 @@ __global__ void __launch_bounds__(128, 1)
         uint32_t phase = 0;
         bool ok = true;
         for (int k = 0; k < nk && ok; k++) {
-            ok = __all_sync(0xffffffffu, mbar_wait(full(s), phase, a.wait_ns, fail));
+            ok = __all_sync(0xffffffffu, mbar_wait(full(s), phase, a.wait_ticks, fail));
             if (!ok) break;
             const uint32_t sb = base + s * a.stage_bytes + a.a_bytes + col;
 #pragma unroll 4
@@ -1022,7 +1024,7 @@ __global__ void __launch_bounds__(128, 1)
             for (int i = 0; i < 8; i++) atomicAdd(&s_db[ch + i], sum[i]);
     }
     __syncwarp();
-    const bool ok = nk > 0 && mbar_wait(done, 0, a.wait_ns);
+    const bool ok = nk > 0 && mbar_wait(done, 0, a.wait_ticks);
     if (!ok && nk > 0 && tid == 0) record_error(a.err, 4u);
     tc_fence_after();
 
@@ -1237,13 +1239,13 @@ int pick_kc(int c) {
     return 16;
 }
 
-// Limit of the kernels' bounded waits (pt_conv_set_wait_limit; 0 = kWaitNs)
+// Limit of the kernels' bounded waits (pt_conv_set_wait_limit; 0 = kWaitTicks)
 // and the one-shot request to stall the next forward convolution.
 static std::atomic<unsigned long long> g_wait_ns{0};
 static std::atomic<int> g_stall_next{0};
-unsigned long long wait_limit_ns() {
+unsigned long long wait_limit() {
     const unsigned long long v = g_wait_ns.load();
-    return v ? v : kWaitNs;
+    return v ? wait_ticks(v) : kWaitTicks;
 }
 bool take_stall_request() { return g_stall_next.exchange(0) != 0; }
 void set_wait_limit(unsigned long long ns, bool stall_next) {
@@ -1403,7 +1405,7 @@ int fwd_prepare(FwdOp *op, const Act &in, const void *w, int w_rows, int cout, c
                 (!mask || al32(mask->ptr, mask->ctot, mask->coff)) && (!a.up || al32(a.up, a.up_ctot, 0)) &&
                 !getenv_flag("PT_CONV_NO_WIDE_IO");
     a.err = err;
-    a.wait_ns = wait_limit_ns();
+    a.wait_ticks = wait_limit();
     a.stall = take_stall_request() ? 1 : 0;
     op->kc = kc;
     // no more CTAs on an SM than tensor memory holds accumulators for
@@ -1497,7 +1499,7 @@ static int wgrad_prepare_halo(WgradOp *op, const Act &x, const Act &gy, float *d
     a.ones_row = -1;
     a.dw = dw;
     a.err = err;
-    a.wait_ns = wait_limit_ns();
+    a.wait_ticks = wait_limit();
     op->bias_fused = db != nullptr;
     op->smem = std::max(a.stages * a.stage_bytes + 1024, (228 * 1024) / (512 / a.tmem_cols + 1) + 1024);
     const int base_ctas = a.nchunks_a * (gy.c / n_tile);
@@ -1572,7 +1574,7 @@ int wgrad_prepare(WgradOp *op, const Act &x, const Act &gy, float *dw, float *db
     splits = (a.total_tiles + a.tiles_per_split - 1) / a.tiles_per_split;
     a.dw = dw;
     a.err = err;
-    a.wait_ns = wait_limit_ns();
+    a.wait_ticks = wait_limit();
     op->kca = kca;
     op->kcb = kcb;
     op->halo = false;

@@ -49,7 +49,7 @@ struct FwdArgs {
     const uint16_t *mask;
     int mask_ctot, mask_coff;
     unsigned *err;
-    unsigned long long wait_ns;  // limit of every bounded wait (kWaitNs unless pt_conv_set_wait_limit changed it)
+    unsigned long long wait_ticks;  // limit of every bounded wait (kWaitTicks unless pt_conv_set_wait_limit changed it)
     int stall;                   // test of the timeout path: the MMA warp first waits on a barrier nothing arrives at
     int wide_io;                 // BF16 output / mask rows 32-byte aligned: 256-bit accesses in the epilogue
     int bias16;                  // bias 16-byte aligned: the epilogue reads it in 16-byte loads
@@ -72,7 +72,7 @@ struct WgradArgs {
     float *db;            // [cout] FP32, accumulated through the ones row (null: not fused)
     int ones_row;         // row of the last M tile whose A block holds ones (its D row = sum of gy)
     unsigned *err;
-    unsigned long long wait_ns;
+    unsigned long long wait_ticks;
 };
 
 struct FwdOp {
@@ -100,7 +100,7 @@ int pick_kc(int c);
 // forward convolution first waits on a barrier nothing arrives at, so that the
 // wait runs out and the kernel takes its error path (test of that path).
 void set_wait_limit(unsigned long long ns, bool stall_next);
-unsigned long long wait_limit_ns();
+unsigned long long wait_limit();  // in ticks of two SM cycles
 bool take_stall_request();
 
 // Forward (or data-gradient) launch over `in`.  Images at least 128 pixels
