@@ -9,10 +9,11 @@
 //     `stages` buffers, warp 1 issues the MMAs into one of two accumulators,
 //     warps 2-9 run the epilogue of the other (k_conv_fwd_persistent);
 //   weight gradient: 128 (tap, input channel) rows x n_tile output channels,
-//     accumulated over a range of pixel tiles and added to the FP32 result,
-//     one CTA of 4 warps per (row tile, channel tile, pixel range): thread 0
-//     loads, thread 32 issues the MMAs, all four warps read the accumulator
-//     (warp w owns TMEM lanes 32w..32w+31).
+//     accumulated over a range of pixel tiles and added to the FP32 result, by
+//     CTAs of 4 warps: thread 0 loads, warp 1 issues the MMAs, all four warps read
+//     the accumulators (warp w owns TMEM lanes 32w..32w+31).  One CTA per (chunk
+//     of input channels with all nine taps, channel tile, pixel range)
+//     (k_conv_wgrad_halo) or per (row tile, channel tile, pixel range) (k_conv_wgrad).
 //
 // Shared-memory operand layouts are the canonical swizzled ones for a row of
 // R = 2 * KC bytes (R = 32, 64, 128 B, TMA swizzle of the same width):
